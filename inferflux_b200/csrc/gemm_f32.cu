@@ -3,65 +3,330 @@
 // The reference has no 32-bit model path (its traits cover half and bfloat16
 // only, runtime/backends/cuda/native/common/dtype_traits.cuh:13-30) and calls
 // cuBLAS with float32 accumulation for every projection
-// (runtime/backends/cuda/native/cublas_gemm.cpp:84-102).  This kernel uses
-// plain FFMA on CUDA cores, no tensor cores and no reduced-precision mode, and
-// adds the K products of an output element in index order whatever M is, so a
-// row's result does not depend on what else is in the batch.
+// (runtime/backends/cuda/native/cublas_gemm.cpp:84-102).  These kernels use
+// plain float32 multiply-adds on CUDA cores, no tensor cores and no
+// reduced-precision mode.  How an output element is summed depends on N and K
+// only: K is cut into k_slices(N, K) slices, the products of a slice are added
+// in index order and the slices' sums in slice order, whatever M is and
+// whichever kernel runs, so a row's result does not depend on what else is in
+// the batch.
+//
+// Many rows (many_kernel): bound by the multiply-add pipe, with the 128 bytes a cycle that
+// shared memory hands to registers close behind: the operands of an 8 x 8 tile a thread take
+// as many cycles as its arithmetic (4 x 8 tiles were a tenth slower, A's values stored twice
+// over to save their copies a fifth, 8 x 16 tiles no faster and too few blocks for a narrow
+// product).  The paired multiply-add (two independent float32 operations an instruction, each
+// rounded as fmaf is) leaves issue slots for the rest.  Tiles are stored K-major, columns
+// permuted so that neither the transposing stores nor the 16-byte reads meet on a bank; the
+// next tile is loaded into registers while the present one is multiplied.  301 rows: N 22,016
+// K 2,048 629 us (43 TFLOP/s; 64 x 64 blocks of 4 x 4 a thread 1,167), N 2,048 K 11,008
+// 425 us (2,116).
+//
+// Up to 16 rows (few_kernel): bound by reading W.  A thread owns one output column and
+// runs along its row of W, which arrives through a ring of cp.async copies.  One row
+// against N 151,936 K 2,048: 205 us, 6.0 TB/s (1,406 us by 64 x 64 blocks).
 #include "common.cuh"
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;   // 256 threads, 4x4 outputs each
+constexpr int BN = 128;
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                float* __restrict__ C, int M, int N, int K, long long lda, long long ldc) {
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// the same place in the shared memory of the cluster's block `rank`
+__device__ __forceinline__ float4 read_peer4(const float* p, int rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), ra;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
+  return v;
+}
+
+// Four values of a row at k .. k + 3, zeros beyond `end` (VEC: all rows 16-byte aligned and k, end multiples of 4).
+template <bool VEC> __device__ __forceinline__ float4 load4(const float* row, int k, int end) {
+  if (VEC) return k < end ? __ldg(reinterpret_cast<const float4*>(row + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(k < end ? row[k] : 0.f, k + 1 < end ? row[k + 1] : 0.f, k + 2 < end ? row[k + 2] : 0.f, k + 3 < end ? row[k + 3] : 0.f);
+}
+
+constexpr int MK = 16;      // K per tile of many_kernel
+constexpr int BM = 64;
+
+// 128 threads, a warp as 8 x 4 lanes, the warps side by side along N: a lane has 2 groups of 4 rows, 32 apart, and 2
+// groups of 4 columns, 16 apart.
+template <bool VEC, bool SPLIT>
+__global__ void __launch_bounds__(128, 3)
+many_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+            int M, int N, int K, long long lda, long long ldc, int slice_len) {
+  constexpr int WR = BN / 32;                                  // rows of W a thread loads
   pdl_enter();
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid % 16, ty = tid / 16;          // tx -> N direction, ty -> M direction
+  extern __shared__ __align__(16) float f32_smem[];
+  float* As = f32_smem;                          // [2][MK][BM]
+  float* Ws = f32_smem + 2 * MK * BM;            // [2][MK][BN]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+  const int k_begin = SPLIT ? min(K, (int)blockIdx.z * slice_len) : 0, k_end = SPLIT ? min(K, k_begin + slice_len) : K;
+  const int mc = (lane >> 2) * 4, nc = warp * 32 + (lane & 3) * 4;
 
-  // each thread loads 4 elements of A and 4 of W per K-slab: row = tid / 4, k = (tid % 4) * 4 .. +3
-  const int lrow = tid / 4, lk = (tid % 4) * 4;
-  for (int k0 = 0; k0 < K; k0 += BK) {
+  const int lrow = tid >> 2, kq = tid & 3, lk = kq * 4;       // loads: rows lrow, + 32, ...; four values along K
+  float4 ra[2], rw[WR];
+  auto load = [&](int k0) {                                    // rows out of range read nothing
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = k0 + lk + u;
-      const int am = m0 + lrow, wn = n0 + lrow;
-      As[lk + u][lrow] = (am < M && k < K) ? A[(size_t)am * lda + k] : 0.0f;
-      Ws[lk + u][lrow] = (wn < N && k < K) ? W[(size_t)wn * K + k] : 0.0f;
+    for (int i = 0; i < 2; ++i) {
+      const int m = m0 + lrow + 32 * i;
+      ra[i] = load4<VEC>(A + (size_t)(m < M ? m : 0) * lda, k0 + lk, m < M ? k_end : 0);
     }
+#pragma unroll
+    for (int i = 0; i < WR; ++i) {
+      const int n = n0 + lrow + 32 * i;
+      rw[i] = load4<VEC>(W + (size_t)(n < N ? n : 0) * K, k0 + lk, n < N ? k_end : 0);
+    }
+  };
+  auto store = [&](int buf) {                                  // column c of row k stands at c ^ 8 (k / 4)
+    float* a = As + buf * MK * BM + lk * BM + (lrow ^ (kq << 3));
+    float* w = Ws + buf * MK * BN + lk * BN + (lrow ^ (kq << 3));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { a[32 * i] = ra[i].x; a[32 * i + BM] = ra[i].y; a[32 * i + 2 * BM] = ra[i].z; a[32 * i + 3 * BM] = ra[i].w; }
+#pragma unroll
+    for (int i = 0; i < WR; ++i) { w[32 * i] = rw[i].x; w[32 * i + BN] = rw[i].y; w[32 * i + 2 * BN] = rw[i].z; w[32 * i + 3 * BN] = rw[i].w; }
+  };
+
+  unsigned long long acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  load(k_begin);
+  store(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = k_begin; k0 < k_end; k0 += MK) {
+    const bool more = k0 + MK < k_end;
+    if (more) load(k0 + MK);
+    const float* a = As + buf * MK * BM;
+    const float* w = Ws + buf * MK * BN;
+#pragma unroll
+    for (int kk = 0; kk < MK; ++kk) {
+      const int x = (kk >> 2) << 3;
+      float av[8];
+      unsigned long long wv[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(av + 4 * i) = *reinterpret_cast<const float4*>(a + kk * BM + ((mc + 32 * i) ^ x));
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(w + kk * BN + ((nc + 16 * i) ^ x));
+        wv[2 * i] = v.x;
+        wv[2 * i + 1] = v.y;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const unsigned long long aa = pack2(av[i], av[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) fma2(acc[i][j], aa, wv[j]);
+      }
+    }
+    if (more) store(buf ^ 1);
     __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[TM], w[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-    }
-    __syncthreads();
+    buf ^= 1;
   }
+  if (!SPLIT) {
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty * TM + i;
-    if (m >= M) continue;
+    for (int i = 0; i < 8; ++i) {
+      const int m = m0 + mc + (i >> 2) * 32 + (i & 3);
+      if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx * TN + j;
-      if (n < N) C[(size_t)m * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.0f);
+      for (int j = 0; j < 4; ++j) {
+        const int n = n0 + nc + (j >> 1) * 16 + (j & 1) * 2;
+        float lo, hi;
+        unpack2(acc[i][j], lo, hi);
+        if (n < N) C[(size_t)m * ldc + n] = lo + (bias ? bias[n] : 0.0f);
+        if (n + 1 < N) C[(size_t)m * ldc + n + 1] = hi + (bias ? bias[n + 1] : 0.0f);
+      }
+    }
+    return;
+  }
+  // the cluster's blocks hold the slices of one tile: each leaves its sums in shared memory and adds up its share of the rows
+  const int slices = gridDim.z, rank = (int)cluster_rank();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float* row = f32_smem + (mc + (i >> 2) * 32 + (i & 3)) * BN + nc;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<unsigned long long*>(row + (j >> 1) * 16 + (j & 1) * 2) = acc[i][j];
+  }
+  cluster_sync();
+  const int rows = BM / slices;                                // 2, 4 or 8 slices
+  for (int p = tid; p < rows * (BN / 4); p += 128) {
+    const int r = rank * rows + p / (BN / 4), c = (p % (BN / 4)) * 4, m = m0 + r, n = n0 + c;
+    if (m >= M || n >= N) continue;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int z = 0; z < slices; ++z) {
+      const float4 v = read_peer4(f32_smem + r * BN + c, z);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    const float o[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n + i < N) C[(size_t)m * ldc + n + i] = o[i] + (bias ? bias[n + i] : 0.0f);
+  }
+  cluster_sync();                                              // no block leaves while another still reads its sums
+}
+
+constexpr int FK = 32, FSTAGES = 4, FPITCH = FK + 4;           // rows 36 floats apart: eight lanes' 16-byte reads meet no bank twice
+
+__device__ __forceinline__ void cp16(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp4(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+
+template <int R, bool VEC>
+__global__ void __launch_bounds__(128)
+few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+           int M, int N, int K, long long lda, long long ldc, int slice_len) {
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) float f32_smem[];
+  float* Wr = f32_smem;                                        // [FSTAGES][BN][FPITCH]
+  float* Ar = f32_smem + FSTAGES * BN * FPITCH;                // [FSTAGES][R][FK]
+  const int tid = threadIdx.x, n0 = blockIdx.x * BN;
+  const int k_begin = min(K, (int)blockIdx.z * slice_len), k_end = min(K, k_begin + slice_len);
+  const int steps = (k_end - k_begin + FK - 1) / FK;
+  auto copy_w = [&](int s) {
+    if (s >= steps) return;
+    float* dst = Wr + (s % FSTAGES) * BN * FPITCH;
+    const int k0 = k_begin + s * FK;
+    if (VEC) {
+#pragma unroll
+      for (int i = 0; i < BN * FK / 4 / 128; ++i) {
+        const int p = tid + i * 128, r = p / (FK / 4), c = (p % (FK / 4)) * 4;
+        const bool ok = n0 + r < N && k0 + c < k_end;
+        cp16(dst + r * FPITCH + c, W + (ok ? (size_t)(n0 + r) * K + k0 + c : 0), ok);
+      }
+    } else {
+      for (int p = tid; p < BN * FK; p += 128) {
+        const int r = p / FK, c = p % FK;
+        const bool ok = n0 + r < N && k0 + c < k_end;
+        cp4(dst + r * FPITCH + c, W + (ok ? (size_t)(n0 + r) * K + k0 + c : 0), ok);
+      }
+    }
+  };
+  auto copy_a = [&](int s) {
+    if (s >= steps) return;
+    const int k0 = k_begin + s * FK;
+    for (int p = tid; p < R * FK; p += 128) {
+      const int r = p / FK, c = p % FK;
+      const bool ok = r < M && k0 + c < k_end;
+      cp4(Ar + (s % FSTAGES) * R * FK + p, A + (ok ? (size_t)r * lda + k0 + c : 0), ok);
+    }
+  };
+  // W is a parameter, which no kernel of a step writes: its first tiles are on their way before the kernel ahead has finished
+#pragma unroll
+  for (int s = 0; s < FSTAGES - 1; ++s) copy_w(s);
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < FSTAGES - 1; ++s) {
+    copy_a(s);
+    cp_async_commit();
+  }
+  float acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(FSTAGES - 2) : "memory");
+    __syncthreads();                                           // tile s is there for all, tile s - 1 has been read by all
+    copy_w(s + FSTAGES - 1);
+    copy_a(s + FSTAGES - 1);
+    cp_async_commit();
+    const float* w = Wr + (s % FSTAGES) * BN * FPITCH + tid * FPITCH;
+    const float* a = Ar + (s % FSTAGES) * R * FK;
+#pragma unroll
+    for (int c = 0; c < FK; c += 4) {
+      const float4 wv = *reinterpret_cast<const float4*>(w + c);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float4 av = *reinterpret_cast<const float4*>(a + r * FK + c);
+        acc[r] = fmaf(av.w, wv.w, fmaf(av.z, wv.z, fmaf(av.y, wv.y, fmaf(av.x, wv.x, acc[r]))));
+      }
     }
   }
+  cp_async_wait_all();
+  const int n = n0 + tid, slices = gridDim.z;
+  if (slices == 1) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (r < M && n < N) C[(size_t)r * ldc + n] = acc[r] + (bias ? bias[n] : 0.0f);
+    return;
+  }
+  __syncthreads();                                             // the ring is free: the slices' sums go there
+#pragma unroll
+  for (int r = 0; r < R; ++r) f32_smem[r * BN + tid] = acc[r];
+  cluster_sync();
+  const int rank = (int)cluster_rank();
+  for (int p = rank * 128 + tid; p < R * (BN / 4); p += slices * 128) {
+    const int r = p / (BN / 4), c = (p % (BN / 4)) * 4;
+    if (r >= M || n0 + c >= N) continue;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int z = 0; z < slices; ++z) {
+      const float4 v = read_peer4(f32_smem + r * BN + c, z);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    const float o[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n0 + c + i < N) C[(size_t)r * ldc + n0 + c + i] = o[i] + (bias ? bias[n0 + c + i] : 0.0f);
+  }
+  cluster_sync();
+}
+
+// Slices of K, from N and K alone (1, 2, 4 or 8): enough that a few hundred rows of a narrow product fill the SMs, each
+// at least 256 long.
+int k_slices(int N, int K) {
+  const int cols = (N + BN - 1) / BN;
+  int s = 1;
+  while (s < 8 && cols * s < 128 && K / (2 * s) >= 256) s *= 2;
+  return s;
+}
+int slice_length(int K, int slices) { return ((K + slices - 1) / slices + FK - 1) / FK * FK; }
+
+template <typename Kern>
+int launch_f32(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, const float* A, const float* W, const float* bias,
+               float* C, int M, int N, int K, long long lda, long long ldc, int slice_len) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  const int rc = launch_pdl_cluster(kern, grid, dim3(threads), smem, stream, dim3(1, 1, grid.z), A, W, bias, C, M, N, K, lda, ldc, slice_len);
+  return rc ? rc : IFX_LAUNCH_CHECK();
+}
+
+template <int R>
+int few(bool vec, const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
+        cudaStream_t stream) {
+  const int slices = k_slices(N, K);
+  const dim3 grid((N + BN - 1) / BN, 1, slices);
+  const size_t smem = (size_t)FSTAGES * (BN * FPITCH + R * FK) * sizeof(float);
+  return vec ? launch_f32(few_kernel<R, true>, grid, 128, smem, stream, A, W, bias, C, M, N, K, lda, ldc, slice_length(K, slices))
+             : launch_f32(few_kernel<R, false>, grid, 128, smem, stream, A, W, bias, C, M, N, K, lda, ldc, slice_length(K, slices));
+}
+
+template <bool SPLIT>
+int many(bool vec, const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
+         int slices, cudaStream_t stream) {
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, slices);
+  size_t smem = (size_t)2 * MK * (BM + BN) * sizeof(float);
+  if (SPLIT && smem < (size_t)BM * BN * sizeof(float)) smem = (size_t)BM * BN * sizeof(float);
+  const int len = slice_length(K, slices);
+  return vec ? launch_f32(many_kernel<true, SPLIT>, grid, 128, smem, stream, A, W, bias, C, M, N, K, lda, ldc, len)
+             : launch_f32(many_kernel<false, SPLIT>, grid, 128, smem, stream, A, W, bias, C, M, N, K, lda, ldc, len);
 }
 }  // namespace
 
@@ -69,8 +334,13 @@ IFX_API int ifx_gemm_f32(const float* A, const float* W, const float* bias, floa
                          long long lda, long long ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return IFX_ERR_UNSUPPORTED;
-  int ifx_rc = 0;
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  ifx_rc = launch_pdl(gemm_f32_kernel, dim3(grid), dim3(256), 0, stream, A, W, bias, C, M, N, K, lda, ldc);
-  return ifx_rc ? ifx_rc : IFX_LAUNCH_CHECK();
+  const bool vec = (K % 4 == 0) && (((uintptr_t)W & 15) == 0);                       // of W's rows
+  const bool vec_a = vec && (lda % 4 == 0) && (((uintptr_t)A & 15) == 0);
+  if (M == 1) return few<1>(vec, A, W, bias, C, M, N, K, lda, ldc, stream);
+  if (M <= 4) return few<4>(vec, A, W, bias, C, M, N, K, lda, ldc, stream);
+  if (M <= 8) return few<8>(vec, A, W, bias, C, M, N, K, lda, ldc, stream);
+  if (M <= 16) return few<16>(vec, A, W, bias, C, M, N, K, lda, ldc, stream);
+  const int slices = k_slices(N, K);
+  if (slices > 1) return many<true>(vec_a, A, W, bias, C, M, N, K, lda, ldc, slices, stream);
+  return many<false>(vec_a, A, W, bias, C, M, N, K, lda, ldc, 1, stream);
 }

@@ -134,6 +134,25 @@ def test_gemm_f32(ops, m, n, k):
     assert torch.equal(one[0], out[m - 1])
 
 
+@pytest.mark.parametrize("m,n,k,offset", [(4, 300, 2052, 0), (8, 129, 515, 0), (16, 2048, 2048, 0), (17, 2048, 2048, 0), (33, 257, 1030, 0),
+                                          (64, 100, 4096, 1), (129, 200, 4096, 0), (128, 16500, 64, 0), (130, 16500, 40, 0), (200, 2, 1028, 3)])
+def test_gemm_f32_tiles_and_slices(ops, m, n, k, offset):
+    """Every kernel and both ways of loading, one slice of K and several (narrow products), rows that begin off the 16-byte
+    boundaries; a row's sums are the same bits whichever kernel makes them."""
+    a = _rand((m, k + 4 + offset), torch.float32, 18)[:, offset:offset + k]
+    w, b = _rand((n, k), torch.float32, 19), _rand((n,), torch.float32, 20)
+    out = torch.full((m + 1, n), 7.0, dtype=torch.float32, device=DEV)
+    ops.gemm_f32(a, w, b, out[:m])
+    want = a.double().cpu() @ w.double().cpu().T + b.double().cpu()
+    # a chain of k roundings, each half a unit of 2^-23 of a partial sum: their random sum stays far below k units
+    _close(out[:m], want, 2e-6, "gemm_f32")
+    assert bool((out[m] == 7.0).all())
+    for rows in (1, 3, 8, 12, 40, m):
+        part = torch.empty((min(rows, m), n), dtype=torch.float32, device=DEV)
+        ops.gemm_f32(a[m - part.shape[0]:], w, b, part)
+        assert torch.equal(part, out[m - part.shape[0]:m]), rows
+
+
 def test_gemm_f32_is_true_float32(ops):
     """Values that a reduced-precision (tf32, 10-bit mantissa) product would lose."""
     k = 64
