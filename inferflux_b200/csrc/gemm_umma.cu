@@ -477,8 +477,8 @@ int pick_tile_n(int M, int n_out, int pairs) {
 
 template <int MODE, typename TOut>
 int launch_gemm_pair(const void* A, long long lda, const void* W, const float* bias, void* out, long long ldo, int M, int n_out,
-                     int K, int* error_flag, cudaStream_t stream) {
-  constexpr bool SWIGLU = MODE == 1;
+                     int K, GluShape glu, int* error_flag, cudaStream_t stream) {
+  constexpr bool SWIGLU = MODE == 1 || MODE == 5;
   auto kern = gemm_umma_pair_kernel<MODE, TOut>;
   static int sms = 0;
   if (!sms) {
@@ -497,7 +497,7 @@ int launch_gemm_pair(const void* A, long long lda, const void* W, const float* b
   const int tiles = ((M + 255) / 256) * ((n_out + out_cols - 1) / out_cols);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
   rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
-                          ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, (const int*)nullptr, 0, GluShape{});
+                          ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, (const int*)nullptr, 0, glu);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
 
@@ -603,22 +603,24 @@ int launch_gemm_skinny(const void* X, long long ldx, const void* W, float* out, 
 }  // namespace
 
 // out[M, n_out] = A[M, K] * W^T (+ bias), W [n_out, K] contiguous; or, with act 1, W [2 * n_out, K] =
-// [gate; up] and out = silu(A gate^T) * (A up^T), or, with act 2, out = relu(A W^T)^2.  A rows lda elements apart; K and lda multiples of 8;
+// [gate; up] and out = silu(A gate^T) * (A up^T), or, with act 2, out = relu(A W^T)^2, or, with act 3, act 1's two halves through clamped_glu of (limit, alpha, shift) (both bfloat16 out).  A rows lda elements apart; K and lda multiples of 8;
 // A and W 16-byte aligned.  out_dtype: float32 or bfloat16.  error_flag: a device word set if a bounded
 // wait inside the kernel runs out.
 IFX_API int ifx_gemm_umma(const void* A, long long lda, const void* W, const float* bias, void* out, long long ldo,
-                          int out_dtype, int M, int n_out, int K, int act, int* error_flag, cudaStream_t stream) {
+                          int out_dtype, int M, int n_out, int K, int act, float limit, float alpha, float shift, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || n_out <= 0) return 0;
-  if (act < 0 || act > 2 || K <= 0 || (K & 7) || (lda & 7) || !error_flag) return IFX_ERR_UNSUPPORTED;
+  if (act < 0 || act > 3 || K <= 0 || (K & 7) || (lda & 7) || !error_flag) return IFX_ERR_UNSUPPORTED;
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return IFX_ERR_ALIGNMENT;
   if (act && bias) return IFX_ERR_UNSUPPORTED;
+  const GluShape glu{limit, alpha, shift};
   if (out_dtype == IFX_BF16)
-    return act == 1 ? launch_gemm_pair<1, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, error_flag, stream)
-         : act == 2 ? launch_gemm_pair<4, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, error_flag, stream)
-                    : launch_gemm_pair<0, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, error_flag, stream);
+    return act == 1 ? launch_gemm_pair<1, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, glu, error_flag, stream)
+         : act == 3 ? launch_gemm_pair<5, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, glu, error_flag, stream)
+         : act == 2 ? launch_gemm_pair<4, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, glu, error_flag, stream)
+                    : launch_gemm_pair<0, bf16>(A, lda, W, bias, out, ldo, M, n_out, K, glu, error_flag, stream);
   if (out_dtype == IFX_F32 && act < 2)
-    return act ? launch_gemm_pair<1, float>(A, lda, W, bias, out, ldo, M, n_out, K, error_flag, stream)
-               : launch_gemm_pair<0, float>(A, lda, W, bias, out, ldo, M, n_out, K, error_flag, stream);
+    return act ? launch_gemm_pair<1, float>(A, lda, W, bias, out, ldo, M, n_out, K, glu, error_flag, stream)
+               : launch_gemm_pair<0, float>(A, lda, W, bias, out, ldo, M, n_out, K, glu, error_flag, stream);
   return IFX_ERR_UNSUPPORTED;
 }
 

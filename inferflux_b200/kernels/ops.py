@@ -69,9 +69,9 @@ def _lib():
         lib.ifx_attn_decode_even_pieces.argtypes = [c_int, c_int, c_int, c_int]
         lib.ifx_attn_decode_even_pieces.restype = c_int
         lib.ifx_gemv_bf16.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll,
-                                      c_int, c_int, c_void_p]
+                                      c_int, c_int, c_float, c_float, c_float, c_void_p]
         lib.ifx_gemm_umma.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int,
-                                      c_void_p, c_void_p]
+                                      c_float, c_float, c_float, c_void_p, c_void_p]
         lib.ifx_gemm_umma.restype = c_int
         lib.ifx_gemm_umma_skinny.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_int,
                                              c_void_p, c_void_p]
@@ -413,17 +413,29 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
 GEMV_MAX_ROWS = 16
 
 
+def _glu_shape(glu, other: bool, what: str):
+    """(limit, alpha, shift) of a clamped gated activation in a product's epilogue; zeros without one."""
+    if glu is None:
+        return 0.0, 0.0, 0.0
+    limit, alpha, shift = (float(v) for v in glu)
+    _need(limit > 0.0 and not other, f"{what}: a clamped activation needs a positive limit and no other activation")
+    return limit, alpha, shift
+
+
 def gemv_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-              swiglu: bool = False, k_splits: int = 1, relu2: bool = False) -> torch.Tensor:
+              swiglu: bool = False, k_splits: int = 1, relu2: bool = False, glu=None) -> torch.Tensor:
     """out[M, N] = x[M, K] @ w[N, K]^T (+ bias) for M <= 16, bfloat16 operands,
     float32 accumulation, bfloat16 or float32 result.  With ``swiglu`` w is
     [2N, K] = [gate; up] and out = silu(x gate^T) * (x up^T); with ``relu2`` out =
-    relu(x w^T)^2.  With ``k_splits`` > 1 out is float32 [k_splits, M, N]: slice s is the sum over the
+    relu(x w^T)^2; with ``glu`` = (limit, alpha, shift) the stacked halves meet as in :func:`glu_clamped`.
+    With ``k_splits`` > 1 out is float32 [k_splits, M, N]: slice s is the sum over the
     s-th part of K and the caller adds the slices.  ``w`` is a parameter: the
     kernel starts to read it before the kernel launched before it has finished,
     so it must not be that kernel's output."""
     m, k = x.shape
     n = out.shape[-1]
+    limit, alpha, shift = _glu_shape(glu, swiglu or relu2, "gemv_bf16")
+    swiglu = swiglu or glu is not None
     _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous(), "gemv_bf16: bfloat16 operands")
     _need(w.shape == ((2 * n if swiglu else n), k), "gemv_bf16: shapes")
     _need(m <= GEMV_MAX_ROWS and k % 8 == 0, f"gemv_bf16: at most {GEMV_MAX_ROWS} rows and K a multiple of 8")
@@ -438,21 +450,24 @@ def gemv_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n and not swiglu and not relu2, "gemv_bf16: bias float32 [N]")
     _check(_lib().ifx_gemv_bf16(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _code(out), m, n, k,
-                                x.stride(0) if m > 1 else k, ldo, 1 if swiglu else 2 if relu2 else 0, int(k_splits),
-                                _stream()), "gemv_bf16")
+                                x.stride(0) if m > 1 else k, ldo, 3 if glu else 1 if swiglu else 2 if relu2 else 0, int(k_splits),
+                                limit, alpha, shift, _stream()), "gemv_bf16")
     return out
 
 
 def gemm_umma(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-              swiglu: bool = False, relu2: bool = False) -> torch.Tensor:
+              swiglu: bool = False, relu2: bool = False, glu=None) -> torch.Tensor:
     """out[M, N] = x[M, K] @ w[N, K]^T (+ bias) for many rows, on the tcgen05 tensor
     cores (TMA operands, accumulators in tensor memory), bfloat16 operands, float32
     accumulation, bfloat16 or float32 result.  With ``swiglu`` w is [2N, K] =
     [gate; up] and out = silu(x gate^T) * (x up^T), the activation applied in the
-    product's epilogue; with ``relu2`` (bfloat16 out) out = relu(x w^T)^2 likewise.  Two SMs share each tile (cta_group::2).  A bounded wait
+    product's epilogue; with ``relu2`` (bfloat16 out) out = relu(x w^T)^2 likewise, with
+    ``glu`` = (limit, alpha, shift) (bfloat16 out) the stacked halves meet as in :func:`glu_clamped`.  Two SMs share each tile (cta_group::2).  A bounded wait
     that runs out sets the device's error flag (see :func:`check_device_errors`)."""
     m, k = x.shape
     n = out.shape[-1]
+    limit, alpha, shift = _glu_shape(glu, swiglu or relu2, "gemm_umma")
+    swiglu = swiglu or glu is not None
     _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous(), "gemm_umma: bfloat16 operands")
     _need(w.shape == ((2 * n if swiglu else n), k), "gemm_umma: shapes")
     _need(out.dim() == 2 and out.shape[0] == m and out.stride(1) == 1 and x.stride(1) == 1,
@@ -461,7 +476,8 @@ def gemm_umma(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n and not swiglu and not relu2, "gemm_umma: bias float32 [N]")
     _check(_lib().ifx_gemm_umma(_ptr(x), x.stride(0) if m > 1 else k, _ptr(w), _ptr(bias), _ptr(out), out.stride(0),
-                                _code(out), m, n, k, 1 if swiglu else 2 if relu2 else 0, _ptr(error_flag(x.device)), _stream()),
+                                _code(out), m, n, k, 3 if glu else 1 if swiglu else 2 if relu2 else 0, limit, alpha, shift,
+                                _ptr(error_flag(x.device)), _stream()),
            "gemm_umma")
     return out
 

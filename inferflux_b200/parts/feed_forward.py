@@ -154,7 +154,7 @@ class ClampedGLU(Part):
         y = W_down ( g * sigmoid(alpha * g) * (u + shift) ) + b_down
 
     Gate and up are one stacked projection whose sums stay float32; biases, clamps and the activation are one
-    kernel that rounds once into the engine's type.  params: ``hidden``, ``intermediate``, ``limit``, ``alpha``
+    kernel, or without biases the product's epilogue, that rounds once into the engine's type.  params: ``hidden``, ``intermediate``, ``limit``, ``alpha``
     (default 1.702), ``shift`` (default 1), ``bias`` (default true), ``name`` (tensors
     ``<prefix>.<name>.{gate,up,down}`` and ``.{gate,up,down}.b``)."""
 
@@ -191,8 +191,19 @@ class ClampedGLU(Part):
         self.down = Linear(tensors.pop(n("down")), tensors.pop(n("down.b")) if self.has_bias else None)
 
     def forward(self, x: torch.Tensor, ctx):
-        z = self.gate_up.forward(x, out_dtype=torch.float32, allow_partials=True, f32_sums=True)
+        w = self.gate_up.weight
         act = torch.empty((x.shape[0], self.intermediate), dtype=x.dtype, device=x.device)
+        # without biases the activation sits in the epilogue of the product, which rounds once from float32 sums too, for few
+        # rows (8: 47 us against 54 at 7B sizes) and for many (2,048: 336 us against 357 + 96, the sums written and read back)
+        fused = (w.dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.limit > 0.0
+                 and not self.has_bias)
+        if fused and x.shape[0] <= GEMV_ROWS:
+            ops.gemv_bf16(x, w, None, act, glu=(self.limit, self.alpha, self.shift))
+            return self.down.forward(act, out_dtype=torch.float32, allow_partials=True, f32_sums=True)
+        if fused and x.is_contiguous() and x.shape[0] > FUSED_PRODUCT_ROWS:
+            ops.gemm_umma(x, w, None, act, glu=(self.limit, self.alpha, self.shift))
+            return self.down.forward(act, out_dtype=torch.float32, allow_partials=True, f32_sums=True)
+        z = self.gate_up.forward(x, out_dtype=torch.float32, allow_partials=True, f32_sums=True)
         ops.glu_clamped(z.tensor if isinstance(z, PartialSums) else z, self.gate_up_bias, act, self.limit, self.alpha, self.shift)
         return self.down.forward(act, out_dtype=torch.float32, allow_partials=True, f32_sums=True)
 

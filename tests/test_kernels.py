@@ -797,6 +797,23 @@ def test_gemm_umma_swiglu(ops, m, inter, k):
     _close(out, gate / (1 + torch.exp(-gate)) * up, 6e-3, "gemm_umma swiglu")
 
 
+@pytest.mark.parametrize("m,inter,k", [(1, 5, 40), (8, 176, 64), (8, 2368, 3584), (5, 100, 96), (256, 128, 64), (700, 1000, 328), (129, 131, 64)])
+def test_products_with_a_clamped_activation(ops, m, inter, k):
+    """The weight-streaming and the tcgen05 product with the clamped gated activation in their epilogues; the inputs pass the
+    limits on both sides."""
+    x, w = _rand((m, k), torch.bfloat16, 56), _rand((2 * inter, k), torch.bfloat16, 57, 4.0 / math.sqrt(k))
+    limit, alpha, shift = 3.0, 1.702, 1.0
+    out = torch.full((m, inter), float("nan"), dtype=torch.bfloat16, device=DEV)
+    (ops.gemv_bf16 if m <= 8 else ops.gemm_umma)(x, w, None, out, glu=(limit, alpha, shift))
+    ops.check_device_errors(DEV)
+    gu = x.double().cpu() @ w.double().cpu().T
+    g, u = gu[:, :inter].clamp(max=limit), gu[:, inter:].clamp(-limit, limit)
+    _close(out, g * torch.sigmoid(alpha * g) * (u + shift), 6e-3, "clamped activation in the epilogue")
+    for bad in (dict(glu=(0.0, 1.0, 1.0)), dict(glu=(1.0, 1.0, 1.0), swiglu=True)):
+        with pytest.raises(ops.KernelError):
+            (ops.gemv_bf16 if m <= 8 else ops.gemm_umma)(x, w, None, out, **bad)
+
+
 @pytest.mark.parametrize("m", [1, 17, 32, 40, 64, 100, 256])
 @pytest.mark.parametrize("n,k", [(3584, 3584), (4608, 3584), (3584, 18944), (100, 96), (300, 1096), (257, 64)])
 def test_gemm_umma_skinny(ops, m, n, k):
