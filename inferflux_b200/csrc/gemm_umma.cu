@@ -280,7 +280,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else {
     const int quarter = warp & 3;
     const int row_in_tile = (int)rank * 128 + quarter * 32 + lane;
-    const bool vec = (ldo % 8 == 0) && ((uintptr_t)out % 16 == 0);
+    const bool vec = (ldo * sizeof(TOut) % 16 == 0) && ((uintptr_t)out % 16 == 0);   // rows on 16-byte boundaries
     int count = 0;
     for (int t = pair; t < tiles; t += n_pairs) {
       if (tile_expert && tile_expert[t % m_tiles] < 0) continue;

@@ -46,7 +46,7 @@ from ..config.registry import register_part
 from ..kernels import ops
 from ..weights.loader import MATRIX, VECTOR, WeightSpec
 from .base import Part, RunInfo, StateNeed
-from .linear import Linear
+from .linear import Linear, stack_rows
 from .state_space import describe_row_entries
 
 DECAY_SCALE = math.exp(-0.5)
@@ -241,9 +241,7 @@ class GatedDelta(Part):
         for k, m in mats.items():
             self.at[k], row = row, row + m.shape[0]
         self.at["inner"] = self.at.get("a1", self.at.get("g1", 0))
-        if outer and row % 4:                              # rows of float32 sums that start on 16-byte boundaries
-            mats["end"] = mats["b"].new_zeros((4 - row % 4, self.hidden))
-        self.stacked = Linear(torch.cat(list(mats.values()), dim=0))
+        self.stacked = Linear(stack_rows(list(mats.values())))       # (and its rows of float32 sums start on 16-byte boundaries)
         del mats, outer
         self.conv_w = torch.cat([f32(f"{x}.conv") for x in ("q", "k", "v")]).contiguous()
         self.a_log, self.dt_bias = f32("A_log"), f32("dt_bias")

@@ -45,7 +45,7 @@ from ..config.registry import register_part
 from ..kernels import ops
 from ..weights.loader import MATRIX, VECTOR, WeightSpec
 from .base import KVNeed, Part, RunInfo, StateNeed
-from .linear import Linear
+from .linear import Linear, stack_rows
 
 QUERY_TILE = 16     # tokens per query tile of the plain attention kernel
 CHUNK_TILE = 64     # tokens per query tile of the tensor-core kernel for prompt portions
@@ -233,7 +233,10 @@ class WindowAttention(Part):
                              + ([torch.zeros(mats[3].shape[0], device=mats[3].device)] if self.gate else [])).contiguous()
         # where heads are normed one by one, the kernel that norms them adds the biases
         self.head_bias = bias if self.qk_norm == "heads" else None
-        self.qkvg = Linear(torch.cat(mats, dim=0), None if self.qk_norm == "heads" else bias)
+        stacked = stack_rows(mats)
+        if bias is not None and self.qk_norm != "heads":
+            bias = torch.nn.functional.pad(bias, (0, stacked.shape[0] - bias.numel()))
+        self.qkvg = Linear(stacked, None if self.qk_norm == "heads" else bias)
         del mats
         if self.distance_toll:
             self.toll = tuple(tensors.pop(n(x)).to(torch.float32).contiguous() for x in ("r1", "r2"))
