@@ -3,7 +3,8 @@
 //
 // Same formulas as the other attention kernels (attention_generic.cu): kv head
 // = head / (n_heads / n_kv), s = (q . k) * scale, causal with an optional
-// window, float32 softmax, o = sum p v / sum p.  The reference's kernel for this
+// window or within chunks, float32 softmax, o = sum p v / sum p, and with a gate
+// per head o times its sigmoid.  The reference's kernel for this
 // case is scalar or mma.sync with fp16 operands
 // (runtime/backends/cuda/kernels/flash_attention.cu:52-173,
 // runtime/backends/cuda/kernels/flash_attention_mma.cuh:153-379).
@@ -170,7 +171,7 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
                          int page_size, int page_shift, UmmaMeta m, const int* __restrict__ tile_entry,
                          const int* __restrict__ tile_q0, int n_heads, int n_kv, float scale, int window,
                          int* __restrict__ error_flag, float* __restrict__ part_o, float* __restrict__ part_ml, int n_splits,
-                         int tile_rows) {
+                         int tile_rows, HeadGate gate) {
   // The kernel before this one (it rotates the queries and writes the new keys and values) is waited for only
   // where its results are first read or the scratch of an earlier launch first written; until then the block
   // reads the step's description, sets up its barriers and gets its tensor memory.
@@ -201,7 +202,7 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
   const int* bt = m.block_tables + (size_t)e * m.bt_stride;
   const int rows0 = min(UM, rows_all), rows1 = rows_all - rows0;  // rows of the two slots (the second may have none)
   const int kend = pos0 + rows_all;                              // keys [.., kend) may be seen by the block's last row
-  const int kfirst = window > 0 ? max(0, pos0 - window + 1) : 0; // first key the block's first row may see
+  const int kfirst = first_visible(pos0, window);                // first key the block's first row may see
   // gridDim.z > 1: the key tiles are cut into n_splits consecutive parts, one block each; the parts leave
   // their unnormalised O and (maximum, sum) in scratch for the merge kernel.  Few query tiles over a long
   // context (a short portion of a long prompt) would otherwise leave most of the GPU idle.
@@ -389,12 +390,13 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
   const int my_n = sl ? n_t1 : n_t0, my_rows = (sl && !narrow) ? rows1 : rows0;
   const int my_pos0 = pos0 + (narrow ? 0 : sl * UM);
   const int my_kend = my_pos0 + my_rows;
-  const int my_kfirst = window > 0 ? max(0, my_pos0 - window + 1) : 0;
+  const int my_klast_first = first_visible(my_kend - 1, window);  // from here on every row of the slot sees back far enough
   const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;  // this warp's quarter of the 128 lanes
   const unsigned tm_base = tmem + sl * TM_SLOT + lane_base, tm_o = tm_base + TM_O;
   float mrow = -INFINITY, lrow = 0.0f;
   const float sl2 = scale * LOG2E_U;
   const int p_row = my_pos0 + row;                                // this thread's query position
+  const int p_first = first_visible(p_row, window);
   bool failed = false;
 
   // O accumulates in tensor memory over all key tiles.  The running maximum of a row is only moved when a
@@ -423,11 +425,11 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
 #pragma unroll
         for (int c = 0; c < 32; ++c) { s[c] = __uint_as_float(r0[c]); s[32 + c] = __uint_as_float(r1[c]); }
       }
-      if (key0 + UN - 1 > my_pos0 || window > 0 || key0 < my_kfirst || key0 + UN > my_kend) {   // diagonal, window, edges
+      if (key0 + UN - 1 > my_pos0 || key0 < my_klast_first || key0 + UN > my_kend) {   // diagonal, window, edges
 #pragma unroll
         for (int c = 0; c < UN; ++c) {
           const int key = key0 + c;
-          const bool vis = key <= p_row && key < my_kend && (window <= 0 || key > p_row - window);
+          const bool vis = key <= p_row && key < my_kend && key >= p_first;
           if (!vis) s[c] = -INFINITY;
         }
       }
@@ -575,7 +577,8 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
       return;
     }
     if (my_n <= 0) return;
-    const float inv = lrow > 0.0f ? 1.0f / lrow : 0.0f;
+    float inv = lrow > 0.0f ? 1.0f / lrow : 0.0f;
+    if (gate.p && row < my_rows) inv *= gate.factor(tok0 + (narrow ? 0 : sl * UM) + row, head, UD, 0);
 #pragma unroll
     for (int j = 0; j < UD / 32; ++j) {
       unsigned r[32];
@@ -645,7 +648,7 @@ __global__ void __launch_bounds__(UD)
 attn_prefill_umma_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                bf16* __restrict__ out, long long out_stride, UmmaMeta m,
                                const int* __restrict__ tile_entry, const int* __restrict__ tile_q0, int n_heads, int n_splits,
-                               int tile_rows) {
+                               int tile_rows, HeadGate gate) {
   pdl_launch_dependents();
   __shared__ float ml_s[MERGE_ROWS][MERGE_MAX_SPLITS][2];
   __shared__ float f_s[MERGE_ROWS][MERGE_MAX_SPLITS];
@@ -676,7 +679,7 @@ attn_prefill_umma_merge_kernel(const float* __restrict__ part_o, const float* __
       f_s[rr][sp] = f;
       l += ml_s[rr][sp][1] * f;
     }
-    inv_s[rr] = l > 0.0f ? 1.0f / l : 0.0f;
+    inv_s[rr] = (l > 0.0f ? 1.0f / l : 0.0f) * (gate.p && r0 + rr < rows ? gate.factor(tok0 + r0 + rr, head, UD, 0) : 1.0f);
   }
   __syncthreads();
 #pragma unroll
@@ -746,7 +749,9 @@ IFX_API int ifx_attn_prefill_umma_plan(int n_tiles, int n_heads, int max_key_til
 // with 128 every tile's key tiles are dealt out to both halves of its block: twice the blocks, for steps whose
 // tiles of 256 would leave SMs idle).
 // q rows, out rows, k_layer and v_layer 16-byte aligned.  error_flag: a device int set to 1 if a bounded
-// wait inside the kernel ran out (the output is then invalid).  n_splits > 1: scratch part_o float32
+// wait inside the kernel ran out (the output is then invalid).  window as first_visible takes it (negative: chunks).
+// gate: null, or one float32 number a token and head in gate_parts slices to be added, the result is multiplied by the
+// sigmoid of their sum.  n_splits > 1: scratch part_o float32
 // [n_tiles * n_heads * n_splits * 256 * 128] (16-byte aligned) and part_ml float32 [n_tiles * n_heads * n_splits * 256 * 2].
 IFX_API int ifx_attn_prefill_umma(const void* q, long long q_stride, void* out, long long out_stride,
                                   void* k_layer, void* v_layer, long long page_stride, int page_size,
@@ -754,8 +759,11 @@ IFX_API int ifx_attn_prefill_umma(const void* q, long long q_stride, void* out, 
                                   int n_tiles, const int* entry_q_start, const int* entry_q_len,
                                   const int* entry_ctx_start, int n_heads, int n_kv, int head_dim, float scale,
                                   int window, int* error_flag, float* part_o, float* part_ml, int n_splits,
-                                  int num_pages, int tile_rows, cudaStream_t stream) {
+                                  int num_pages, int tile_rows, const float* gate, int gate_parts, long long gate_part_stride,
+                                  int gate_stride, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
+  if (gate && gate_parts < 1) return IFX_ERR_UNSUPPORTED;
+  const HeadGate hg{gate, gate_parts, gate_part_stride, gate_stride, 1};
   if (head_dim != UD || n_kv < 1 || n_heads % n_kv || n_tiles > 65535 || !error_flag) return IFX_ERR_UNSUPPORTED;
   if (tile_rows != UM && tile_rows != 2 * UM) return IFX_ERR_UNSUPPORTED;
   if (n_splits < 1 || n_splits > MERGE_MAX_SPLITS || (n_splits > 1 && (!part_o || !part_ml))) return IFX_ERR_UNSUPPORTED;
@@ -774,10 +782,10 @@ IFX_API int ifx_attn_prefill_umma(const void* q, long long q_stride, void* out, 
   if (e != cudaSuccess) return (int)e;
   ifx_rc = launch_pdl(attn_prefill_umma_kernel, dim3(n_heads, n_tiles, n_splits), dim3(U_THREADS), SMEM_UMMA, stream,
                       (const bf16*)q, q_stride, (bf16*)out, out_stride, map_k, map_v, page_size, page_shift, m,
-                      tile_entry, tile_q0, n_heads, n_kv, scale, window, error_flag, part_o, part_ml, n_splits, tile_rows);
+                      tile_entry, tile_q0, n_heads, n_kv, scale, window, error_flag, part_o, part_ml, n_splits, tile_rows, hg);
   if (!ifx_rc) ifx_rc = IFX_LAUNCH_CHECK();
   if (ifx_rc || n_splits == 1) return ifx_rc;
   ifx_rc = launch_pdl(attn_prefill_umma_merge_kernel, dim3(n_heads, n_tiles, tile_rows / MERGE_ROWS), dim3(UD), 0, stream, (const float*)part_o,
-                      (const float*)part_ml, (bf16*)out, out_stride, m, tile_entry, tile_q0, n_heads, n_splits, tile_rows);
+                      (const float*)part_ml, (bf16*)out, out_stride, m, tile_entry, tile_q0, n_heads, n_splits, tile_rows, hg);
   return ifx_rc ? ifx_rc : IFX_LAUNCH_CHECK();
 }

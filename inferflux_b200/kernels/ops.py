@@ -88,7 +88,7 @@ def _lib():
         lib.ifx_attn_prefill_umma.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int,
                                               c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                               c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p,
-                                              c_void_p, c_int, c_int, c_int, c_void_p]
+                                              c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_ll, c_int, c_void_p]
         lib.ifx_attn_prefill_umma_plan.argtypes = [c_int, c_int, c_int]
         lib.ifx_attn_prefill_umma_plan.restype = c_int
         lib.ifx_argmax.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p]
@@ -675,17 +675,19 @@ def attn_prefill_umma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_layer
                       tile_entry: torch.Tensor, tile_q0: torch.Tensor, n_tiles: int,
                       entry_q_start: torch.Tensor, entry_q_len: torch.Tensor, entry_ctx_start: torch.Tensor,
                       n_heads: int, n_kv: int, head_dim: int, scale: float, window: int,
-                      n_splits: int = 1, tile_rows: int = 256) -> torch.Tensor:
+                      n_splits: int = 1, tile_rows: int = 256, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention of prompt portions with tcgen05.mma and tensor-memory
     accumulators (bfloat16, head_dim 128); query tiles of ``tile_rows`` = 256 or
     128 tokens listed by tile_entry / tile_q0 (a block takes a tile and a head;
     with 128 the tile's key tiles are dealt out to both halves of the block:
     twice the blocks, for steps whose tiles of 256 would leave SMs idle).  With ``n_splits`` > 1 the keys of every tile are cut
     into that many parts (see :func:`attn_prefill_umma_splits`), merged by a
-    second kernel.  A bounded wait that runs out sets the device error flag
-    (see :func:`check_device_errors`)."""
+    second kernel.  A negative ``window`` = -c: a token sees its own chunk of c positions.  With ``gate`` (float32 sums
+    ``[N, >= heads]`` or slices of them) a head's result is multiplied by the sigmoid of its number.  A bounded wait that
+    runs out sets the device error flag (see :func:`check_device_errors`)."""
     _need(q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and k_layer.dtype == torch.bfloat16,
           "attn_prefill_umma: bfloat16 operands")
+    gp, g_parts, g_pstride, g_stride = _gate_slices(gate, n_heads, "attn_prefill_umma")
     _need(head_dim == UMMA_ATTENTION_HEAD_DIM, f"attn_prefill_umma: head_dim {head_dim} is not 128")
     _need(block_tables.dtype == torch.int32 and block_tables.stride(1) == 1, "attn: block_tables int32 [R, B]")
     # The kernel reads the cache through a TMA tensor map, which wants to know how many pages lie behind page 0:
@@ -706,7 +708,8 @@ def attn_prefill_umma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_layer
                                         _ptr(tile_entry), _ptr(tile_q0), n_tiles, _ptr(entry_q_start),
                                         _ptr(entry_q_len), _ptr(entry_ctx_start), n_heads, n_kv, head_dim,
                                         float(scale), int(window), _ptr(error_flag(q.device)), _ptr(part_o),
-                                        _ptr(part_ml), int(n_splits), int(num_pages), int(tile_rows), _stream()),
+                                        _ptr(part_ml), int(n_splits), int(num_pages), int(tile_rows), gp, g_parts, g_pstride,
+                                        g_stride, _stream()),
            "attn_prefill_umma")
     return out
 

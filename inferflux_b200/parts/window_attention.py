@@ -58,8 +58,8 @@ class QueryTiles:
     (entry, place in the entry) per token of the entries with fewer than PORTION_MIN new tokens (decoded tokens
     among them); ``dec_entry``: the entries that bring exactly one token, and ``short_*``: the tokens of the other
     entries below PORTION_MIN (the two together are ``single_*`` again, for mixers whose single tokens take the split
-    tensor-core kernel); ``tile_*`` and ``chunk_*``: the other entries cut into tiles of QUERY_TILE and of CHUNK_TILE
-    tokens."""
+    tensor-core kernel); ``tile_*``, ``chunk_*`` and ``umma_*``: the other entries cut into tiles of QUERY_TILE, of
+    CHUNK_TILE and of ``umma_rows`` tokens."""
 
     single_entry: torch.Tensor
     single_q0: torch.Tensor
@@ -76,11 +76,15 @@ class QueryTiles:
     short_entry: torch.Tensor = None
     short_q0: torch.Tensor = None
     n_short: int = 0
+    umma_entry: torch.Tensor = None
+    umma_q0: torch.Tensor = None
+    n_umma: int = 0
+    umma_rows: int = 0
 
 
-def describe_query_tiles(layout, put) -> QueryTiles:
+def describe_query_tiles(layout, put, umma_rows: int = ops.UMMA_ATTENTION_TILE) -> QueryTiles:
     single_entry, single_q0, tile_entry, tile_q0, chunk_entry, chunk_q0 = [], [], [], [], [], []
-    dec_entry, short_entry, short_q0 = [], [], []
+    dec_entry, short_entry, short_q0, umma_entry, umma_q0 = [], [], [], [], []
     for i in range(layout.n_entries):
         n = int(layout.q_len[i])
         if n < PORTION_MIN:
@@ -95,10 +99,12 @@ def describe_query_tiles(layout, put) -> QueryTiles:
             tile_entry.append(i), tile_q0.append(q0)
         for q0 in range(0, n, CHUNK_TILE):
             chunk_entry.append(i), chunk_q0.append(q0)
+        for q0 in range(0, n, umma_rows):
+            umma_entry.append(i), umma_q0.append(q0)
     rows = np.repeat(np.arange(layout.n_entries), layout.q_len[:layout.n_entries])
     return QueryTiles(put(single_entry), put(single_q0), len(single_entry), put(tile_entry), put(tile_q0), len(tile_entry),
                       put(chunk_entry), put(chunk_q0), len(chunk_entry), put(rows), put(dec_entry), len(dec_entry),
-                      put(short_entry), put(short_q0), len(short_entry))
+                      put(short_entry), put(short_q0), len(short_entry), put(umma_entry), put(umma_q0), len(umma_entry), umma_rows)
 
 
 class WindowAttention(Part):
@@ -250,7 +256,20 @@ class WindowAttention(Part):
         self.o = Linear(tensors.pop(n("o")), tensors.pop(n("o.b")) if self.bias == "all" else None)
 
     def describe_step(self, layout, put) -> QueryTiles:
-        return describe_query_tiles(layout, put)
+        # tiles of 256 tokens of the tcgen05 kernel where they (a block a tile and head) are more than half the SMs, else of
+        # 128: twice the blocks (as the plain attention layers choose them, with the figures there)
+        tile = ops.UMMA_ATTENTION_TILE
+        blocks = sum((int(n) + tile - 1) // tile for n in layout.q_len[:layout.n_entries] if n >= PORTION_MIN) * self.heads
+        if torch.device(self.device).type == "cuda" and 2 * blocks <= ops.sm_count(self.device):
+            tile //= 2
+        return describe_query_tiles(layout, put, tile)
+
+    def _umma(self, out: torch.Tensor) -> bool:
+        """Whether prompt portions of a fast layer go to the tcgen05 kernel: heads of 128 and nothing that it does not know
+        (it knows windows, chunks and a gate per head).  2,048 tokens of the 7B sizes in chunks of 8,192: 47 us against 165 for
+        the mma.sync kernel."""
+        return (self.dim == ops.UMMA_ATTENTION_HEAD_DIM and not (self.softcap or self.keep_first or self.sink or self.q_temp)
+                and self.toll is None and self.gate in (None, "heads") and out.data_ptr() % 16 == 0)
 
     @property
     def inner_width(self) -> int:
@@ -319,7 +338,12 @@ class WindowAttention(Part):
             singles = (step.short_entry, step.short_q0, step.n_short)
         if singles[2]:          # decoded tokens and the shortest portions: a block a token and head
             ops.attn_paged_options(q, q.stride(0), out, *pages, *singles, *common, *rest, single_tokens=True, **more)
-        if step.n_chunk and fast:
+        if step.n_umma and fast and self._umma(out):
+            max_keys = min(ctx.max_ctx_len, abs(self.reach) + 256) if self.reach else ctx.max_ctx_len
+            ops.attn_prefill_umma(q, q.stride(0), out, *pages, step.umma_entry, step.umma_q0, step.n_umma, *common,
+                                  ops.attn_prefill_umma_splits(step.n_umma, self.heads, max_keys), tile_rows=step.umma_rows,
+                                  gate=gate)
+        elif step.n_chunk and fast:
             ops.attn_prefill_options_bf16(q, q.stride(0), out, *pages, step.chunk_entry, step.chunk_q0, step.n_chunk, *common,
                                           self.softcap, self.keep_first, self.sink, gate, **more)      # portions on tensor cores
         elif step.n_tiles:

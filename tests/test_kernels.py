@@ -842,3 +842,75 @@ def test_gemv_plan_depends_on_the_matrix_only(ops):
         assert 1 <= s <= 8 and s == ops.gemv_k_splits(n, k)
         assert s == 1 or (k + 31) // 32 // s >= 16
     assert ops.gemv_k_splits(48, 64) == 1
+
+
+@pytest.mark.parametrize("window", [0, 40, 200, -64, -100, -256, -1000])
+@pytest.mark.parametrize("entries", [[(0, 300)], [(250, 70), (0, 9), (95, 600)], [(1000, 129)]])
+def test_attn_prefill_umma_chunks_and_gate(ops, window, entries):
+    """Chunks and windows that begin anywhere within the tiles, a gate per head in slices, pages that were given back."""
+    nh, nkv, hd, ps = 6, 2, 128, 16
+    g = torch.Generator().manual_seed(len(entries) * 1000 + window)
+    width = max((c + n + ps - 1) // ps for c, n in entries)
+    pages = sum((c + n + ps - 1) // ps for c, n in entries)
+    pool = torch.randn((pages + 1, 1, 2, nkv, ps, hd), generator=g).bfloat16()
+    bt = torch.full((len(entries), width), -1, dtype=torch.int32)
+    perm, total = iter(torch.randperm(pages, generator=g).tolist()), sum(n for _, n in entries)
+    q = torch.randn((total, nh * hd), generator=g).bfloat16()
+    gate = torch.randn((2, total, nh + 2), generator=g)
+    first = lambda p: 0 if window == 0 else max(0, p - window + 1) if window > 0 else p - p % -window
+    want, row = torch.zeros((total, nh, hd), dtype=torch.float64), 0
+    starts, tiles = [], {256: [], 128: []}
+    for e, (c, n) in enumerate(entries):
+        ids = [next(perm) for _ in range((c + n + ps - 1) // ps)]
+        kv = pool[ids, 0].double().permute(1, 0, 3, 2, 4).reshape(2, -1, nkv, hd)[:, :c + n]
+        for i, p in enumerate(ids):
+            bt[e, i] = p if (i + 1) * ps > first(c) else -1
+        pos = torch.arange(c, c + n)
+        lo = torch.tensor([first(int(p)) for p in pos])
+        hidden = (torch.arange(c + n)[None, :] > pos[:, None]) | (torch.arange(c + n)[None, :] < lo[:, None])
+        for h in range(nh):
+            s = q[row:row + n, h * hd:(h + 1) * hd].double() @ kv[0, :, h // 3].T * hd ** -0.5
+            want[row:row + n, h] = torch.softmax(s.masked_fill(hidden, -math.inf), -1) @ kv[1, :, h // 3]
+        starts.append(row)
+        row += n
+        for rows in tiles:
+            tiles[rows] += [(e, q0) for q0 in range(0, n, rows)]
+    gated = want * torch.sigmoid(gate.sum(0)[:, :nh].double())[:, :, None]
+    it = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    poold, qd = pool.to(DEV), q.to(DEV)
+    meta = (it(starts), it([n for _, n in entries]), it([c for c, _ in entries]))
+    for rows, parts in ((256, (1, 3)), (128, (1, 2))):
+        te, tq = it([t[0] for t in tiles[rows]]), it([t[1] for t in tiles[rows]])
+        for splits in parts:
+            for gd, ref_out in ((None, want), (gate.to(DEV), gated)):
+                out = torch.full((total, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+                ops.attn_prefill_umma(qd, nh * hd, out, poold[0, 0, 0], poold[0, 0, 1], poold.stride(0), ps, bt.to(DEV), te, tq,
+                                      len(te), *meta, nh, nkv, hd, hd ** -0.5, window, splits, rows, gate=gd)
+                ops.check_device_errors(DEV)
+                _close(out, ref_out.reshape(total, -1), 1.5e-2, f"window {window}, tiles of {rows}, {splits} parts")
+
+
+@pytest.mark.parametrize("hidden", [4, 1024, 1028, 3584, 8192, 8196])
+@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+def test_add_group_rmsnorm_of_whole_rows(ops, hidden, odt):
+    """The kernel that keeps a row in registers, both of its widths and the sizes on either side of its limits: against 64
+    bits, and a row's result does not depend on how many others there are."""
+    n = 150
+    r, a, b = _rand((n, hidden), torch.float32, 61), _rand((2, n, hidden), torch.float32, 62), _rand((n, hidden), torch.float32, 63)
+    x, vec, w = _rand((n, hidden), torch.float32, 64), _rand((hidden,), torch.float32, 65), _rand((hidden,), torch.float32, 66)
+    want_r = r.double() + 0.5 * a.double().sum(0) + 2.0 * b.double() + x.double() + vec.double()
+    want = want_r / torch.sqrt((want_r * want_r).mean(-1, keepdim=True) + 1e-6) * w.double()
+    whole = None
+    for rows in (n, 148, 3):
+        res, out = r[:rows].clone(), torch.empty((rows, hidden), dtype=odt, device=DEV)
+        ops.add_group_rmsnorm(res, a[:, :rows].contiguous(), w, 1e-6, 1, out, None, 0.5, b[:rows].contiguous(), 2.0, x[:rows].contiguous(), vec)
+        _close(res, want_r[:rows].cpu(), 1e-6, "stream")
+        _close(out, want[:rows].cpu(), 2e-6 if odt == torch.float32 else 6e-3, "normed rows")
+        whole = out if whole is None else whole
+        assert torch.equal(out, whole[:rows])
+    pick = torch.tensor([7, 0, 149], dtype=torch.int32, device=DEV)
+    res, out = r.clone(), torch.empty((3, hidden), dtype=odt, device=DEV)
+    ops.add_group_rmsnorm(res, None, w, 1e-6, 1, out, pick)
+    alone = r[pick.long()].double()
+    _close(out, (alone / torch.sqrt((alone * alone).mean(-1, keepdim=True) + 1e-6) * w.double()).cpu(), 2e-6 if odt == torch.float32 else 6e-3, "picked rows")
+    assert torch.equal(res, r)
