@@ -9,7 +9,7 @@
 // (sa * left + sb * right): the weighted sum, the sum into the stream and the norm are one pass.  x (float32 rows) and
 // v (one float32 vector for all rows) are what joins the stream where a pass over a stretch of layers begins.
 //
-// One block per output row; the row lies in shared memory between the passes.  A part's squares are added by one
+// One block per output row; the row lies in shared memory between the passes (in registers where it is one part).  A part's squares are added by one
 // warp, lane by lane and then over the warp, or, where the row is one part, by the whole block, so the order of
 // additions depends on the part's length alone, never on what else is in the batch.  Source row = rows ? rows[blockIdx.x] : blockIdx.x; in that gather mode the stream is
 // left untouched.
@@ -124,6 +124,104 @@ __global__ void add_group_rmsnorm_kernel(float* __restrict__ residual, const TD*
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = Num<TO>::from_f(row_buf[i] * rstd[i / gs] * weight[i]);
 }
 
+// Whole rows (groups = 1) of float32 addends, everything on 16-byte boundaries, up to 8,192 wide: the row lies in registers.
+// Bound by memory with many rows: blocks of 256 threads, so that several rows of an SM are under way at once (2,048 rows of
+// 3,584 with a float32 addend 24 us; 43 by the kernel above, a block of 1,024 threads and the row in shared memory).  Few
+// rows are bound by the latency of one: up to 1,024 threads share it (WIDE).  Both add in the same order: the squares of a
+// group of four, then the groups 1,024 columns apart, then the 256 threads by warps.
+template <typename TO, int J, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? (J < 4 ? J : 4) * 256 : 256)
+add_row_rmsnorm_kernel(float* __restrict__ residual, const float* __restrict__ a, int a_parts, long long a_stride, float a_scale,
+                       const float* __restrict__ b, int b_parts, long long b_stride, float b_scale,
+                       const float* __restrict__ weight, float eps, TO* __restrict__ out, const int* __restrict__ rows, int hidden,
+                       int write_residual, const float* __restrict__ x, const float* __restrict__ vec) {
+  constexpr int JT = WIDE ? (J < 4 ? J : 4) : 1, VT = (J + JT - 1) / JT;
+  pdl_launch_dependents();
+  __shared__ float sq[WIDE ? J : 1][256];
+  __shared__ float red[8];
+  const int t = threadIdx.x & 255, jt = threadIdx.x >> 8, lane = threadIdx.x & 31;
+  const bool adds = a || b || x || vec;
+  float4 w[VT];
+#pragma unroll
+  for (int k = 0; k < VT; ++k) {            // a parameter: read before the kernel ahead has finished
+    const int j = jt + k * JT, i = 4 * (j * 256 + t);
+    w[k] = (out && j < J && i < hidden) ? __ldg(reinterpret_cast<const float4*>(weight + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_wait();
+  const size_t at = (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * hidden;
+  float4 v[VT];
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < VT; ++k) {
+    const int j = jt + k * JT, i = 4 * (j * 256 + t);
+    float e = 0.0f;
+    if (j < J && i < hidden) {
+      float4 r = *reinterpret_cast<const float4*>(residual + at + i);
+      if (adds) {
+        float4 sa = make_float4(0.f, 0.f, 0.f, 0.f), sb = sa;
+        for (int p = 0; a && p < a_parts; ++p) {
+          const float4 y = *reinterpret_cast<const float4*>(a + at + (size_t)p * a_stride + i);
+          sa.x += y.x; sa.y += y.y; sa.z += y.z; sa.w += y.w;
+        }
+        for (int p = 0; b && p < b_parts; ++p) {
+          const float4 y = *reinterpret_cast<const float4*>(b + at + (size_t)p * b_stride + i);
+          sb.x += y.x; sb.y += y.y; sb.z += y.z; sb.w += y.w;
+        }
+        r.x += fmaf(b_scale, sb.x, a_scale * sa.x); r.y += fmaf(b_scale, sb.y, a_scale * sa.y);
+        r.z += fmaf(b_scale, sb.z, a_scale * sa.z); r.w += fmaf(b_scale, sb.w, a_scale * sa.w);
+        if (x) {
+          const float4 y = *reinterpret_cast<const float4*>(x + at + i);
+          r.x += y.x; r.y += y.y; r.z += y.z; r.w += y.w;
+        }
+        if (vec) {
+          const float4 y = *reinterpret_cast<const float4*>(vec + i);
+          r.x += y.x; r.y += y.y; r.z += y.z; r.w += y.w;
+        }
+        if (write_residual) *reinterpret_cast<float4*>(residual + at + i) = r;
+      }
+      v[k] = r;
+      e = fmaf(r.w, r.w, fmaf(r.z, r.z, fmaf(r.y, r.y, r.x * r.x)));
+    }
+    if (WIDE) { if (j < J) sq[j][t] = e; }
+    else ss += e;
+  }
+  if (!out) return;
+  if (WIDE) {
+    __syncthreads();
+    if (jt == 0)
+#pragma unroll
+      for (int j = 0; j < J; ++j) ss += sq[j][t];
+  }
+  if (jt == 0) {
+    ss = warp_sum(ss);
+    if (lane == 0) red[t >> 5] = ss;
+  }
+  __syncthreads();
+  ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) ss += red[k];
+  const float rstd = 1.0f / sqrtf(ss / (float)hidden + eps);
+  TO* o = out + (size_t)blockIdx.x * hidden;
+#pragma unroll
+  for (int k = 0; k < VT; ++k) {
+    const int j = jt + k * JT, i = 4 * (j * 256 + t);
+    if (j < J && i < hidden)
+      GnOut4<TO>::store(o + i, make_float4(v[k].x * rstd * w[k].x, v[k].y * rstd * w[k].y, v[k].z * rstd * w[k].z, v[k].w * rstd * w[k].w));
+  }
+}
+
+template <typename TO, int J>
+int launch_row_norm(float* residual, const float* a, int a_parts, long long a_stride, float a_scale, const float* b, int b_parts,
+                    long long b_stride, float b_scale, const float* weight, float eps, TO* out, const int* rows, int n_rows, int hidden,
+                    int write_residual, const float* x, const float* vec_add, cudaStream_t stream) {
+  // up to a row an SM: nothing else could hide the latency of a narrow block
+  auto kern = n_rows <= 148 ? add_row_rmsnorm_kernel<TO, J, true> : add_row_rmsnorm_kernel<TO, J, false>;
+  const int threads = n_rows <= 148 ? (J < 4 ? J : 4) * 256 : 256;
+  const int rc = launch_pdl(kern, dim3(n_rows), dim3(threads), 0, stream, residual, a, a_parts, a_stride, a_scale, b, b_parts, b_stride,
+                            b_scale, weight, eps, out, rows, hidden, write_residual, x, vec_add);
+  return rc ? rc : IFX_LAUNCH_CHECK();
+}
+
 template <typename TD, typename TO>
 int launch_group_norm(float* residual, const void* a, int a_parts, long long a_stride, float a_scale, const void* b,
                       int b_parts, long long b_stride, float b_scale, const float* weight, float eps, int groups,
@@ -135,6 +233,12 @@ int launch_group_norm(float* residual, const void* a, int a_parts, long long a_s
   const bool vec = sizeof(TD) == 4 && hidden % 4 == 0 && (a_stride & 3) == 0 && (b_stride & 3) == 0 &&
                    (((uintptr_t)residual | (uintptr_t)a | (uintptr_t)b | (uintptr_t)weight | (uintptr_t)out | (uintptr_t)x |
                      (uintptr_t)vec_add) & 15) == 0;
+  if (vec && groups == 1 && hidden <= 8192) {
+#define IFX_ROW(J) case J: return launch_row_norm<TO, J>(residual, (const float*)a, a_parts, a_stride, a_scale, (const float*)b, b_parts, \
+                                                         b_stride, b_scale, weight, eps, (TO*)out, rows, n_rows, hidden, write_residual, x, vec_add, stream);
+    switch ((hidden + 1023) / 1024) { IFX_ROW(1) IFX_ROW(2) IFX_ROW(3) IFX_ROW(4) IFX_ROW(5) IFX_ROW(6) IFX_ROW(7) IFX_ROW(8) }
+#undef IFX_ROW
+  }
   auto kern = vec ? add_group_rmsnorm_kernel<TD, TO, true> : add_group_rmsnorm_kernel<TD, TO, false>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
