@@ -266,7 +266,7 @@ class WindowAttention(Part):
 
     def _umma(self, out: torch.Tensor) -> bool:
         """Whether prompt portions of a fast layer go to the tcgen05 kernel: heads of 128 and nothing that it does not know
-        (it knows windows, chunks and a gate per head).  2,048 tokens of the 7B sizes in chunks of 8,192: 47 us against 165 for
+        (it knows windows, chunks and a gate per head).  2,048 tokens of the 7B sizes in chunks of 8,192: 49 us against 165 for
         the mma.sync kernel."""
         return (self.dim == ops.UMMA_ATTENTION_HEAD_DIM and not (self.softcap or self.keep_first or self.sink or self.q_temp)
                 and self.toll is None and self.gate in (None, "heads") and out.data_ptr() % 16 == 0)
