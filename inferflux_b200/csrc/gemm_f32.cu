@@ -75,7 +75,7 @@ many_kernel(const float* __restrict__ A, const float* __restrict__ W, const floa
   float* As = f32_smem;                          // [2][MK][BM]
   float* Ws = f32_smem + 2 * MK * BM;            // [2][MK][BN]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;         // the blocks that share a tile of W run side by side
   const int k_begin = SPLIT ? min(K, (int)blockIdx.z * slice_len) : 0, k_end = SPLIT ? min(K, k_begin + slice_len) : K;
   const int mc = (lane >> 2) * 4, nc = warp * 32 + (lane & 3) * 4;
 
@@ -321,7 +321,7 @@ int few(bool vec, const float* A, const float* W, const float* bias, float* C, i
 template <bool SPLIT>
 int many(bool vec, const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
          int slices, cudaStream_t stream) {
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, slices);
+  const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, slices);
   size_t smem = (size_t)2 * MK * (BM + BN) * sizeof(float);
   if (SPLIT && smem < (size_t)BM * BN * sizeof(float)) smem = (size_t)BM * BN * sizeof(float);
   const int len = slice_length(K, slices);
