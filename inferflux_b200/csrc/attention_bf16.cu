@@ -60,82 +60,67 @@ __device__ __forceinline__ float fast_exp2(float x) {
 
 // A tile in shared memory: rows of HD bfloat16 = HD/8 chunks of 16 bytes; chunk c of
 // row r is stored at chunk (c ^ (r & 7)) so that ldmatrix reads are conflict-free.
-template <int HD>
-__device__ __forceinline__ bf16* tile_chunk(bf16* tile, int row, int chunk) {
-  return tile + row * HD + ((chunk ^ (row & 7)) << 3);
-}
 
-// Copy `n_rows` keys (or values) starting at absolute key index `key0` into a tile.
-// Rows outside [lo, hi) or in pages that were given back are zero-filled.
-template <int HD, int THREADS>
-__device__ __forceinline__ void load_kv_tile(bf16* tile, const bf16* base, const PagedKV& kv, const int* bt,
-                                             int key0, int n_rows, int lo, int hi, int tid) {
-  constexpr int CPR = HD / 8;
-  for (int idx = tid; idx < n_rows * CPR; idx += THREADS) {
-    const int r = idx / CPR, c = idx - r * CPR;
-    const int key = key0 + r;
-    bool ok = key >= lo && key < hi;
-    const bf16* src = base;
-    if (ok) {
-      const int page = bt[key >> kv.page_shift];
-      ok = page >= 0;
-      if (ok) src = base + (size_t)page * kv.page_stride + (size_t)(key & (kv.page_size - 1)) * HD + c * 8;
-    }
-    cp_async16(tile_chunk<HD>(tile, r, c), src, ok);
+// 16 bytes to shared memory, both addresses with a constant added in the instruction
+template <int SOFF, int GOFF> __device__ __forceinline__ void cp_async16_at(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0 + %2], [%1 + %3], 16;\n" ::"r"(dst), "l"(src), "n"(SOFF), "n"(GOFF));
+}
+// The copies of one lane for 16 rows of a page that lie behind one another; dst[i]: where its chunk of row i goes (the swizzle
+// of the rows repeats after eight)
+template <int HD, int RPI, int J> struct RowCopies {
+  static __device__ __forceinline__ void go(const unsigned (&k)[8 / RPI], unsigned v_ahead, const bf16* ks, const bf16* vs) {
+    RowCopies<HD, RPI, J - 1>::go(k, v_ahead, ks, vs);
+    constexpr int I = (J - 1) % (8 / RPI), S = (J - 1) / (8 / RPI) * 8 * HD * 2, G = (J - 1) * RPI * HD * 2;
+    cp_async16_at<S, G>(k[I], ks);
+    cp_async16_at<S, G>(k[I] + v_ahead, vs);
+  }
+};
+template <int HD, int RPI> struct RowCopies<HD, RPI, 0> {
+  static __device__ __forceinline__ void go(const unsigned (&)[8 / RPI], unsigned, const bf16*, const bf16*) {}
+};
+
+// Copy 64 keys and their values into two tiles with 128 threads.  Thread t brings the page of row t / 2 (negative: no such key,
+// the row is zero-filled); key0 is the absolute index of row 0, a multiple of 64.  A warp copies its own 16 rows, HD / 8 lanes
+// side by side on a row, so an instruction reads whole rows of 2 * HD bytes.  With pages of at least 16 tokens the 16 rows are
+// one piece of memory, and unless some of them do not exist (the ends of a sequence or window) a copy is one instruction.  The
+// kernels below have two warps a scheduler and are bound by how many instructions those go through: 64 requests of 500 to
+// 3,600 tokens (7B sizes) took 67 us a layer with two lanes a row and an address for every copy, 59 with whole rows.
+template <int HD>
+__device__ __forceinline__ void load_kv_tile64_paged(bf16* ktile, bf16* vtile, const bf16* kbase, const bf16* vbase,
+                                                     const PagedKV& kv, int page, int key0, int tid) {
+  constexpr int CPR = HD / 8, RPI = 32 / CPR;                    // chunks of a row, rows of an instruction
+  const int lane = tid & 31, row0 = (tid >> 5) * 16, c = lane % CPR, r_in = lane / CPR;
+  if (kv.page_size >= 16 && __all_sync(0xffffffffu, page >= 0)) {
+    const size_t off = (size_t)page * kv.page_stride + (size_t)(((key0 + row0) & (kv.page_size - 1)) + r_in) * HD + c * 8;
+    const unsigned k0 = (unsigned)__cvta_generic_to_shared(ktile + (row0 + r_in) * HD);
+    unsigned k[8 / RPI];
+#pragma unroll
+    for (int i = 0; i < 8 / RPI; ++i) k[i] = k0 + i * RPI * HD * 2 + ((c ^ (i * RPI + r_in)) << 4);
+    RowCopies<HD, RPI, 16 / RPI>::go(k, (unsigned)((vtile - ktile) * 2), kbase + off, vbase + off);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 16 / RPI; ++j) {
+    const int rl = j * RPI + r_in, r = row0 + rl;
+    const int pg = __shfl_sync(0xffffffffu, page, 2 * rl);
+    const bool ok = pg >= 0;
+    const size_t off = ok ? (size_t)pg * kv.page_stride + (size_t)((key0 + r) & (kv.page_size - 1)) * HD + c * 8 : 0;
+    const int at = r * HD + ((c ^ (r & 7)) << 3);
+    cp_async16(ktile + at, kbase + off, ok);
+    cp_async16(vtile + at, vbase + off, ok);
   }
 }
 
-// Copy 64 keys and their values (absolute key index key0 ..) into two tiles with 128 threads:
-// two threads per key, one block-table lookup per thread for both; a pair of lanes covers 32
-// contiguous bytes per instruction.  Rows outside [lo, hi) or in pages given back are zero-filled.
+// The same with the pages looked up here.  Rows outside [lo, hi) or in pages given back are zero-filled.
 // `bt` may point to a copy of the block table in shared memory that starts at logical block
 // `bt_first` (the copy removes a global load from the path between two tiles).
 template <int HD>
 __device__ __forceinline__ void load_kv_tile64(bf16* ktile, bf16* vtile, const bf16* kbase, const bf16* vbase,
                                                const PagedKV& kv, const int* bt, int key0, int lo, int hi, int tid,
                                                int bt_first = 0) {
-  constexpr int CPR = HD / 8;
-  const int r = tid >> 1, half = tid & 1;
-  const int key = key0 + r;
-  bool ok = key >= lo && key < hi;
-  size_t off = 0;
-  if (ok) {
-    const int page = bt[(key >> kv.page_shift) - bt_first];
-    ok = page >= 0;
-    if (ok) off = (size_t)page * kv.page_stride + (size_t)(key & (kv.page_size - 1)) * HD;
-  }
-  const bf16* ksrc = kbase + off;
-  const bf16* vsrc = vbase + off;
-  bf16* krow = ktile + r * HD;
-  bf16* vrow = vtile + r * HD;
-  const int sw = r & 7;
-#pragma unroll
-  for (int j = 0; j < CPR / 2; ++j) {
-    const int c = j * 2 + half;
-    cp_async16(krow + ((c ^ sw) << 3), ksrc + c * 8, ok);
-    cp_async16(vrow + ((c ^ sw) << 3), vsrc + c * 8, ok);
-  }
-}
-
-// The same with the row's page already looked up by the caller (page < 0: the row is zero-filled).
-template <int HD>
-__device__ __forceinline__ void load_kv_tile64_paged(bf16* ktile, bf16* vtile, const bf16* kbase, const bf16* vbase,
-                                                     const PagedKV& kv, int page, int key, int tid) {
-  constexpr int CPR = HD / 8;
-  const int r = tid >> 1, half = tid & 1;
-  const bool ok = page >= 0;
-  const size_t off = ok ? (size_t)page * kv.page_stride + (size_t)(key & (kv.page_size - 1)) * HD : 0;
-  const bf16* ksrc = kbase + off;
-  const bf16* vsrc = vbase + off;
-  bf16* krow = ktile + r * HD;
-  bf16* vrow = vtile + r * HD;
-  const int sw = r & 7;
-#pragma unroll
-  for (int j = 0; j < CPR / 2; ++j) {
-    const int c = j * 2 + half;
-    cp_async16(krow + ((c ^ sw) << 3), ksrc + c * 8, ok);
-    cp_async16(vrow + ((c ^ sw) << 3), vsrc + c * 8, ok);
-  }
+  const int key = key0 + (tid >> 1);
+  const int page = key >= lo && key < hi ? bt[(key >> kv.page_shift) - bt_first] : -1;
+  load_kv_tile64_paged<HD>(ktile, vtile, kbase, vbase, kv, page, key0, tid);
 }
 
 constexpr int BT_CACHE = 1024;      // block-table entries a block keeps in shared memory
@@ -920,7 +905,7 @@ attn_decode_even_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __
     const int kvh = ld.j / head_chunks;
     bf16* st = ring + (size_t)stage * 2 * BK * HD;
     load_kv_tile64_paged<HD>(st, st + BK * HD, (const bf16*)kv.k + (size_t)kvh * kv.head_stride,
-                             (const bf16*)kv.v + (size_t)kvh * kv.head_stride, kv, ld_page, (ld.tile0 + ld.t) * BK + (tid >> 1), tid);
+                             (const bf16*)kv.v + (size_t)kvh * kv.head_stride, kv, ld_page, (ld.tile0 + ld.t) * BK, tid);
     advance(ld);
     look_up();                                                 // the next tile's page: the load is under way until its copy starts
   };
