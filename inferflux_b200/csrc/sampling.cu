@@ -319,7 +319,8 @@ struct SampleShared {
   unsigned long long hist[2][SC_BINS];                  // the limbs put together; two buffers: one is read by the cluster
                                                         // while the next fills
   unsigned long long warp_tot[32];
-  unsigned long long part_base, part_total, bcast;      // what this block tells the others
+  unsigned long long part_total, bcast;                 // what this block tells the others; what lies above the chosen bin
+  int chosen;
   ArgPair best;
   ArgPair ascratch[32];
 };
@@ -363,54 +364,61 @@ __device__ __forceinline__ unsigned long long block_scan_incl_u64(unsigned long 
   __syncthreads();
   return v + warp_tot[warp];
 }
-__device__ __forceinline__ unsigned long long block_total_u64(unsigned long long v, unsigned long long* warp_tot) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = v;
-  __syncthreads();
-  unsigned long long t = warp_tot[threadIdx.x & 31];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  return t;
+// One weight into this level's histogram.
+template <bool COUNT>
+__device__ __forceinline__ void radix_add(SampleShared& sh, unsigned key, float v) {
+  if (COUNT) {
+    atomicAdd(&sh.limb[0][key], 1u);
+  } else {                                              // a slice has at most 51,200 entries: no limb's sum passes 2^32
+    const unsigned long long q = weight_fix(v);
+    const unsigned l0 = (unsigned)(q & 0x1FFFu), l1 = (unsigned)((q >> 13) & 0x1FFFu), l2 = (unsigned)(q >> 26);
+    if (l0) atomicAdd(&sh.limb[0][key], l0);
+    if (l1) atomicAdd(&sh.limb[1][key], l1);
+    if (l2) atomicAdd(&sh.limb[2][key], l2);            // most weights are below 2^-13
+  }
+}
+__device__ __forceinline__ void radix_clear(SampleShared& sh) {
+  sh.limb[0][threadIdx.x] = 0;
+  sh.limb[1][threadIdx.x] = 0;
+  sh.limb[2][threadIdx.x] = 0;
 }
 
-// The largest threshold T >= floor_bits such that the entries with bits >= T number (COUNT) or weigh (fixed
-// point) at least `target`; floor_bits if even that does not reach it.  w: this block's n weights.
+// f(w[i]) for this block's n weights, four neighbours a 16-byte read
+template <typename F> __device__ __forceinline__ void for_weights(const float* w, int n, F f) {
+  for (int i = 4 * threadIdx.x; i < (n & ~3); i += 4 * SC_THREADS) {
+    const float4 v = *reinterpret_cast<const float4*>(w + i);
+    f(v.x); f(v.y); f(v.z); f(v.w);
+  }
+  if ((int)threadIdx.x < (n & 3)) f(w[(n & ~3) + threadIdx.x]);
+}
+
+// The largest threshold T >= floor_bits such that the entries with bits >= T number (COUNT) or weigh (fixed point) at least
+// a target; floor_bits if even that does not reach it.  w: this block's n weights.  The target is `count` or, of masses, the
+// share p of all that the histogram's first level holds (the entries from floor_bits on).  The caller has cleared the limbs
+// and filled the first level (bits 20 to 29 as the key).
 template <bool COUNT>
-__device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, unsigned floor_bits,
-                                    unsigned long long target, int& buffer, int cl) {
-  const int tid = threadIdx.x;
+__device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, unsigned floor_bits, unsigned long long count, float p,
+                                    int& buffer, int cl) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned prefix = 0;                                  // the bits above the level's ten, once decided
-  unsigned long long above = 0;                         // count / mass of the entries above the prefix's range
+  unsigned long long above = 0, target = count;         // count / mass of the entries above the prefix's range
+#pragma unroll 1
   for (int lev = 0; lev < 3; ++lev) {
     const int shift = 20 - 10 * lev;
     unsigned long long* h = sh.hist[buffer & 1];
     ++buffer;
-    sh.limb[0][tid] = 0;
-    if (!COUNT) { sh.limb[1][tid] = 0; sh.limb[2][tid] = 0; }
-    __syncthreads();
-    for (int i = tid; i < n; i += SC_THREADS) {
-      const float v = w[i];
-      const unsigned b = __float_as_uint(v);
-      if (b >= floor_bits && (lev == 0 || (b >> (shift + 10)) == prefix)) {
-        const unsigned key = (b >> shift) & (SC_BINS - 1);
-        if (COUNT) {
-          atomicAdd(&sh.limb[0][key], 1u);
-        } else {                                        // a slice has at most 51,200 entries: no limb's sum passes 2^32
-          const unsigned long long q = weight_fix(v);
-          if (q) {
-            atomicAdd(&sh.limb[0][key], (unsigned)(q & 0x1FFFu));
-            atomicAdd(&sh.limb[1][key], (unsigned)((q >> 13) & 0x1FFFu));
-            atomicAdd(&sh.limb[2][key], (unsigned)(q >> 26));
-          }
-        }
-      }
+    if (lev > 0) {
+      for_weights(w, n, [&](float v) {
+        const unsigned b = __float_as_uint(v);
+        if ((b >> (shift + 10)) == prefix && b >= floor_bits) radix_add<COUNT>(sh, (b >> shift) & (SC_BINS - 1), v);
+      });
     }
     __syncthreads();
     h[tid] = COUNT ? (unsigned long long)sh.limb[0][tid]
                    : (unsigned long long)sh.limb[0][tid] + ((unsigned long long)sh.limb[1][tid] << 13) +
                          ((unsigned long long)sh.limb[2][tid] << 26);
+    radix_clear(sh);                                    // (every thread its own bins) for the next level
+    if (tid == 0) { sh.chosen = 0; sh.bcast = above; }
     cluster_sync_all();
     const int bin = SC_BINS - 1 - tid;                  // thread order = bins from the top
     unsigned long long part[SC_MAX_CL];
@@ -419,18 +427,40 @@ __device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, uns
     unsigned long long tot = 0;
 #pragma unroll
     for (int r = 0; r < SC_MAX_CL; ++r) tot += part[r];
-    const unsigned long long reach = block_scan_incl_u64(tot, sh.warp_tot) + above;    // entries in this bin and above it
-    const int n_reach = __syncthreads_count(reach >= target);                          // they are the last n_reach threads
-    const int chosen = n_reach > 0 ? n_reach - 1 : 0;
-    if (n_reach > 0 && n_reach < SC_BINS && tid == SC_BINS - n_reach - 1) sh.bcast = reach;   // the bins above the chosen one
+    unsigned long long reach = tot;                     // the entries in this bin and above it: within the warp, then what
+#pragma unroll                                          // the warps before hold
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, reach, o);
+      if (lane >= o) reach += t;
+    }
+    if (lane == 31) sh.warp_tot[warp] = reach;
     __syncthreads();
-    if (n_reach > 0 && n_reach < SC_BINS) above = sh.bcast;
-    prefix = (prefix << 10) | (unsigned)chosen;
-    __syncthreads();                                    // bcast is free again
+    const unsigned long long wt = sh.warp_tot[lane];
+    unsigned long long before = lane < warp ? wt : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (!COUNT && lev == 0) {
+      unsigned long long base = wt;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+      target = (unsigned long long)((double)p * (double)base);
+      if (target < 1) target = 1;
+    }
+    reach += before + above;
+    if (reach >= target && reach - tot < target) {      // one bin at most; none: the lowest, and nothing above it is let go
+      sh.chosen = bin;
+      sh.bcast = reach - tot;
+    }
+    __syncthreads();
+    above = sh.bcast;
+    prefix = (prefix << 10) | (unsigned)sh.chosen;
   }
   return prefix > floor_bits ? prefix : floor_bits;
 }
 
+// Bound by latency: a row goes through its blocks' shared memory a few times, with a barrier of the cluster between.  So the
+// first level of the first histogram is made while the weights are, the mass that top-p refers to is the histogram's own sum,
+// and the masses for the draw are added once, by the segments that the draw then looks into.
 __global__ void __launch_bounds__(SC_THREADS, 2)        // two blocks per SM: 32 registers a thread
 sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, const float* __restrict__ temperature,
                       const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
@@ -445,6 +475,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
   const int begin = min(vocab, rank * slice), n = min(vocab, begin + slice) - begin;
   const float* lg = logits + (size_t)row * row_stride + begin;
   // the slice into shared memory, and its best logit
+  radix_clear(sh);
   ArgPair best{-INFINITY, -1};
   if ((((uintptr_t)lg) & 15) == 0) {
     for (int i = tid * 4; i < n; i += SC_THREADS * 4) {
@@ -481,52 +512,60 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
   }
   const float inv_t = 1.0f / temp;
   const float mx = top.v * inv_t;
-  for (int i = tid; i < n; i += SC_THREADS) {
-    const float v = w_s[i];
-    w_s[i] = (v == v) ? expf(v * inv_t - mx) : 0.0f;    // in [0, 1], the maximum is exactly 1
+  const int k = top_k[row];
+  const float mp = min_p[row], p = top_p[row];
+  const bool by_count = k > 0 && k < vocab, by_mass = p > 0.0f && p < 1.0f;
+  const unsigned thr_min = mp > 0.0f ? __float_as_uint(fminf(mp, 1.0f)) : 0u;
+  auto weight = [&](float v) { return (v == v) ? expf(v * inv_t - mx) : 0.0f; };      // in [0, 1], the maximum is exactly 1
+  auto first_level = [&](float w) {
+    const unsigned b = __float_as_uint(w);
+    if (by_count) radix_add<true>(sh, (b >> 20) & (SC_BINS - 1), w);
+    else if (by_mass && b >= thr_min) radix_add<false>(sh, (b >> 20) & (SC_BINS - 1), w);
+  };
+  for (int i = 4 * tid; i < (n & ~3); i += 4 * SC_THREADS) {
+    float4 v = *reinterpret_cast<float4*>(w_s + i);
+    v = make_float4(weight(v.x), weight(v.y), weight(v.z), weight(v.w));
+    *reinterpret_cast<float4*>(w_s + i) = v;
+    if (by_count || by_mass) { first_level(v.x); first_level(v.y); first_level(v.z); first_level(v.w); }
+  }
+  if (tid < (n & 3)) {
+    const float w = weight(w_s[(n & ~3) + tid]);
+    w_s[(n & ~3) + tid] = w;
+    first_level(w);
   }
   __syncthreads();
   int buffer = 0;
   unsigned thr = 0u;                                    // keep entries with weight bits >= thr
-  const int k = top_k[row];
-  if (k > 0 && k < vocab) thr = radix_threshold<true>(sh, w_s, n, 0u, (unsigned long long)k, buffer, cl);
-  const float mp = min_p[row];
-  if (mp > 0.0f) thr = max(thr, __float_as_uint(fminf(mp, 1.0f)));
-  const float p = top_p[row];
-  if (p > 0.0f && p < 1.0f) {                           // the largest threshold whose kept mass is >= p of the mass kept so far
-    unsigned long long mine = 0;
-    for (int i = tid; i < n; i += SC_THREADS) { const float v = w_s[i]; if (__float_as_uint(v) >= thr) mine += weight_fix(v); }
-    mine = block_total_u64(mine, sh.warp_tot);
-    if (tid == 0) sh.part_base = mine;
-    cluster_sync_all();
-    unsigned long long base = 0;
-#pragma unroll
-    for (int r = 0; r < SC_MAX_CL; ++r) base += r < cl ? *cluster_peer(&sh.part_base, r) : 0ull;
-    unsigned long long need = (unsigned long long)((double)p * (double)base);
-    if (need < 1) need = 1;
-    thr = radix_threshold<false>(sh, w_s, n, thr, need, buffer, cl);
+  if (by_count) thr = radix_threshold<true>(sh, w_s, n, 0u, (unsigned long long)k, 0.0f, buffer, cl);
+  thr = max(thr, thr_min);
+  if (by_mass) {                                        // the largest threshold whose kept mass is >= p of the mass kept so far
+    if (by_count) {
+      for_weights(w_s, n, [&](float v) {
+        const unsigned b = __float_as_uint(v);
+        if (b >= thr) radix_add<false>(sh, (b >> 20) & (SC_BINS - 1), v);
+      });
+    }
+    thr = radix_threshold<false>(sh, w_s, n, thr, 0ull, p, buffer, cl);
   }
   // inverse CDF over the kept entries in index order: first the block that holds the target, then the thread, then the entry
-  unsigned long long mine = 0;
-  for (int i = tid; i < n; i += SC_THREADS) { const float v = w_s[i]; if (__float_as_uint(v) >= thr) mine += weight_fix(v); }
-  const unsigned long long block_total = block_total_u64(mine, sh.warp_tot);
-  if (tid == 0) sh.part_total = block_total;
+  const int seg = ((n + SC_THREADS - 1) / SC_THREADS) | 1;      // odd: the threads' entries lie in different banks
+  const int sb = min(n, tid * seg), se = min(n, sb + seg);
+  unsigned long long s = 0;
+  for (int i = sb; i < se; ++i) { const float v = w_s[i]; if (__float_as_uint(v) >= thr) s += weight_fix(v); }
+  const unsigned long long incl = block_scan_incl_u64(s, sh.warp_tot), before = incl - s;
+  if (tid == SC_THREADS - 1) sh.part_total = incl;
   cluster_sync_all();
-  unsigned long long total = 0, offset = 0;
+  unsigned long long total = 0, offset = 0, block_total = 0;
 #pragma unroll
   for (int r = 0; r < SC_MAX_CL; ++r) {
     const unsigned long long t = r < cl ? *cluster_peer(&sh.part_total, r) : 0ull;
     if (r < rank) offset += t;
+    if (r == rank) block_total = t;
     total += t;
   }
   const unsigned long long target = (unsigned long long)((double)uniform01(seeds[row], counters[row]) * (double)total);   // < total
   if (target >= offset && target - offset < block_total) {                    // block-uniform
     const unsigned long long local = target - offset;
-    const int seg = (n + SC_THREADS - 1) / SC_THREADS;
-    const int sb = min(n, tid * seg), se = min(n, sb + seg);
-    unsigned long long s = 0;
-    for (int i = sb; i < se; ++i) { const float v = w_s[i]; if (__float_as_uint(v) >= thr) s += weight_fix(v); }
-    const unsigned long long incl = block_scan_incl_u64(s, sh.warp_tot), before = incl - s;
     if (s > 0 && before <= local && local < incl) {     // exactly one thread
       unsigned long long run = before;
       int pick = se - 1;

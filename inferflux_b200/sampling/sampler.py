@@ -16,6 +16,7 @@ from __future__ import annotations
 
 from typing import Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..kernels import ops
@@ -117,12 +118,17 @@ class Sampler:
         r, dev = logits.shape[0], self.device
         if all(p.greedy for p in params):
             return ops.argmax(logits, out)
-        f = lambda vals, dt: torch.tensor(vals, dtype=dt).to(dev, non_blocking=True)
-        ops.sample(logits, self._scratch(r),
-                   f([p.temperature for p in params], torch.float32),
-                   f([p.top_k for p in params], torch.int32),
-                   f([p.top_p for p in params], torch.float32),
-                   f([p.min_p for p in params], torch.float32),
-                   f([s & 0x7FFFFFFFFFFFFFFF for s in seeds], torch.int64),
-                   f(list(counters), torch.int64), out)
+        # the rows' six numbers go to the device as one copy: 32 bytes a row, the 8-byte ones first
+        words = np.empty(4 * r, dtype=np.int64)
+        halves = words[2 * r:].view(np.int32)
+        words[:r] = [s & 0x7FFFFFFFFFFFFFFF for s in seeds]
+        words[r:2 * r] = counters
+        halves[:r].view(np.float32)[:] = [p.temperature for p in params]
+        halves[r:2 * r] = [p.top_k for p in params]
+        halves[2 * r:3 * r].view(np.float32)[:] = [p.top_p for p in params]
+        halves[3 * r:].view(np.float32)[:] = [p.min_p for p in params]
+        d = torch.from_numpy(words).to(dev, non_blocking=True)
+        d_ints, d_floats = d[2 * r:].view(torch.int32), d[2 * r:].view(torch.float32)
+        ops.sample(logits, self._scratch(r), d_floats[:r], d_ints[r:2 * r], d_floats[2 * r:3 * r], d_floats[3 * r:], d[:r],
+                   d[r:2 * r], out)
         return out
