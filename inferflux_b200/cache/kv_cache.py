@@ -178,7 +178,7 @@ class KVCacheStorage:
         import torch
         self.page_size = page_size
         self.needs = list(needs)
-        self.pools = []
+        self.pools, self._views = [], {}
         for need, n_runs, pages in zip(needs, runs_per_group, num_pages):
             # zeros, not empty: a masked key is multiplied by 0, which must not meet a NaN
             self.pools.append(torch.zeros((pages, n_runs, page_size * need.elements_per_token),
@@ -189,12 +189,15 @@ class KVCacheStorage:
         inside page 0}, and the number of elements between pages.  Page p's
         block lies ``p * stride`` elements further on."""
         import torch
-        pool, ps = self.pools[group], self.page_size
-        views, at = {}, pool[0, index].storage_offset()
-        for s in self.needs[group].streams:
-            views[s.name] = torch.as_strided(pool, (s.heads, ps, s.width), (ps * s.width, s.width, 1), at)
-            at += s.heads * ps * s.width
-        return views, pool.stride(0)
+        kept = self._views.get((group, index))              # the pools stay where they are: a run's views are made once
+        if kept is None:
+            pool, ps = self.pools[group], self.page_size
+            views, at = {}, pool[0, index].storage_offset()
+            for s in self.needs[group].streams:
+                views[s.name] = torch.as_strided(pool, (s.heads, ps, s.width), (ps * s.width, s.width, 1), at)
+                at += s.heads * ps * s.width
+            kept = self._views[(group, index)] = (views, pool.stride(0))
+        return kept
 
     def layer_views(self, group: int, index: int):
         """(keys of page 0, values of page 0, elements between pages) of one run

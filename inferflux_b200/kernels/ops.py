@@ -30,13 +30,17 @@ class KernelError(RuntimeError):
     pass
 
 
-_sigs_done = False
+_ready = None               # the library with its signatures set
 
 
 def _lib():
-    global _sigs_done
+    return _ready if _ready is not None else _load()
+
+
+def _load():
+    global _ready
     lib = library()
-    if not _sigs_done:
+    if _ready is None:
         lib.ifx_embed_gather.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p]
         lib.ifx_add_rmsnorm.argtypes = [c_void_p, c_void_p, c_int, c_int, c_ll, c_void_p, c_float, c_void_p,
                                         c_int, c_void_p, c_int, c_int, c_int, c_void_p]
@@ -248,7 +252,7 @@ def _lib():
                      "ifx_add_into", "ifx_add_rows_vector", "ifx_attn_latent_mma", "ifx_attn_latent_mma_plan",
                      "ifx_attn_latent_mma_max_rank", "ifx_gather_latents"):
             getattr(lib, name).restype = c_int
-        _sigs_done = True
+        _ready = lib
     return lib
 
 
@@ -274,8 +278,15 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr()
 
 
+# The current stream's handle as torch's own launchers ask for it: torch.cuda.current_stream() makes two Python objects and
+# looks the device up by name on the way, 6 us of the 24 that a launch cost.
+_raw_stream, _current_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _code(t: torch.Tensor) -> int:
@@ -574,10 +585,11 @@ _sm_counts = {}
 
 def sm_count(device) -> int:
     """SMs of the device (where a kernel's plan is made on the host)."""
-    key = torch.device(device).index or 0
-    if key not in _sm_counts:
-        _sm_counts[key] = int(torch.cuda.get_device_properties(key).multi_processor_count)
-    return _sm_counts[key]
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    n = _sm_counts.get(key)
+    if n is None:
+        n = _sm_counts[key] = int(torch.cuda.get_device_properties(key).multi_processor_count)
+    return n
 
 
 _error_flags = {}
@@ -585,10 +597,11 @@ _error_flags = {}
 
 def error_flag(device) -> torch.Tensor:
     """The device word that kernels with bounded waits set when a wait runs out."""
-    key = torch.device(device).index or 0
-    if key not in _error_flags:
-        _error_flags[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _error_flags[key]
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    flag = _error_flags.get(key)
+    if flag is None:
+        flag = _error_flags[key] = torch.zeros(1, dtype=torch.int32, device=device)
+    return flag
 
 
 def check_device_errors(device) -> None:
