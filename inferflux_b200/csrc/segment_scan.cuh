@@ -106,7 +106,7 @@ template <int VC, int NB> inline size_t carry_smem(int dim, bool solve, bool cha
 
 // NR: blocks of 128 state rows (1: dim up to 128, 2: up to 256).  NB: segments the ring holds.
 template <bool FIXED, bool SOLVE, bool CHANNEL, int VC, int NR, int NB>
-__global__ void __launch_bounds__(COMPUTE + HELPERS, 1)
+__global__ void __launch_bounds__(COMPUTE + HELPERS, SOLVE || NR > 1 ? 1 : 2)
 carry_kernel(Args p) {
   extern __shared__ __align__(16) float sm[];
   pdl_enter();
