@@ -170,8 +170,8 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
                          const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                          int page_size, int page_shift, UmmaMeta m, const int* __restrict__ tile_entry,
                          const int* __restrict__ tile_q0, int n_heads, int n_kv, float scale, int window,
-                         int* __restrict__ error_flag, float* __restrict__ part_o, float* __restrict__ part_ml, int n_splits,
-                         int tile_rows, HeadGate gate) {
+                         int* __restrict__ error_flag, float* __restrict__ part_o, float* __restrict__ part_ml, int max_splits,
+                         int tile_rows, HeadGate gate, int n_tiles, int whole) {
   // The kernel before this one (it rotates the queries and writes the new keys and values) is waited for only
   // where its results are first read or the scratch of an earlier launch first written; until then the block
   // reads the step's description, sets up its barriers and gets its tensor memory.
@@ -191,9 +191,13 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
   }
   const unsigned sq0 = sbase, sk0 = sq0 + 2 * SQ_BYTES, sv0 = sk0 + K_STAGES * SKV_BYTES;
   const int tid = threadIdx.x, warp = tid >> 5;
-  // tiles run last to first and heads fastest: the longest blocks (of every head) start first
-  const int tile = gridDim.y - 1 - blockIdx.y;
-  const int e = tile_entry[tile], q0 = tile_q0[tile], head = blockIdx.x;
+  // Units (a tile and a head) run from the last tile to the first and heads fastest: the longest (of every head) start first.
+  // The first `whole` take a block each, the others max_splits blocks, consecutive parts of their key tiles.
+  const int unit = (int)blockIdx.x < whole ? (int)blockIdx.x : whole + ((int)blockIdx.x - whole) / max_splits;
+  const int split = (int)blockIdx.x < whole ? 0 : ((int)blockIdx.x - whole) % max_splits;
+  const int n_splits = (int)blockIdx.x < whole ? 1 : max_splits;
+  const int tile = n_tiles - 1 - unit / n_heads, head = unit % n_heads;
+  const int e = tile_entry[tile], q0 = tile_q0[tile];
   const int rows_all = min(tile_rows, m.entry_q_len[e] - q0);       // tile_rows: 256, or 128 (every tile on both slots)
   if (rows_all <= 0) return;
   const int tok0 = m.entry_q_start[e] + q0;
@@ -203,14 +207,13 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
   const int rows0 = min(UM, rows_all), rows1 = rows_all - rows0;  // rows of the two slots (the second may have none)
   const int kend = pos0 + rows_all;                              // keys [.., kend) may be seen by the block's last row
   const int kfirst = first_visible(pos0, window);                // first key the block's first row may see
-  // gridDim.z > 1: the key tiles are cut into n_splits consecutive parts, one block each; the parts leave
-  // their unnormalised O and (maximum, sum) in scratch for the merge kernel.  Few query tiles over a long
-  // context (a short portion of a long prompt) would otherwise leave most of the GPU idle.
-  const int split = blockIdx.z;
+  // n_splits > 1: the key tiles are cut into that many consecutive parts, one block each; the parts leave their unnormalised
+  // O and (maximum, sum) in scratch for the merge kernel.  Few units over a long context (a short portion of a long prompt),
+  // or the few that remain after the last full round of the SMs, would otherwise leave most of the GPU idle.
   const int t_all0 = kfirst / UN, n_all = (kend - 1) / UN - t_all0 + 1;
   const int per_split = (n_all + n_splits - 1) / n_splits;
   const int t_begin = t_all0 + split * per_split, n_t = min(per_split, n_all - split * per_split);
-  const size_t part_row0 = (((size_t)tile * n_heads + head) * n_splits + split) * (2 * UM);
+  const size_t part_row0 = ((size_t)(unit - whole) * n_splits + split) * (2 * UM);      // (of a unit that is cut)
   if (n_t <= 0) {                                                // (block-uniform) nothing to do: a part that adds nothing
     pdl_wait();
     if (tid < rows_all) {
@@ -637,7 +640,7 @@ attn_prefill_umma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* _
   if (any_failed && tid == 0) atomicExch(error_flag, 1);
 }
 
-// The parts of a query tile's keys put together: block (head, tile, group of MERGE_ROWS rows), thread d takes
+// The parts of a unit's keys put together: block (unit that was cut, group of MERGE_ROWS rows), thread d takes
 // column d of the group's rows.  The (maximum, sum) pairs of the group go through shared memory, where one
 // thread a row turns them into each part's factor 2^(its maximum - the common maximum) and the row's 1 / sum;
 // then every thread loads its column of eight parts at a time before it adds them up (in the order of the
@@ -648,18 +651,19 @@ __global__ void __launch_bounds__(UD)
 attn_prefill_umma_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                bf16* __restrict__ out, long long out_stride, UmmaMeta m,
                                const int* __restrict__ tile_entry, const int* __restrict__ tile_q0, int n_heads, int n_splits,
-                               int tile_rows, HeadGate gate) {
+                               int tile_rows, HeadGate gate, int n_tiles, int whole) {
   pdl_launch_dependents();
   __shared__ float ml_s[MERGE_ROWS][MERGE_MAX_SPLITS][2];
   __shared__ float f_s[MERGE_ROWS][MERGE_MAX_SPLITS];
   __shared__ float inv_s[MERGE_ROWS];
-  const int head = blockIdx.x, tile = blockIdx.y, r0 = blockIdx.z * MERGE_ROWS, d = threadIdx.x;
+  const int unit = whole + blockIdx.x, r0 = blockIdx.y * MERGE_ROWS, d = threadIdx.x;
+  const int head = unit % n_heads, tile = n_tiles - 1 - unit / n_heads;
   const int e = tile_entry[tile], q0 = tile_q0[tile];               // (the step's description: there before any kernel)
   const int rows = min(tile_rows, m.entry_q_len[e] - q0);
   if (r0 >= rows) return;
   const int tok0 = m.entry_q_start[e] + q0;
   pdl_wait();                                                      // the parts are written
-  const size_t base = ((size_t)tile * n_heads + head) * n_splits * (2 * UM);
+  const size_t base = (size_t)blockIdx.x * n_splits * (2 * UM);
   for (int i = threadIdx.x; i < MERGE_ROWS * n_splits; i += UD) {
     const int rr = i / n_splits, sp = i - rr * n_splits;
     const float2 v = r0 + rr < rows ? *reinterpret_cast<const float2*>(part_ml + (base + (size_t)sp * (2 * UM) + r0 + rr) * 2)
@@ -725,24 +729,53 @@ int make_kv_map(CUtensorMap* map, const void* base, int head_dim, int page_size,
 }
 }  // namespace
 
-// Into how many parts the keys of the query tiles are best cut: 1 when the tiles alone fill the GPU, else as
-// many as give every block a place at once, each part at least 8 key tiles of 64.
-IFX_API int ifx_attn_prefill_umma_plan(int n_tiles, int n_heads, int max_key_tiles) {
-  if (n_tiles < 1 || n_heads < 1) return 1;
+namespace {
+// SMs: a block takes all 512 columns of an SM's tensor memory, so as many run at once
+int resident_blocks() {
   static int resident = 0;
   if (!resident) {
-    // one block per SM: a block takes all 512 columns of an SM's tensor memory
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return 1;
     resident = sms > 0 ? sms : 1;
   }
-  const long long blocks = (long long)n_tiles * n_heads;
-  int s = (int)(resident / blocks);
+  return resident;
+}
+// Of `units` (tiles x heads), how many are not cut when the others are: the full rounds of the SMs
+int whole_units(long long units) { return units > resident_blocks() ? (int)(units / resident_blocks() * resident_blocks()) : 0; }
+}  // namespace
+
+// Into how many parts the keys of the units (query tiles x heads) that do not fill a round of the SMs are best cut.  Fewer
+// units than SMs: as many parts as give every block a place at once, each at least 8 key tiles of 64.  More: those behind the
+// last full round, where the contexts are long (64 key tiles and on, 16 a part) and it shortens that round by a sixth or more:
+// with 28 heads and 8 tiles 148 units run whole and 76 remain, which in three parts take two thirds of a unit's time.  The
+// parts' results cost a write and a read of a unit's rows in float32.
+IFX_API int ifx_attn_prefill_umma_plan(int n_tiles, int n_heads, int max_key_tiles) {
+  if (n_tiles < 1 || n_heads < 1) return 1;
+  const int resident = resident_blocks();
+  const long long units = (long long)n_tiles * n_heads;
+  if (units > resident) {
+    const int rest = (int)(units % resident);
+    if (rest == 0 || max_key_tiles < 64) return 1;
+    int best = 1;
+    float best_cost = 1.0f - 1.0f / 6.0f;
+    for (int s = 2; s <= 6 && max_key_tiles / s >= 16; ++s) {
+      const float cost = (float)((rest * s + resident - 1) / resident) / (float)s + 0.04f * (float)(s - 1);
+      if (cost < best_cost) { best = s; best_cost = cost; }
+    }
+    return best;
+  }
+  int s = (int)(resident / units);
   if (s > max_key_tiles / 8) s = max_key_tiles / 8;
   if (s > 16) s = 16;
   return s < 1 ? 1 : s;
+}
+
+// How many of n_tiles x n_heads units ifx_attn_prefill_umma cuts when it is told n_splits > 1
+IFX_API int ifx_attn_prefill_umma_cut_units(int n_tiles, int n_heads) {
+  const long long units = (long long)n_tiles * n_heads;
+  return (int)(units - whole_units(units));
 }
 
 // Prompt portions, head_dim 128, query tiles of tile_rows = 256 or 128 tokens of one entry (tile_entry / tile_q0;
@@ -752,7 +785,7 @@ IFX_API int ifx_attn_prefill_umma_plan(int n_tiles, int n_heads, int max_key_til
 // wait inside the kernel ran out (the output is then invalid).  window as first_visible takes it (negative: chunks).
 // gate: null, or one float32 number a token and head in gate_parts slices to be added, the result is multiplied by the
 // sigmoid of their sum.  n_splits > 1: scratch part_o float32
-// [n_tiles * n_heads * n_splits * 256 * 128] (16-byte aligned) and part_ml float32 [n_tiles * n_heads * n_splits * 256 * 2].
+// [cut units * n_splits * 256 * 128] (16-byte aligned) and part_ml float32 [cut units * n_splits * 256 * 2].
 IFX_API int ifx_attn_prefill_umma(const void* q, long long q_stride, void* out, long long out_stride,
                                   void* k_layer, void* v_layer, long long page_stride, int page_size,
                                   const int* block_tables, int bt_stride, const int* tile_entry, const int* tile_q0,
@@ -780,12 +813,15 @@ IFX_API int ifx_attn_prefill_umma(const void* q, long long q_stride, void* out, 
   UmmaMeta m{block_tables, bt_stride, entry_q_start, entry_q_len, entry_ctx_start};
   cudaError_t e = cudaFuncSetAttribute(attn_prefill_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_UMMA);
   if (e != cudaSuccess) return (int)e;
-  ifx_rc = launch_pdl(attn_prefill_umma_kernel, dim3(n_heads, n_tiles, n_splits), dim3(U_THREADS), SMEM_UMMA, stream,
+  const long long units = (long long)n_heads * n_tiles;
+  if (units * n_splits > 0x7FFFFFFF) return IFX_ERR_UNSUPPORTED;
+  const int whole = n_splits > 1 ? whole_units(units) : (int)units, cut = (int)units - whole;
+  ifx_rc = launch_pdl(attn_prefill_umma_kernel, dim3(whole + cut * n_splits), dim3(U_THREADS), SMEM_UMMA, stream,
                       (const bf16*)q, q_stride, (bf16*)out, out_stride, map_k, map_v, page_size, page_shift, m,
-                      tile_entry, tile_q0, n_heads, n_kv, scale, window, error_flag, part_o, part_ml, n_splits, tile_rows, hg);
+                      tile_entry, tile_q0, n_heads, n_kv, scale, window, error_flag, part_o, part_ml, n_splits, tile_rows, hg, n_tiles, whole);
   if (!ifx_rc) ifx_rc = IFX_LAUNCH_CHECK();
-  if (ifx_rc || n_splits == 1) return ifx_rc;
-  ifx_rc = launch_pdl(attn_prefill_umma_merge_kernel, dim3(n_heads, n_tiles, tile_rows / MERGE_ROWS), dim3(UD), 0, stream, (const float*)part_o,
-                      (const float*)part_ml, (bf16*)out, out_stride, m, tile_entry, tile_q0, n_heads, n_splits, tile_rows, hg);
+  if (ifx_rc || cut == 0) return ifx_rc;
+  ifx_rc = launch_pdl(attn_prefill_umma_merge_kernel, dim3(cut, tile_rows / MERGE_ROWS), dim3(UD), 0, stream, (const float*)part_o,
+                      (const float*)part_ml, (bf16*)out, out_stride, m, tile_entry, tile_q0, n_heads, n_splits, tile_rows, hg, n_tiles, whole);
   return ifx_rc ? ifx_rc : IFX_LAUNCH_CHECK();
 }

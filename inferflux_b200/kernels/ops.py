@@ -95,6 +95,8 @@ def _load():
                                               c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_ll, c_int, c_void_p]
         lib.ifx_attn_prefill_umma_plan.argtypes = [c_int, c_int, c_int]
         lib.ifx_attn_prefill_umma_plan.restype = c_int
+        lib.ifx_attn_prefill_umma_cut_units.argtypes = [c_int, c_int]
+        lib.ifx_attn_prefill_umma_cut_units.restype = c_int
         lib.ifx_argmax.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p]
         lib.ifx_apply_penalties.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                             c_void_p, c_int, c_int, c_void_p]
@@ -693,9 +695,9 @@ def attn_prefill_umma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_layer
     accumulators (bfloat16, head_dim 128); query tiles of ``tile_rows`` = 256 or
     128 tokens listed by tile_entry / tile_q0 (a block takes a tile and a head;
     with 128 the tile's key tiles are dealt out to both halves of the block:
-    twice the blocks, for steps whose tiles of 256 would leave SMs idle).  With ``n_splits`` > 1 the keys of every tile are cut
-    into that many parts (see :func:`attn_prefill_umma_splits`), merged by a
-    second kernel.  A negative ``window`` = -c: a token sees its own chunk of c positions.  With ``gate`` (float32 sums
+    twice the blocks, for steps whose tiles of 256 would leave SMs idle).  With ``n_splits`` > 1 the keys of every
+    (tile, head), or where they are more than the SMs of those behind the last full round, are cut into that many parts (see
+    :func:`attn_prefill_umma_splits`), merged by a second kernel.  A negative ``window`` = -c: a token sees its own chunk of c positions.  With ``gate`` (float32 sums
     ``[N, >= heads]`` or slices of them) a head's result is multiplied by the sigmoid of its number.  A bounded wait that
     runs out sets the device error flag (see :func:`check_device_errors`)."""
     _need(q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and k_layer.dtype == torch.bfloat16,
@@ -712,7 +714,7 @@ def attn_prefill_umma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_layer
     part_o = part_ml = None
     global launch_count
     if n_splits > 1:
-        rows = n_tiles * n_heads * n_splits * UMMA_ATTENTION_TILE
+        rows = int(_lib().ifx_attn_prefill_umma_cut_units(n_tiles, n_heads)) * n_splits * UMMA_ATTENTION_TILE
         part_o = torch.empty(rows * head_dim, dtype=torch.float32, device=q.device)
         part_ml = torch.empty(rows * 2, dtype=torch.float32, device=q.device)
         launch_count += 1          # the merge kernel

@@ -890,6 +890,33 @@ def test_attn_prefill_umma_chunks_and_gate(ops, window, entries):
                 _close(out, ref_out.reshape(total, -1), 1.5e-2, f"window {window}, tiles of {rows}, {splits} parts")
 
 
+@pytest.mark.parametrize("window,ctx,n", [(0, 600, 1100), (500, 3, 1281), (-700, 600, 1100)])
+def test_attn_prefill_umma_cuts_the_last_round(ops, window, ctx, n):
+    """More (tile, head) units than SMs: those behind the last full round are cut into parts, and everything comes out as
+    with no unit cut (which the tests above hold against other implementations)."""
+    nh, nkv, hd, ps = 40, 8, 128, 16
+    g = torch.Generator().manual_seed(n + window)
+    pages = (ctx + n + ps - 1) // ps
+    pool = torch.randn((pages, 1, 2, nkv, ps, hd), generator=g).bfloat16().to(DEV)
+    q = torch.randn((n, nh * hd), generator=g).bfloat16().to(DEV)
+    it = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    bt, tq = it([torch.randperm(pages, generator=g).tolist()]), it(list(range(0, n, 256)))
+    gate = torch.randn((n, nh), generator=g).to(DEV)
+    outs = []
+    for splits in (1, 2, 3, 7):
+        out = torch.full((n, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.attn_prefill_umma(q, nh * hd, out, pool[0, 0, 0], pool[0, 0, 1], pool.stride(0), ps, bt, torch.zeros_like(tq), tq, len(tq),
+                              it([0]), it([n]), it([ctx]), nh, nkv, hd, hd ** -0.5, window, splits, gate=gate)
+        ops.check_device_errors(DEV)
+        outs.append(out)
+    units = len(tq) * nh
+    assert units > ops.sm_count(DEV)
+    for out in outs[1:]:
+        _close(out, outs[0].double().cpu(), 1e-2, "parts of the last round")      # two roundings to bfloat16, of sums in another order
+        first = (units % ops.sm_count(DEV)) // nh * 256                           # tiles ahead of the cut ones are the same bits
+        assert torch.equal(out[first + 256:], outs[0][first + 256:])
+
+
 @pytest.mark.parametrize("hidden", [4, 1024, 1028, 3584, 8192, 8196])
 @pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
 def test_add_group_rmsnorm_of_whole_rows(ops, hidden, odt):
