@@ -25,6 +25,9 @@
 // threads of both blocks.  The pair synchronises as a cluster after set-up and before it frees tensor
 // memory, so neither block leaves while the other may still signal it.
 //
+// The weights are parameters, which no kernel of a step writes: a block sets itself up and sends for the first stages'
+// weights before it waits for the kernel ahead of it in the stream; only what that kernel made is waited for.
+//
 // Every mbarrier wait is bounded: if one runs out the thread sets *error_flag and the block's abort
 // word, the other warps leave their loops, the block waits a moment for TMA copies in flight, and the
 // pair frees its tensor memory and returns.
@@ -106,6 +109,9 @@ constexpr int P_STAGES = 6;
 constexpr int P_HALF_BYTES = 128 * TK * 2;            // 16 KB: 128 rows of 128 bytes
 constexpr int P_STAGE_BYTES = 2 * P_HALF_BYTES;       // this block's rows of A, then its rows of W
 constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + 1024;
+// Modes 2 and 6 (few tokens): a stage is as small as the tile's rows and the tokens allow, and there are as many as fit.
+constexpr int S_MAX_STAGES = 12;
+constexpr int S_SMEM = 212 * 1024;                    // with 1 KB for alignment and 16 KB behind the last stage, which the MMA may read (see below)
 constexpr int P_THREADS = 192;                        // producer warp, MMA warp, 4 epilogue warps
 constexpr unsigned LEADER_MASK = 0xFEFFFFFFu;         // a shared-memory address of this block -> the same place in the pair's leader
 // kind::f16 instruction descriptor: D float32, A and B bfloat16, both K-major, M 256 (over the pair), N 256
@@ -169,33 +175,40 @@ struct QkvEpilogue {
 // change places, so that the 256 rows of a tile are rows of the weights and its (few) columns the tokens: the
 // kernel is given the weights as map_a (M = their rows) and the activations as map_w (n_out = the tokens, all
 // in one tile), K is cut into k_parts parts that are tiles of their own, and the epilogue writes each part's
-// sums transposed, as float32 [k_parts][tokens][ldo] part_stride elements apart, for the consumer to add.
+// sums transposed, as float32 [k_parts][tokens][ldo] part_stride elements apart, for the consumer to add.  Mode 6 is
+// the same with the stacked [gate; up] weights (M = the rows of one of them, K whole): a tile takes the same rows of both, each
+// into columns of its own (tokens up to 128), so a thread finds gate and up of an output in its lane, and writes bfloat16
+// silu(gate) * up.  In both a tile has tile_h <= 256 rows (a multiple of 16) of which each block loads half: the MMA still
+// works on 128 rows a block, and what the others hold is never read.
 template <int MODE, typename TOut>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       TOut* __restrict__ out, long long ldo, const float* __restrict__ bias, int M, int n_out, int K,
                       int tile_n, int* __restrict__ error_flag, int k_parts, long long part_stride, QkvEpilogue qe,
-                      const int* __restrict__ tile_expert, int expert_rows, GluShape glu) {
+                      const int* __restrict__ tile_expert, int expert_rows, GluShape glu, int tile_h, int n_stages) {
   // tile_expert (modes 0, 1, 4 and 5, or null): the rows of A are sorted by expert into groups of 256, tile_expert[i]
   // names the expert whose weights row tile i multiplies (its rows of W start at expert * expert_rows) or is
   // negative for a row tile that is not in use, which every role of the kernel skips.
-  constexpr bool SWIGLU = MODE == 1 || MODE == 5, SKINNY = MODE == 2, QKV = MODE == 3, RELU2 = MODE == 4;
-  pdl_enter();
+  constexpr bool SWIGLU = MODE == 1 || MODE == 5, SKINNY_GLU = MODE == 6, SKINNY = MODE == 2 || SKINNY_GLU,
+                 QKV = MODE == 3, RELU2 = MODE == 4;
+  constexpr int MAX_STAGES = SKINNY ? S_MAX_STAGES : P_STAGES;
+  pdl_launch_dependents();
   extern __shared__ unsigned char g_smem_raw[];
-  __shared__ __align__(8) unsigned long long bars[2 * P_STAGES + 4];    // full[s], empty[s], acc_full[2], acc_empty[2]
+  __shared__ __align__(8) unsigned long long bars[2 * MAX_STAGES + 4];  // full[s], empty[s], acc_full[2], acc_empty[2]
   __shared__ unsigned tmem_slot;
   __shared__ int abort_s;
   const unsigned sbase = (g_smem_addr(g_smem_raw) + 1023u) & ~1023u;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned rank = p_cluster_rank();
   const bool leader = rank == 0;
-  const unsigned bar_full = g_smem_addr(&bars[0]), bar_empty = g_smem_addr(&bars[P_STAGES]);
-  const unsigned bar_acc_full = g_smem_addr(&bars[2 * P_STAGES]), bar_acc_empty = g_smem_addr(&bars[2 * P_STAGES + 2]);
+  const unsigned bar_full = g_smem_addr(&bars[0]), bar_empty = g_smem_addr(&bars[MAX_STAGES]);
+  const unsigned bar_acc_full = g_smem_addr(&bars[2 * MAX_STAGES]), bar_acc_empty = g_smem_addr(&bars[2 * MAX_STAGES + 2]);
+  const int stages = SKINNY ? n_stages : P_STAGES;
   volatile int* abort_flag = &abort_s;
 
   if (tid == 0) {
     abort_s = 0;
-    for (int s = 0; s < P_STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_full + 8 * s));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_empty + 8 * s));
     }
@@ -218,41 +231,69 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
   // tile_n: accumulator columns of a tile (a multiple of 16 up to 256; SwiGLU: 256 = 128 gate + 128 up)
   const int out_cols = SWIGLU ? 128 : tile_n;
-  const int m_tiles = (M + 255) / 256, n_tiles = SKINNY ? k_parts : (n_out + out_cols - 1) / out_cols;
+  const int height = SKINNY ? tile_h : 256, half_h = height / 2;       // rows of a tile; of a block
+  const int m_tiles = (M + height - 1) / height, n_tiles = SKINNY ? k_parts : (n_out + out_cols - 1) / out_cols;
   const int tiles = m_tiles * n_tiles, k_steps = (K + TK - 1) / TK;
   const int part_steps = SKINNY ? (k_steps + k_parts - 1) / k_parts : k_steps;   // no part is empty: the host sees to that
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int w_half_rows = tile_n / 2;                            // rows of W this block loads per step
+  const int w_half_rows = tile_n / 2;                            // rows of map_w this block loads per step
+  // a stage: this block's rows of A (mode 6: of gate, then of up), then its rows of map_w
+  const int a_bytes = SKINNY ? half_h * 128 : P_HALF_BYTES, w_at = SKINNY_GLU ? 2 * a_bytes : a_bytes;
+  const int stage_bytes = SKINNY ? w_at + w_half_rows * 128 : P_STAGE_BYTES;
   bool gave_up = false;
 
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
+      int stage = 0, ahead = 0;                                  // ahead: stages of the first tile whose weights are on their way
       unsigned phase = 0;
+      auto expect = [&](int st) { if (leader) g_expect_tx(bar_full + 8 * st, 2 * (w_at + w_half_rows * 128)); };
+      auto load_a = [&](int st, int ks, int m0) {
+        const unsigned sa = sbase + st * stage_bytes, full = (bar_full + 8 * st) & LEADER_MASK;
+        p_tma_load(sa, &map_a, ks * TK, m0, full);
+        if (SKINNY_GLU) p_tma_load(sa + a_bytes, &map_a, ks * TK, M + m0, full);
+      };
+      auto load_w = [&](int st, int ks, int w_row) {
+        p_tma_load(sbase + st * stage_bytes + w_at, &map_w, ks * TK, w_row, (bar_full + 8 * st) & LEADER_MASK);
+      };
       for (int t = pair; t < tiles && !gave_up; t += n_pairs) {
-        int w_first = 0;
+        const int m0 = (t % m_tiles) * height + (int)rank * half_h;
+        const int n0 = SKINNY ? 0 : (t / m_tiles) * out_cols;
+        const int ks0 = SKINNY ? (t / m_tiles) * part_steps : 0, ks1 = SKINNY ? min(k_steps, ks0 + part_steps) : k_steps;
+        int w_row = SWIGLU ? (int)rank * n_out + n0 : n0 + (int)rank * w_half_rows;
+        if (t == pair) {
+          if (!tile_expert) {
+            ahead = min(stages, ks1 - ks0);
+            for (int i = 0; i < ahead; ++i) {
+              expect(i);
+              if (SKINNY) load_a(i, ks0 + i, m0);
+              else load_w(i, ks0 + i, w_row);
+            }
+          }
+          pdl_wait();
+        }
         if (tile_expert) {
           const int e = tile_expert[t % m_tiles];
           if (e < 0) continue;
-          w_first = e * expert_rows;
+          w_row += e * expert_rows;
         }
-        const int m0 = (t % m_tiles) * 256 + (int)rank * 128;
-        const int n0 = SKINNY ? 0 : (t / m_tiles) * out_cols;
-        const int w_row = w_first + (SWIGLU ? (int)rank * n_out + n0 : n0 + (int)rank * w_half_rows);
-        const int ks0 = SKINNY ? (t / m_tiles) * part_steps : 0, ks1 = SKINNY ? min(k_steps, ks0 + part_steps) : k_steps;
         for (int ks = ks0; ks < ks1; ++ks) {
-          if (!g_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { gave_up = true; break; }
-          const unsigned sa = sbase + stage * P_STAGE_BYTES, sw = sa + P_HALF_BYTES;
-          const unsigned full = (bar_full + 8 * stage) & LEADER_MASK;
-          if (leader) g_expect_tx(bar_full + 8 * stage, 2 * (P_HALF_BYTES + w_half_rows * 128));
-          p_tma_load(sa, &map_a, ks * TK, m0, full);
-          p_tma_load(sw, &map_w, ks * TK, w_row, full);
-          if (++stage == P_STAGES) { stage = 0; phase ^= 1u; }
+          if (ahead > 0) {                                       // the weights have been sent for
+            --ahead;
+            if (SKINNY) load_w(stage, ks, w_row);
+            else load_a(stage, ks, m0);
+          } else {
+            if (!g_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { gave_up = true; break; }
+            expect(stage);
+            load_a(stage, ks, m0);
+            load_w(stage, ks, w_row);
+          }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {
+      if (tile_expert) pdl_wait();
       int stage = 0, count = 0;
       unsigned phase = 0;
       const unsigned idesc = P_IDESC | ((unsigned)(tile_n >> 3) << 17);
@@ -268,18 +309,23 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         for (int ks = ks0; ks < ks1; ++ks) {
           if (!g_wait(bar_full + 8 * stage, phase, abort_flag)) { gave_up = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const unsigned sa = sbase + stage * P_STAGE_BYTES, sw = sa + P_HALF_BYTES;
+          const unsigned sa = sbase + stage * stage_bytes, sw = sa + w_at;
 #pragma unroll
-          for (int k = 0; k < TK / 16; ++k) p_mma(d, g_desc(sa + k * 32), g_desc(sw + k * 32), idesc, ks != ks0 || k != 0);
+          for (int k = 0; k < TK / 16; ++k) {
+            p_mma(d, g_desc(sa + k * 32), g_desc(sw + k * 32), idesc, ks != ks0 || k != 0);
+            if (SKINNY_GLU) p_mma(d + 128, g_desc(sa + a_bytes + k * 32), g_desc(sw + k * 32), idesc, ks != ks0 || k != 0);
+          }
           p_commit_both(bar_empty + 8 * stage);                  // both blocks' stage is free once these MMAs have read it
-          if (++stage == P_STAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
         if (!gave_up) p_commit_both(bar_acc_full + 8 * acc);
       }
     }
   } else {
     const int quarter = warp & 3;
-    const int row_in_tile = (int)rank * 128 + quarter * 32 + lane;
+    const int row_in_tile = (int)rank * half_h + quarter * 32 + lane;
+    const bool row_there = quarter * 32 + lane < half_h;         // (modes 2 and 6: tiles of fewer than 256 rows)
+    pdl_wait();
     const bool vec = (ldo * sizeof(TOut) % 16 == 0) && ((uintptr_t)out % 16 == 0);   // rows on 16-byte boundaries
     int count = 0;
     for (int t = pair; t < tiles; t += n_pairs) {
@@ -287,20 +333,34 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       const int acc = count & 1;
       const unsigned acc_parity = (unsigned)(count >> 1) & 1u;
       ++count;
-      const int m0 = (t % m_tiles) * 256, n0 = SKINNY ? 0 : (t / m_tiles) * out_cols;
+      const int m0 = (t % m_tiles) * height, n0 = SKINNY ? 0 : (t / m_tiles) * out_cols;
       if (!g_wait(bar_acc_full + 8 * acc, acc_parity, abort_flag)) { gave_up = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * 256);
       const int row = m0 + row_in_tile;
       TOut* orow = out + (size_t)(row < M ? row : 0) * (SKINNY ? 1 : ldo);
-      if (SKINNY) {                                              // this lane's row of the weights is a column of the output
+      if (SKINNY_GLU) {                                          // this lane's row of gate and up is a column of the output
+#pragma unroll 1
+        for (int c = 0; c * 32 < tile_n; ++c) {
+          float g[32], u[32];
+          if (tile_n - c * 32 >= 32) { g_tmem_ld32(taddr + c * 32, g); g_tmem_ld32(taddr + 128 + c * 32, u); }
+          else { g_tmem_ld16(taddr + c * 32, g); g_tmem_ld16(taddr + 128 + c * 32, u); }
+          if (row < M && row_there) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const int token = c * 32 + i;
+              if (token < n_out) orow[(size_t)token * ldo] = Num<TOut>::from_f(g[i] / (1.0f + __expf(-g[i])) * u[i]);
+            }
+          }
+        }
+      } else if (SKINNY) {                                       // this lane's row of the weights is a column of the output
         TOut* opart = orow + (size_t)(t / m_tiles) * part_stride;
 #pragma unroll 1
         for (int c = 0; c * 32 < tile_n; ++c) {
           float v[32];
           if (tile_n - c * 32 >= 32) g_tmem_ld32(taddr + c * 32, v);
           else g_tmem_ld16(taddr + c * 32, v);                   // warp-uniform: the tile's last 16 columns
-          if (row < M) {
+          if (row < M && row_there) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const int token = c * 32 + i;
@@ -497,7 +557,7 @@ int launch_gemm_pair(const void* A, long long lda, const void* W, const float* b
   const int tiles = ((M + 255) / 256) * ((n_out + out_cols - 1) / out_cols);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
   rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
-                          ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, (const int*)nullptr, 0, glu);
+                          ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, (const int*)nullptr, 0, glu, 256, P_STAGES);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
 
@@ -526,19 +586,33 @@ int launch_gemm_grouped(const void* A, long long lda, const void* W, void* out, 
   const int tiles = ((M + 255) / 256) * ((n_out + out_cols - 1) / out_cols);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
   rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
-                          ldo, (const float*)nullptr, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, tile_expert, expert_rows, glu);
+                          ldo, (const float*)nullptr, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, tile_expert, expert_rows, glu, 256, P_STAGES);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
 
-// Parts into which the product of a few rows cuts K: as many as give every pair of SMs a tile, each part at
-// least 8 steps of 64, none empty.
-int skinny_parts(int n_out, int K, int pairs) {
-  const int m_tiles = (n_out + 255) / 256, k_steps = (K + TK - 1) / TK;
-  int parts = pairs / m_tiles;
-  if (parts > k_steps / 8) parts = k_steps / 8;
-  if (parts < 1) parts = 1;
-  const int per = (k_steps + parts - 1) / parts;
-  return (k_steps + per - 1) / per;
+// How the product of a few rows is cut: rows of a tile (a multiple of 16) and parts of K (each at least 8 steps of 64, none
+// empty; `parts` > 0: that many).  A pair's time goes by what it reads of the weights and of the tokens, and every part costs
+// a write and a read of its sums, which measured like 16 bytes a sum: at 64 tokens of the 7B sizes four parts of the q, k, v
+// product's K with tiles of 256 rows and two with tiles of 128 read the same weights a pair, but the sums take 9.4 MB or 4.7.
+struct SkinnyPlan { int h, parts; };
+SkinnyPlan skinny_plan(int n_out, int K, int pairs, int tokens, int parts_wanted) {
+  const int k_steps = (K + TK - 1) / TK;
+  SkinnyPlan best{256, parts_wanted > 0 ? parts_wanted : 1};
+  long long best_cost = -1;
+  for (int h = 256; h >= 96; h -= 16) {
+    const int m_tiles = (n_out + h - 1) / h;
+    int most = parts_wanted > 0 ? parts_wanted : pairs / m_tiles;
+    if (parts_wanted <= 0 && most > k_steps / 8) most = k_steps / 8;
+    if (most < 1) most = 1;
+    for (int want = parts_wanted > 0 ? most : 1; want <= most; ++want) {
+      const int per = (k_steps + want - 1) / want, parts = (k_steps + per - 1) / per;
+      if (parts != want) continue;
+      const long long rounds = ((long long)m_tiles * parts + pairs - 1) / pairs;
+      const long long cost = rounds * per * (h + tokens) * 128 + (long long)(parts - 1) * tokens * n_out * 16 / pairs;
+      if (best_cost < 0 || cost < best_cost) { best = SkinnyPlan{h, parts}; best_cost = cost; }
+    }
+  }
+  return best;
 }
 
 int device_sms(int* sms) {
@@ -573,16 +647,18 @@ int launch_gemm_qkv(const void* A, long long lda, const void* W, const float* bi
   const int tiles = ((M + 255) / 256) * ((n_out + tile_n - 1) / tile_n);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
   rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, q_out,
-                          ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, qe, (const int*)nullptr, 0, GluShape{});
+                          ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, qe, (const int*)nullptr, 0, GluShape{}, 256, P_STAGES);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
 
-int launch_gemm_skinny(const void* X, long long ldx, const void* W, float* out, long long ldo, int tokens, int n_out, int K,
+template <int MODE, typename TOut>
+int launch_gemm_skinny(const void* X, long long ldx, const void* W, TOut* out, long long ldo, int tokens, int n_out, int K,
                        int k_parts, long long part_stride, int* error_flag, cudaStream_t stream) {
-  auto kern = gemm_umma_pair_kernel<2, float>;
+  constexpr bool GLU = MODE == 6;
+  auto kern = gemm_umma_pair_kernel<MODE, TOut>;
   static bool ready = false;
   if (!ready) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_SMEM);
     if (e != cudaSuccess) return (int)e;
     ready = true;
   }
@@ -590,14 +666,19 @@ int launch_gemm_skinny(const void* X, long long ldx, const void* W, float* out, 
   int rc = device_sms(&sms);
   if (rc) return rc;
   const int tile_n = tokens <= 32 ? 32 : (tokens + 15) / 16 * 16;      // the tokens, all in one tile
+  const SkinnyPlan plan = skinny_plan(n_out, K, sms / 2, tile_n, GLU ? 1 : k_parts);
+  const int stage_bytes = ((GLU ? 2 : 1) * plan.h / 2 + tile_n / 2) * 128;
+  int stages = (S_SMEM - 17 * 1024) / stage_bytes;
+  if (stages > S_MAX_STAGES) stages = S_MAX_STAGES;
   CUtensorMap map_w, map_x;
-  rc = make_map(&map_w, W, n_out, K, K, 128);
+  rc = make_map(&map_w, W, GLU ? 2ll * n_out : n_out, K, K, plan.h / 2);
   if (!rc) rc = make_map(&map_x, X, tokens, K, ldx, tile_n / 2);
   if (rc) return rc;
-  const int tiles = ((n_out + 255) / 256) * k_parts;
+  const int tiles = ((n_out + plan.h - 1) / plan.h) * plan.parts;
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_w, map_x, out, ldo,
-                          (const float*)nullptr, n_out, tokens, K, tile_n, error_flag, k_parts, part_stride, QkvEpilogue{}, (const int*)nullptr, 0, GluShape{});
+  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)S_SMEM, stream, dim3(2, 1, 1), map_w, map_x, out, ldo,
+                          (const float*)nullptr, n_out, tokens, K, tile_n, error_flag, plan.parts, part_stride, QkvEpilogue{},
+                          (const int*)nullptr, 0, GluShape{}, plan.h, stages);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
 }  // namespace
@@ -637,7 +718,17 @@ IFX_API int ifx_gemm_umma_skinny(const void* X, long long ldx, const void* W, fl
   const int k_steps = (K + TK - 1) / TK, per = (k_steps + k_parts - 1) / k_parts;
   if ((k_steps + per - 1) / per != k_parts) return IFX_ERR_UNSUPPORTED;            // a part would be empty
   if (((uintptr_t)X & 15) || ((uintptr_t)W & 15) || ((uintptr_t)out & 3)) return IFX_ERR_ALIGNMENT;
-  return launch_gemm_skinny(X, ldx, W, out, ldo, tokens, n_out, K, k_parts, part_stride, error_flag, stream);
+  return launch_gemm_skinny<2, float>(X, ldx, W, out, ldo, tokens, n_out, K, k_parts, part_stride, error_flag, stream);
+}
+
+// The same for a stacked [gate; up] weight W [2 * inter, K] and up to 128 tokens: out[tokens, inter] = silu(X gate^T) * (X
+// up^T) in bfloat16 (rows ldo elements apart), K in one piece.
+IFX_API int ifx_gemm_umma_skinny_glu(const void* X, long long ldx, const void* W, void* out, long long ldo, int tokens, int inter,
+                                     int K, int* error_flag, cudaStream_t stream) {
+  if (tokens <= 0 || inter <= 0) return 0;
+  if (tokens > 128 || K <= 0 || (K & 7) || (ldx & 7) || !error_flag) return IFX_ERR_UNSUPPORTED;
+  if (((uintptr_t)X & 15) || ((uintptr_t)W & 15) || ((uintptr_t)out & 1)) return IFX_ERR_ALIGNMENT;
+  return launch_gemm_skinny<6, bf16>(X, ldx, W, (bf16*)out, ldo, tokens, inter, K, 1, 0ll, error_flag, stream);
 }
 
 // Rows of A sorted by expert in groups of 256 (M a multiple of 256): out[row] = A[row] W_e^T with e =
@@ -663,11 +754,11 @@ IFX_API int ifx_gemm_umma_grouped(const void* A, long long lda, const void* W, v
   return IFX_ERR_UNSUPPORTED;
 }
 
-IFX_API int ifx_gemm_umma_skinny_parts(int n_out, int K) {
+IFX_API int ifx_gemm_umma_skinny_parts(int n_out, int K, int tokens) {
   int sms = 0;
   const int rc = device_sms(&sms);
   if (rc) return -rc;
-  return skinny_parts(n_out, K, sms / 2);
+  return skinny_plan(n_out, K, sms / 2, tokens <= 32 ? 32 : (tokens + 15) / 16 * 16, 0).parts;
 }
 
 // The stacked q, k, v projection of a step's tokens with everything that follows it before attention in its

@@ -80,10 +80,12 @@ def _load():
         lib.ifx_gemm_umma_skinny.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_int,
                                              c_void_p, c_void_p]
         lib.ifx_gemm_umma_skinny.restype = c_int
+        lib.ifx_gemm_umma_skinny_glu.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_void_p, c_void_p]
+        lib.ifx_gemm_umma_skinny_glu.restype = c_int
         lib.ifx_gemm_umma_qkv.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p,
                                           c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
         lib.ifx_gemm_umma_qkv.restype = c_int
-        lib.ifx_gemm_umma_skinny_parts.argtypes = [c_int, c_int]
+        lib.ifx_gemm_umma_skinny_parts.argtypes = [c_int, c_int, c_int]
         lib.ifx_gemm_umma_skinny_parts.restype = c_int
         lib.ifx_gemv_bf16_plan.argtypes = [c_int, c_int, c_int]
         lib.ifx_gemv_bf16_plan.restype = c_int
@@ -536,29 +538,31 @@ def gemm_umma_qkv(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
 SKINNY_MAX_ROWS = 256       # rows of x that gemm_umma_skinny takes
 
 
-def gemm_umma_skinny_parts(n: int, k: int) -> int:
-    """Into how many parts :func:`gemm_umma_skinny` cuts K for an [n, k] matrix."""
-    key = ("skinny", n, k)
-    if key not in _gemv_plans:
-        s = int(_lib().ifx_gemm_umma_skinny_parts(n, k))
+def gemm_umma_skinny_parts(n: int, k: int, rows: int = 64) -> int:
+    """Into how many parts :func:`gemm_umma_skinny` is best told to cut K for an [n, k] matrix and so many rows of x."""
+    key = ("skinny", n, k, (rows + 15) // 16)
+    s = _gemv_plans.get(key)
+    if s is None:
+        s = int(_lib().ifx_gemm_umma_skinny_parts(n, k, rows))
         if s < 1:
             raise KernelError(f"gemm_umma_skinny_parts: CUDA error {-s}")
         _gemv_plans[key] = s
-    return _gemv_plans[key]
+    return s
 
 
 def gemm_umma_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """Partial sums of x[M, K] @ w[N, K]^T for a few rows (up to
     SKINNY_MAX_ROWS), where the time goes to reading w once: out float32
-    [S, M, N], S = ``gemm_umma_skinny_parts(N, K)`` parts of K, to be added by
-    the consumer.  tcgen05 with the operands' places changed: 256 rows of w are
-    the rows of a tile and the rows of x its columns."""
+    [S, M, N], S parts of K (see :func:`gemm_umma_skinny_parts`), to be added by
+    the consumer.  tcgen05 with the operands' places changed: up to 256 rows of w are
+    the rows of a tile and the rows of x its columns.  ``w`` is a parameter: the kernel starts to read it before the kernel
+    launched before it has finished, so it must not be that kernel's output."""
     m, k = x.shape
     s, m2, n = out.shape
     _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous() and tuple(w.shape) == (n, k),
           "gemm_umma_skinny: bfloat16 x [M, K], w [N, K]")
-    _need(out.dtype == torch.float32 and out.is_contiguous() and m2 == m and 1 <= m <= SKINNY_MAX_ROWS
-          and s == gemm_umma_skinny_parts(n, k), "gemm_umma_skinny: out float32 [parts, M, N]")
+    _need(out.dtype == torch.float32 and out.is_contiguous() and m2 == m and 1 <= m <= SKINNY_MAX_ROWS,
+          "gemm_umma_skinny: out float32 [parts, M, N]")
     _need(k % 8 == 0 and x.stride(1) == 1 and (m == 1 or x.stride(0) % 8 == 0),
           "gemm_umma_skinny: K and the row stride of x must be multiples of 8")
     _check(_lib().ifx_gemm_umma_skinny(_ptr(x), x.stride(0) if m > 1 else k, _ptr(w), _ptr(out), n, m * n, m, n, k, s,
@@ -567,6 +571,21 @@ def gemm_umma_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> tor
 
 
 _gemv_plans = {}
+
+
+def gemm_umma_skinny_glu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out[M, I] = silu(x gate^T) * (x up^T) in bfloat16 for few rows (M <= 128) and w = [gate; up] [2I, K], which streams
+    through the tensor cores once.  ``w`` is a parameter: the kernel starts to read it before the kernel launched before it
+    has finished, so it must not be that kernel's output."""
+    m, k = x.shape
+    n = out.shape[-1]
+    _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape == (2 * n, k)
+          and out.dtype == torch.bfloat16, "gemm_umma_skinny_glu: bfloat16, w [2I, K]")
+    _need(out.dim() == 2 and out.shape[0] == m and out.stride(1) == 1 and x.stride(1) == 1, "gemm_umma_skinny_glu: out [M, I], unit inner strides")
+    _need(m <= 128 and k % 8 == 0 and (m == 1 or x.stride(0) % 8 == 0), "gemm_umma_skinny_glu: at most 128 rows, K and the row stride multiples of 8")
+    _check(_lib().ifx_gemm_umma_skinny_glu(_ptr(x), x.stride(0) if m > 1 else k, _ptr(w), _ptr(out), out.stride(0) if m > 1 else n,
+                                           m, n, k, _ptr(error_flag(x.device)), _stream()), "gemm_umma_skinny_glu")
+    return out
 
 
 def gemv_k_splits(n: int, k: int, max_splits: int = 8) -> int:

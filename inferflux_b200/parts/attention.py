@@ -204,7 +204,8 @@ class GQAttention(Part):
         # kernel below can add such up; rounded to bfloat16 first, the logits behind 2,048 tokens were off by
         # 2 % of the largest instead of 1.2 %)
         sums = 2 * cos.shape[1] == self.head_dim and self.head_dim % 16 == 0
-        qkv = self.qkv.forward(x, allow_partials=sums, f32_sums=sums)
+        launched = step.n_decode != n                  # (steps of single tokens run as captured graphs)
+        qkv = self.qkv.forward(x, allow_partials=sums, f32_sums=sums, launched=launched)
         if isinstance(qkv, PartialSums):
             partials = qkv.tensor
             qkv = torch.empty(partials.shape[1:], dtype=x.dtype, device=x.device)
@@ -215,12 +216,12 @@ class GQAttention(Part):
             # single tokens only: the attention kernel adds the bias, rotates and writes the cache itself
             self.decode(qkv, attn, ctx, step, g, k_layer, v_layer, page_stride,
                         prep=(self.qkv_bias, cos, sin, ctx.slot_maps[g], partials))
-            return self.o.forward(attn, out_dtype=x.dtype, allow_partials=True)
+            return self.o.forward(attn, out_dtype=x.dtype, allow_partials=True, launched=launched)
         ops.qkv_rope_kv_write(qkv, self.qkv_bias, cos, sin, ctx.slot_maps[g] if nkv_w else None,
                               k_layer if nkv_w else None, v_layer if nkv_w else None, page_stride,
                               ctx.page_size, self.n_heads, nkv_w, self.head_dim, partials)
         self.attend(qkv, attn, ctx, step, g, k_layer, v_layer, page_stride)
-        return self.o.forward(attn, out_dtype=x.dtype, allow_partials=True)
+        return self.o.forward(attn, out_dtype=x.dtype, allow_partials=True, launched=launched)
 
     def _fused_qkv(self, x: torch.Tensor, n: int, cos: torch.Tensor) -> bool:
         """Whether the step's q, k, v come from the tcgen05 product with bias,

@@ -20,9 +20,12 @@ from .base import PartialSums
 
 
 GEMV_ROWS = 8     # up to this many rows go to the weight-streaming kernel (it matches the library there)
-# From 9 to 128 rows a product is still bound by reading W once.  The tcgen05 kernel with the weights as the
-# tiles' rows beats the library there by a tenth when K is long (the down projection: 27 against 31 us at 64
-# rows); with a short K its set-up weighs more than it saves (qkv, o: 10 against 9 us), so those stay.
+# From 9 to 128 rows a product is still bound by reading W once: the tcgen05 kernel with the weights as the tiles' rows.  It
+# leaves float32 partial sums, so it serves consumers that add such up.  With a long K it beats the library by a quarter (the
+# down projection of the 7B sizes at 64 rows: 25 against 31 us).  With a short K the two take the same time (q, k, v at 64 rows
+# 9.3 against 9.0 us) and the sums cost the consumer 1 to 2 us, but a launch of the library costs the host more: a
+# prompt of 77 tokens (3B sizes, 8 layers), bound by its launches, takes 1,126 us with the kernel and 1,200 to 1,330 with the
+# library, a captured step of 64 single tokens (7B sizes, 6 layers) 1,210 and 1,158.
 FEW_ROWS, FEW_ROWS_MIN_K = 128, 8192
 
 
@@ -42,14 +45,15 @@ class Linear:
         self.bias = None if bias is None else bias.to(torch.float32).contiguous()
 
     def forward(self, x: torch.Tensor, out_dtype: Optional[torch.dtype] = None, allow_partials: bool = False,
-                f32_sums: bool = False):
+                f32_sums: bool = False, launched: bool = False):
         """x [M, in] -> [M, out] in ``out_dtype`` (default: x's type).  With
         ``allow_partials`` the result may be a :class:`PartialSums` (the
         weight-streaming kernel cuts K between blocks when a matrix has too few
         rows to fill the GPU).  With ``f32_sums`` on top of that, a bfloat16
         product always comes as float32 sums (one slice from the library): for
         a consumer that computes on with the sums, to which a rounding to
-        bfloat16 in between would only add error."""
+        bfloat16 in between would only add error.  ``launched``: the step's launches are the host's, not a graph's, so that
+        9 to 128 rows against a short K go to the kernel that is the cheaper one to launch."""
         m = x.shape[0]
         out_dtype = out_dtype or x.dtype
         w = self.weight
@@ -75,9 +79,9 @@ class Linear:
                 return PartialSums(ops.gemv_bf16(x, w, self.bias, y).unsqueeze(0))
             y = torch.empty((m, self.out_features), dtype=out_dtype, device=x.device)
             return ops.gemv_bf16(x, w, self.bias, y)
-        if (allow_partials and self.bias is None and m <= FEW_ROWS and self.in_features >= FEW_ROWS_MIN_K
-                and self.in_features % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0):
-            parts = ops.gemm_umma_skinny_parts(self.out_features, self.in_features)
+        if (allow_partials and self.bias is None and m <= FEW_ROWS and (launched or self.in_features >= FEW_ROWS_MIN_K)
+                and self.in_features % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
+            parts = ops.gemm_umma_skinny_parts(self.out_features, self.in_features, m)
             y = torch.empty((parts, m, self.out_features), dtype=torch.float32, device=x.device)
             return PartialSums(ops.gemm_umma_skinny(x, w, y))
         if allow_partials and f32_sums and self.bias is None:

@@ -834,6 +834,36 @@ def test_gemm_umma_skinny(ops, m, n, k):
     assert torch.equal(got[m // 2].float(), w[:, k // 3].float().cpu())
 
 
+@pytest.mark.parametrize("m,n,k", [(9, 2560, 2048), (33, 2048, 2048), (64, 4608, 3584), (100, 5120, 13824), (128, 112, 520)])
+def test_gemm_umma_skinny_any_parts(ops, m, n, k):
+    """Tiles of fewer than 256 rows, and every number of parts that leaves none empty."""
+    x, w = _rand((m, k), torch.bfloat16, 82), _rand((n, k), torch.bfloat16, 83, 0.1)
+    want, steps = x.double().cpu() @ w.double().cpu().T, (k + 63) // 64
+    for parts in sorted({1, 2, 3, ops.gemm_umma_skinny_parts(n, k, m)}):
+        if -(-steps // -(-steps // parts)) != parts:
+            continue
+        out = torch.full((parts, m, n), float("nan"), dtype=torch.float32, device=DEV)
+        ops.gemm_umma_skinny(x, w, out)
+        ops.check_device_errors(DEV)
+        # the tensor core adds K / 16 times into a float32 accumulator and drops what lies below its last place: at most a
+        # unit of 2^-23 of a partial sum each time, and no partial sum is far above the largest result
+        _close(out.double().sum(0).cpu(), want, max(1e-5, k / 16 * 2.0 ** -23), f"few-row product in {parts} parts")
+
+
+@pytest.mark.parametrize("m", [1, 9, 32, 33, 64, 100, 128])
+@pytest.mark.parametrize("inter,k", [(8, 64), (100, 72), (1000, 520), (2752, 2048), (13824, 512), (18944, 264)])
+def test_gemm_umma_skinny_glu(ops, m, inter, k):
+    """One tile and several a pair of SMs, tiles of few rows, K and the stacked halves that end inside a tile."""
+    x, w = _rand((m, k), torch.bfloat16, 58), _rand((2 * inter, k), torch.bfloat16, 59, 2.0 / math.sqrt(k))
+    out = torch.full((m + 1, inter), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_umma_skinny_glu(x, w, out[:m])
+    ops.check_device_errors(DEV)
+    gu = x.double().cpu() @ w.double().cpu().T
+    g, u = gu[:, :inter], gu[:, inter:]
+    _close(out[:m], g * torch.sigmoid(g) * u, 6e-3, "gemm_umma_skinny_glu")
+    assert bool((out[m] == 7.0).all())
+
+
 def test_gemv_plan_depends_on_the_matrix_only(ops):
     """The number of K parts is the kernel's own choice from the matrix sizes; it
     is within bounds, repeatable, and 1 where K is too short to cut."""
