@@ -339,7 +339,7 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], weight: t
             _need(tuple(delta.shape) == (n_partials, n, hidden), "add_rmsnorm: partials [P, N, H]")
             pstride = n * hidden
         else:
-            _need(tuple(delta.shape) == (n, hidden), "add_rmsnorm: delta [N, H]")
+            _need(tuple(delta.shape)[-2:] == (n, hidden) and delta.numel() == n * hidden, "add_rmsnorm: delta [N, H]")
     if out is not None:
         _need(out.is_contiguous() and tuple(out.shape) == (n_rows, hidden), "add_rmsnorm: out [rows, H]")
     dd = _code(delta) if delta is not None else F32

@@ -850,6 +850,18 @@ def test_gemm_umma_skinny_any_parts(ops, m, n, k):
         _close(out.double().sum(0).cpu(), want, max(1e-5, k / 16 * 2.0 ** -23), f"few-row product in {parts} parts")
 
 
+@pytest.mark.parametrize("m,n,k", [(16, 64, 64), (40, 96, 8192)])
+def test_few_row_products_into_the_norm(ops, m, n, k):
+    """Sums in one part (a short K) and in several, added by the norm that follows."""
+    from inferflux_b200.parts.linear import Linear
+    x, w = _rand((m, k), torch.bfloat16, 86), _rand((n, k), torch.bfloat16, 87, 0.1)
+    sums = Linear(w).forward(x, allow_partials=True, launched=True)
+    res, weight, out = torch.zeros((m, n), device=DEV), torch.ones(n, device=DEV), torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    ops.add_rmsnorm(res, sums.tensor, weight, 1e-6, out, None, sums.count)
+    ops.check_device_errors(DEV)
+    _close(res, x.double().cpu() @ w.double().cpu().T, max(1e-5, k / 16 * 2.0 ** -23), "few-row product and norm")
+
+
 @pytest.mark.parametrize("m", [1, 9, 32, 33, 64, 100, 128])
 @pytest.mark.parametrize("inter,k", [(8, 64), (100, 72), (1000, 520), (2752, 2048), (13824, 512), (18944, 264)])
 def test_gemm_umma_skinny_glu(ops, m, inter, k):
