@@ -19,8 +19,8 @@
 // rounded as fmaf is) leaves issue slots for the rest.  Tiles are stored K-major, columns
 // permuted so that neither the transposing stores nor the 16-byte reads meet on a bank; the
 // next tile is loaded into registers while the present one is multiplied.  301 rows: N 22,016
-// K 2,048 629 us (43 TFLOP/s; 64 x 64 blocks of 4 x 4 a thread 1,167), N 2,048 K 11,008
-// 425 us (2,116).
+// K 2,048 623 us (44 TFLOP/s; 64 x 64 blocks of 4 x 4 a thread 1,167), N 2,048 K 11,008
+// 373 us (2,116).
 //
 // Up to 16 rows (few_kernel): bound by reading W.  A thread owns one output column and
 // runs along its row of W, which arrives through a ring of cp.async copies.  One row
@@ -66,7 +66,7 @@ constexpr int BM = 64;
 // 128 threads, a warp as 8 x 4 lanes, the warps side by side along N: a lane has 2 groups of 4 rows, 32 apart, and 2
 // groups of 4 columns, 16 apart.
 template <bool VEC, bool SPLIT>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, SPLIT ? 4 : 3)       // four blocks an SM hide the short slices' first loads (2,048 x 11,008: 373 us, 418 with three)
 many_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
             int M, int N, int K, long long lda, long long ldc, int slice_len) {
   constexpr int WR = BN / 32;                                  // rows of W a thread loads
@@ -330,6 +330,8 @@ int many(bool vec, const float* A, const float* W, const float* bias, float* C, 
 }
 }  // namespace
 
+// A rows lda, C rows ldc elements apart, W contiguous, any K and alignment.  For up to 16 rows W is read before the kernel has
+// waited for the one launched before it (weights are parameters).
 IFX_API int ifx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                          long long lda, long long ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
