@@ -686,7 +686,8 @@ int launch_gemm_skinny(const void* X, long long ldx, const void* W, TOut* out, l
 // out[M, n_out] = A[M, K] * W^T (+ bias), W [n_out, K] contiguous; or, with act 1, W [2 * n_out, K] =
 // [gate; up] and out = silu(A gate^T) * (A up^T), or, with act 2, out = relu(A W^T)^2, or, with act 3, act 1's two halves through clamped_glu of (limit, alpha, shift) (both bfloat16 out).  A rows lda elements apart; K and lda multiples of 8;
 // A and W 16-byte aligned.  out_dtype: float32 or bfloat16.  error_flag: a device word set if a bounded
-// wait inside the kernel runs out.
+// wait inside the kernel runs out.  As in the products below, W is read before the kernel has waited for the one launched
+// before it, so it must not be the output of a kernel of this library launched directly before (weights are parameters).
 IFX_API int ifx_gemm_umma(const void* A, long long lda, const void* W, const float* bias, void* out, long long ldo,
                           int out_dtype, int M, int n_out, int K, int act, float limit, float alpha, float shift, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || n_out <= 0) return 0;

@@ -412,7 +412,8 @@ def qkv_rope_kv_write(qkv: torch.Tensor, bias: Optional[torch.Tensor], cos: torc
 
 # --------------------------------------------------------------- matrix product
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32, plain FFMA."""
+    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32, plain FFMA.  ``w`` is a parameter: for up to 16 rows it is read before
+    the kernel launched before this one has finished, so it must not be that kernel's output."""
     m, k = a.shape
     n = w.shape[0]
     _need(a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32, "gemm_f32: float32")
@@ -477,7 +478,8 @@ def gemm_umma(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     accumulation, bfloat16 or float32 result.  With ``swiglu`` w is [2N, K] =
     [gate; up] and out = silu(x gate^T) * (x up^T), the activation applied in the
     product's epilogue; with ``relu2`` (bfloat16 out) out = relu(x w^T)^2 likewise, with
-    ``glu`` = (limit, alpha, shift) (bfloat16 out) the stacked halves meet as in :func:`glu_clamped`.  Two SMs share each tile (cta_group::2).  A bounded wait
+    ``glu`` = (limit, alpha, shift) (bfloat16 out) the stacked halves meet as in :func:`glu_clamped`.  ``w`` is a
+    parameter: it is read before the kernel launched before this one has finished, so it must not be that kernel's output.  Two SMs share each tile (cta_group::2).  A bounded wait
     that runs out sets the device's error flag (see :func:`check_device_errors`)."""
     m, k = x.shape
     n = out.shape[-1]

@@ -27,6 +27,10 @@ GEMV_ROWS = 8     # up to this many rows go to the weight-streaming kernel (it m
 # prompt of 77 tokens (3B sizes, 8 layers), bound by its launches, takes 1,126 us with the kernel and 1,200 to 1,330 with the
 # library, a captured step of 64 single tokens (7B sizes, 6 layers) 1,210 and 1,158.
 FEW_ROWS, FEW_ROWS_MIN_K = 128, 8192
+# A vocabulary's float32 logits for 9 to 128 rows: the same kernel with K in one piece (152,064 x 3,584: 23 rows 164 us against
+# the library's 180, 64 rows 172 / 188, 128 rows 192 / 212; 151,936 x 2,048: 99 / 105 and 114 / 127; 152,064 x 5,120: 236 / 260
+# and 271 / 288).  At 32,768 columns the two are level, below the library is ahead (14,336: 21.7 / 20.1 at 64 rows).
+WIDE_COLUMNS = 65536
 
 
 def stack_rows(mats) -> torch.Tensor:
@@ -84,6 +88,11 @@ class Linear:
             parts = ops.gemm_umma_skinny_parts(self.out_features, self.in_features, m)
             y = torch.empty((parts, m, self.out_features), dtype=torch.float32, device=x.device)
             return PartialSums(ops.gemm_umma_skinny(x, w, y))
+        if (out_dtype == torch.float32 and self.bias is None and m <= FEW_ROWS and self.out_features >= WIDE_COLUMNS
+                and self.in_features % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
+            y = torch.empty((1, m, self.out_features), dtype=torch.float32, device=x.device)
+            y = ops.gemm_umma_skinny(x, w, y)
+            return PartialSums(y) if allow_partials and f32_sums else y[0]
         if allow_partials and f32_sums and self.bias is None:
             return PartialSums(ops.matmul_library(x, w, torch.float32).unsqueeze(0))
         y = ops.matmul_library(x, w, torch.float32 if (out_dtype == torch.float32 or self.bias is not None)

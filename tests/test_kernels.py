@@ -850,6 +850,17 @@ def test_gemm_umma_skinny_any_parts(ops, m, n, k):
         _close(out.double().sum(0).cpu(), want, max(1e-5, k / 16 * 2.0 ** -23), f"few-row product in {parts} parts")
 
 
+@pytest.mark.parametrize("m,n,k", [(9, 65536, 72), (77, 65560, 264), (128, 151936, 64), (129, 65536, 64), (8, 65536, 64), (64, 65528, 64)])
+def test_linear_wide_float32_logits(ops, m, n, k):
+    """A vocabulary's logits on either side of the rows and columns where the kernel changes."""
+    from inferflux_b200.parts.linear import Linear
+    x, w = _rand((m, k), torch.bfloat16, 84), _rand((n, k), torch.bfloat16, 85, 0.1)
+    out = Linear(w).forward(x, out_dtype=torch.float32)
+    ops.check_device_errors(DEV)
+    assert out.dtype == torch.float32 and tuple(out.shape) == (m, n)
+    _close(out, x.double().cpu() @ w.double().cpu().T, 1e-5, "wide float32 logits")
+
+
 @pytest.mark.parametrize("m,n,k", [(16, 64, 64), (40, 96, 8192)])
 def test_few_row_products_into_the_norm(ops, m, n, k):
     """Sums in one part (a short K) and in several, added by the norm that follows."""
