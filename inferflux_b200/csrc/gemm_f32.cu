@@ -4,8 +4,9 @@
 // only, runtime/backends/cuda/native/common/dtype_traits.cuh:13-30) and calls
 // cuBLAS with float32 accumulation for every projection
 // (runtime/backends/cuda/native/cublas_gemm.cpp:84-102).  These kernels use
-// plain float32 multiply-adds on CUDA cores, no tensor cores and no
-// reduced-precision mode.  How an output element is summed depends on N and K
+// plain float32 multiply-adds on CUDA cores, no reduced-precision mode; they take
+// matrices with fewer than 256 rows, a K below 256 or rows off the 16-byte
+// boundaries, the others go to gemm_f32_umma.cu.  How an output element is summed depends on N and K
 // only: K is cut into k_slices(N, K) slices, the products of a slice are added
 // in index order and the slices' sums in slice order, whatever M is and
 // whichever kernel runs, so a row's result does not depend on what else is in
@@ -28,6 +29,7 @@
 // runs along its row of W, which arrives through a ring of cp.async copies.  One row
 // against N 151,936 K 2,048: 205 us, 6.0 TB/s (1,406 us by 64 x 64 blocks).
 #include "common.cuh"
+#include "gemm_f32_umma.h"
 
 namespace {
 constexpr int BN = 128;
@@ -353,12 +355,15 @@ int many(bool vec, bool narrow, const float* A, const float* W, const float* bia
 }
 }  // namespace
 
-// A rows lda, C rows ldc elements apart, W contiguous, any K and alignment.  w_fixed: 1 = W is a parameter, which for up to 16
-// rows may be read before the kernel has waited for those ahead of it (see common.cuh on what that takes).
+// A rows lda, C rows ldc elements apart, W contiguous, any K and alignment.  w_fixed: 1 = W is a parameter, which may be read
+// before the kernel has waited for those ahead of it (see common.cuh on what that takes; here up to 16 rows, and the tensor
+// cores, use it).  scratch: 6 M ceil8(K) bytes, 16-byte aligned, used for more than 64 rows; may be null with fewer.
+// error_flag: a device word set if a bounded wait inside the kernel runs out.
 IFX_API int ifx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
-                         long long lda, long long ldc, int w_fixed, cudaStream_t stream) {
+                         long long lda, long long ldc, void* scratch, int w_fixed, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return IFX_ERR_UNSUPPORTED;
+  if (gemm_f32_umma_takes(W, N, K)) return gemm_f32_umma(A, W, bias, C, M, N, K, lda, ldc, scratch, w_fixed, error_flag, stream);
   const bool vec = (K % 4 == 0) && (((uintptr_t)W & 15) == 0);                       // of W's rows
   const bool vec_a = vec && (lda % 4 == 0) && (((uintptr_t)A & 15) == 0);
   if (M == 1) return few<1>(vec, A, W, bias, C, M, N, K, lda, ldc, w_fixed, stream);

@@ -1,0 +1,419 @@
+// float32 matrix product C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) on the tcgen05 tensor cores, for matrices that are not small.
+//
+// The tensor cores have no float32 operands.  A float32 number is the exact sum of three bfloat16 numbers, its 24 bits cut
+// into eights from the top (the exponent ranges are the same, so nothing overflows), and the product of two such numbers is
+// exact in float32.  Of the nine products of parts the six largest are taken; the three others together are below 2^-23 of
+// the product.  The tensor core rounds its running sum towards zero at each step of 16 along K, which over a long K would cost
+// more than plain float32 sums do.  So it sums 64 along K at a time, the small products first, and CUDA cores add these sums
+// up in registers, in order and rounded to nearest.  Error against 64 bits (2-norm over 2-norm, normal operands; in brackets the
+// fused multiply-adds in index order that gemm_f32.cu makes): K 256 1.3e-7 (2.9e-7), N 2,560 K 2,048 1.4e-7 (2.9e-7), N 22,016
+// K 2,048 1.6e-7 (8.1e-7), N 2,048 K 11,008 1.6e-7 (6.7e-7).
+//
+// How an output element is summed depends on N and K alone, as in gemm_f32.cu: K is cut into umma_slices(N, K) slices, a slice
+// into steps of 64, whatever M is and whichever tile width runs, so a row's result does not depend on what else is in
+// the batch.  A result that is not finite (an operand was not, or a sum overflowed on the way) is computed again by fused
+// multiply-adds in index order, so infinities and NaN come out as they do there.
+//
+// A block takes 128 rows of W, the tile's M rows of the MMA, and tile_n tokens, its N columns.  W arrives as float32 by TMA
+// (128-byte swizzle, K 64 a stage); a thread of eight warps reads half a row's 64 values, cuts them up with bit masks and
+// subtractions (exact) and writes the three parts into tensor memory, where the MMA takes its A operand from: the parts never go
+// back to shared memory, whose bandwidth the MMA's B operand (the tokens' three parts) needs.  Up to 64 tokens the same
+// threads cut the tokens' values up as well; for more, split_kernel has done it once for all blocks and TMA brings the parts.
+// Parts and sums are double-buffered: while the MMAs of one step run, the threads add the sums of the step before it and
+// cut up the values of the step behind it.
+//
+// What bounds it: six MMAs a product, so 2,250 / 6 = 375 TFLOP/s at most; with few tokens reading W.  301 rows: N 22,016 K 2,048
+// 155 us (623 by multiply-adds), N 2,048 K 11,008 106 us (373), N 2,560 K 2,048 44 us (94); 16 rows 49 us (111), 35 (76), 10 (17).
+#include "gemm_f32_umma.h"
+#include "umma.cuh"
+#include <float.h>
+
+namespace {
+
+constexpr int FK64 = 64;                        // K per step
+constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
+constexpr int U_WORKERS = 256, U_THREADS = U_WORKERS + 96;   // 8 warps of workers, a warp each for W's copies, the MMAs and the tokens' copies
+constexpr unsigned U_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // D float32, A and B bfloat16, K-major, M 128; N (in eighths) at bit 17
+
+__host__ __device__ constexpr int u_w_stages(int tn) { return tn == 16 ? 3 : tn <= 64 ? 5 : tn <= 128 ? 4 : 3; }
+__host__ __device__ constexpr int u_smem(int tn) { return u_w_stages(tn) * W_STAGE + 2 * 3 * tn * 128 + 1024; }
+__host__ __device__ constexpr int u_columns(int tn) { return tn <= 32 ? 256 : 512; }     // of tensor memory: 2 x 3 x 32 for W's parts, 2 x tn for sums
+
+__device__ __forceinline__ unsigned u_cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r)); return r; }
+__device__ __forceinline__ void u_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ float u_read_peer(unsigned saddr, int rank) {
+  unsigned ra;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(saddr), "r"(rank));
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+  return v;
+}
+// one arrival for the warp, once all its lanes have come here
+__device__ __forceinline__ void u_arrive_warp(unsigned bar, int lane) {
+  __syncwarp();
+  if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+
+// Two floats into their three bfloat16 parts each, packed (the first in the low half): x = hi + mid + lo exactly.
+__device__ __forceinline__ void cut(float x0, float x1, unsigned& hi, unsigned& mid, unsigned& lo) {
+  const unsigned a0 = __float_as_uint(x0), a1 = __float_as_uint(x1);
+  hi = __byte_perm(a0, a1, 0x7632);
+  const float r0 = x0 - __uint_as_float(a0 & 0xFFFF0000u), r1 = x1 - __uint_as_float(a1 & 0xFFFF0000u);
+  const unsigned b0 = __float_as_uint(r0), b1 = __float_as_uint(r1);
+  mid = __byte_perm(b0, b1, 0x7632);
+  const float s0 = r0 - __uint_as_float(b0 & 0xFFFF0000u), s1 = r1 - __uint_as_float(b1 & 0xFFFF0000u);
+  lo = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
+}
+
+__device__ __forceinline__ void u_tmem_st8(unsigned taddr, const unsigned (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void u_tmem_ld8(unsigned taddr, unsigned (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+__device__ __forceinline__ void u_mma(unsigned d, unsigned a_tmem, unsigned long long db, unsigned idesc, unsigned accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(d), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void u_commit(unsigned bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+
+// TN: token columns a block can hold.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W, slices of K), the slices of a tile a
+// cluster.  Up to TN 64 A is read here; above, map_x describes split_kernel's parts [3][M][K].
+template <int TN>
+__global__ void __launch_bounds__(U_THREADS, TN == 16 ? 2 : 1)
+gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ A,
+                     const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K, long long lda,
+                     long long ldc, int tile_n, int slice_steps, int vec_a, int w_fixed, int* __restrict__ error_flag) {
+  constexpr bool OWN_X = TN <= 64;
+  constexpr int STAGES = u_w_stages(TN), HALF = TN / 2, X_PER = OWN_X ? TN / 16 : 1;   // X_PER: float4 of the tokens a worker cuts up
+  extern __shared__ unsigned char u_smem_raw[];
+  __shared__ __align__(8) unsigned long long bars[2 * STAGES + 6];   // w_full[s], w_empty[s], x_full[2], parts_full[2], mma_done[2]
+  __shared__ unsigned tmem_slot;
+  __shared__ int abort_s;
+  const unsigned sbase = (g_smem_addr(u_smem_raw) + 1023u) & ~1023u, sx = sbase + STAGES * W_STAGE;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned w_full = g_smem_addr(&bars[0]), w_empty = g_smem_addr(&bars[STAGES]), x_full = g_smem_addr(&bars[2 * STAGES]);
+  const unsigned parts_full = x_full + 16, mma_done = x_full + 32;
+  volatile int* abort_flag = &abort_s;
+  if (tid == 0) {
+    abort_s = 0;
+    for (int s = 0; s < STAGES; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(w_full + 8 * s));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(w_empty + 8 * s), "r"(U_WORKERS / 32));
+    }
+    for (int b = 0; b < 2; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(x_full + 8 * b));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(parts_full + 8 * b), "r"(U_WORKERS / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mma_done + 8 * b));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(g_smem_addr(&tmem_slot)), "n"(u_columns(TN)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  pdl_launch_dependents();                       // behind the allocation: no block of the next kernel can be ahead of it at the tensor memory
+  const unsigned tmem = tmem_slot;
+  const int m0 = blockIdx.x * tile_n, n0 = blockIdx.y * 128;
+  const int steps_all = (K + FK64 - 1) / FK64, step0 = min(steps_all, (int)blockIdx.z * slice_steps);
+  const int steps = min(steps_all, step0 + slice_steps) - step0;
+  bool gave_up = false;
+  float acc[HALF];
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) acc[i] = 0.0f;
+  const int quarter = warp & 3, half = warp >> 2;                      // of a worker: its lanes of tensor memory, its half of K and of the columns
+
+  if (warp == 8) {                                                     // W's copies
+    if (lane == 0) {
+      if (!w_fixed) pdl_wait();
+      for (int c = 0; c < steps; ++c) {
+        const int st = c % STAGES;
+        if (c == STAGES) pdl_wait();                                   // (bounded waits begin when the kernel ahead has finished)
+        if (c >= STAGES && !g_wait(w_empty + 8 * st, (unsigned)((c / STAGES - 1) & 1), abort_flag)) { gave_up = true; break; }
+        g_expect_tx(w_full + 8 * st, W_STAGE);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+                       ::"r"(sbase + st * W_STAGE + h * (W_STAGE / 2)), "l"(&map_w), "r"((step0 + c) * FK64 + 32 * h), "r"(n0), "r"(w_full + 8 * st) : "memory");
+      }
+    }
+  } else if (warp == 10) {                                             // the tokens' copies
+    if (!OWN_X && lane == 0) {
+      pdl_wait();
+      for (int c = 0; c < steps; ++c) {
+        const int b = c & 1;
+        if (c >= 2 && !g_wait(mma_done + 8 * b, (unsigned)((c / 2 - 1) & 1), abort_flag)) { gave_up = true; break; }
+        g_expect_tx(x_full + 8 * b, 3 * tile_n * 128);
+        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
+                     ::"r"(sx + b * 3 * TN * 128), "l"(&map_x), "r"((step0 + c) * FK64), "r"(m0), "r"(0), "r"(x_full + 8 * b) : "memory");
+      }
+    }
+  } else if (warp == 9) {                                              // the MMAs
+    if (lane == 0) {
+      pdl_wait();
+      const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17);
+      for (int c = 0; c < steps; ++c) {
+        const int b = c & 1;
+        const unsigned par = (unsigned)((c >> 1) & 1);
+        if (!g_wait(parts_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
+        if (!OWN_X && !g_wait(x_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const unsigned d = tmem + 192 + b * TN, wp = tmem + b * 96, xp = sx + b * 3 * TN * 128;
+        // (W's part, the tokens' part), 0 the highest: the small products first
+        constexpr int order[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            u_mma(d, wp + order[p][0] * 32 + k * 8, g_desc(xp + order[p][1] * tile_n * 128 + k * 32), idesc, (p | k) != 0);
+        u_commit(mma_done + 8 * b);
+      }
+    }
+  } else {
+    const unsigned lanes = tmem + ((unsigned)(quarter * 32) << 16);
+    const int row = quarter * 32 + lane;
+    auto add_sums = [&](int c) {                                       // step c's sums into the registers
+      if (!__all_sync(0xffffffffu, g_wait(mma_done + 8 * (c & 1), (unsigned)((c >> 1) & 1), abort_flag))) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < HALF / 8; ++i) {
+        if (half * HALF + i * 8 >= tile_n) break;                      // (the same for the warp)
+        unsigned r[8];
+        u_tmem_ld8(lanes + 192 + (c & 1) * TN + half * HALF + i * 8, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i * 8 + j] += __uint_as_float(r[j]);
+      }
+      return true;
+    };
+    float4 xr[X_PER];                                                  // the tokens' values of the step ahead: 16 threads a row, four values each
+    auto load_x = [&](int c) {
+      const int k = (step0 + c) * FK64 + (tid & 15) * 4;
+#pragma unroll
+      for (int i = 0; i < X_PER; ++i) {
+        const int t = (tid >> 4) + 16 * i, m = m0 + t;
+        xr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < tile_n && m < M && k < K && c < steps) {               // K is a multiple of 4
+          const float* p = A + (size_t)m * lda + k;
+          xr[i] = vec_a ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+        }
+      }
+    };
+    if (OWN_X) { pdl_wait(); load_x(0); }
+    else if (!w_fixed) pdl_wait();                                     // (W's copies wait, too)
+    for (int c = 0; c < steps; ++c) {
+      const int b = c & 1, st = c % STAGES;
+      if (!OWN_X && c == 2) pdl_wait();
+      bool ok = c < 2 || add_sums(c - 2);                              // (and its parts' places are free)
+      ok = ok && g_wait(w_full + 8 * st, (unsigned)((c / STAGES) & 1), abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) { gave_up = true; break; }
+      const unsigned wrow = sbase + st * W_STAGE + half * (W_STAGE / 2) + row * 128;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {                                    // 16 values at a time
+        unsigned hi[8], mid[8], lo[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float x, y, z, w;
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(wrow + (((g * 4 + j) ^ (row & 7)) << 4)) : "memory");
+          cut(x, y, hi[2 * j], mid[2 * j], lo[2 * j]);
+          cut(z, w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
+        }
+        const unsigned at = lanes + b * 96 + half * 16 + g * 8;
+        u_tmem_st8(at, hi);
+        u_tmem_st8(at + 32, mid);
+        u_tmem_st8(at + 64, lo);
+      }
+      u_arrive_warp(w_empty + 8 * st, lane);
+      if (OWN_X) {
+#pragma unroll
+        for (int i = 0; i < X_PER; ++i) {
+          const int t = (tid >> 4) + 16 * i, q = tid & 15;
+          if (t >= tile_n) break;
+          unsigned h0, m0_, l0, h1, m1, l1;
+          cut(xr[i].x, xr[i].y, h0, m0_, l0);
+          cut(xr[i].z, xr[i].w, h1, m1, l1);
+          const unsigned to = sx + b * 3 * TN * 128 + t * 128 + (((q >> 1) ^ (t & 7)) << 4) + (q & 1) * 8;
+          asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(to), "r"(h0), "r"(h1) : "memory");
+          asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(to + tile_n * 128), "r"(m0_), "r"(m1) : "memory");
+          asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(to + 2 * tile_n * 128), "r"(l0), "r"(l1) : "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        load_x(c + 1);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      u_arrive_warp(parts_full + 8 * b, lane);
+    }
+    if (steps <= 2) pdl_wait();
+    for (int c = steps < 2 ? 0 : steps - 2; c < steps && !gave_up; ++c) gave_up = !add_sums(c);
+  }
+  if (gave_up) {                                                       // a wait ran out: tell everyone, let copies in flight land
+    atomicExch(error_flag, IFX_DEVICE_ERR_WAIT);
+    abort_s = 1;
+    __nanosleep(2000000);
+  }
+  // Every MMA has been waited for, every copy has landed: the ring's memory can take the slices' sums.
+  const int slices = gridDim.z;
+  auto put = [&](int m, int n, float v) {
+    if (!(fabsf(v) <= FLT_MAX)) {
+      const float *a = A + (size_t)m * lda, *w = W + (size_t)n * K;
+      v = 0.0f;
+#pragma unroll 1
+      for (int k = 0; k < K; ++k) v = fmaf(a[k], w[k], v);
+    }
+    C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.0f);
+  };
+  if (slices == 1) {
+    if (warp < 8) {
+      const int n = n0 + quarter * 32 + lane;
+      if (n < N)
+#pragma unroll
+        for (int i = 0; i < HALF; ++i) {
+          const int t = half * HALF + i;
+          if (t < tile_n && m0 + t < M) put(m0 + t, n, acc[i]);
+        }
+    }
+  } else {
+    __syncthreads();
+    if (warp < 8) {
+#pragma unroll
+      for (int i = 0; i < HALF; ++i) {
+        const int t = half * HALF + i;
+        if (t < tile_n) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sbase + (t * 128 + quarter * 32 + lane) * 4), "f"(acc[i]) : "memory");
+      }
+    }
+    u_cluster_sync();
+    const int rank = (int)u_cluster_rank();
+    if (warp < 8) {
+      const int n = n0 + (tid & 127);
+      for (int t = rank * 2 + (tid >> 7); t < tile_n && m0 + t < M; t += 2 * slices) {
+        float s = 0.0f;
+        for (int z = 0; z < slices; ++z) s += u_read_peer(sbase + (t * 128 + (tid & 127)) * 4, z);
+        if (n < N) put(m0 + t, n, s);
+      }
+    }
+    u_cluster_sync();                                                  // no block leaves while another still reads its sums
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(u_columns(TN)) : "memory");
+}
+
+// A's values cut into their parts [3][M][pitch] (zeros behind K), eight a thread.
+__global__ void __launch_bounds__(256)
+split_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, int K, long long lda, int pitch, int vec_a) {
+  pdl_enter();
+  const int groups = pitch / 8;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)M * groups) return;
+  const int m = (int)(i / groups), k = (int)(i % groups) * 8;
+  const float* p = A + (size_t)m * lda + k;
+  float4 v[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    v[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k + 4 * h < K) v[h] = vec_a ? *reinterpret_cast<const float4*>(p + 4 * h) : make_float4(p[4 * h], p[4 * h + 1], p[4 * h + 2], p[4 * h + 3]);
+  }
+  uint4 o[3];
+  cut(v[0].x, v[0].y, o[0].x, o[1].x, o[2].x);
+  cut(v[0].z, v[0].w, o[0].y, o[1].y, o[2].y);
+  cut(v[1].x, v[1].y, o[0].z, o[1].z, o[2].z);
+  cut(v[1].z, v[1].w, o[0].w, o[1].w, o[2].w);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) parts[(long long)q * M * groups + i] = o[q];
+}
+
+// Slices of K, from N and K alone (1, 2, 4 or 8): a narrow product's blocks fill the SMs, each slice at least 256 long.
+int umma_slices(int N, int K) {
+  const int rows = (N + 127) / 128;
+  int s = 1;
+  while (s < 8 && rows * s < 128 && K / (2 * s) >= 256) s *= 2;
+  return s;
+}
+
+struct TokenTiles { int tn, count; };
+// Tiles of tokens: as few rounds of blocks over the SMs as the widths allow.  A step's cycles go by its MMAs (6 a token) or by
+// the workers (cutting up W, adding sums, and up to 64 tokens cutting these up too); a block has some 4,000 of its own.
+TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
+  TokenTiles best{16, 1};
+  long long best_cost = -1;
+  const long long blocks = (long long)((N + 127) / 128) * slices;
+  for (int count = (M + 159) / 160; count <= (M + 15) / 16; ++count) {
+    const int tn = ((M + count - 1) / count + 15) / 16 * 16;
+    const long long per_sm = tn <= 16 ? 2 : 1, rounds = (blocks * count + sms * per_sm - 1) / (sms * per_sm);
+    const int workers = 600 + (tn <= 64 ? 7 : 3) * tn, mma = 6 * tn;
+    const long long cost = rounds * ((long long)steps * (workers > mma ? workers : mma) * per_sm + 4000);
+    if (best_cost < 0 || cost < best_cost) { best = TokenTiles{tn, count}; best_cost = cost; }
+  }
+  return best;
+}
+
+int u_sm_count(int* sms) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+  return (int)e;
+}
+
+template <int TN>
+int launch_umma_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
+                    int tn, int count, int slices, int steps, bool vec_a, void* scratch, int w_fixed, int* error_flag, cudaStream_t stream) {
+  auto kern = gemm_f32_umma_kernel<TN>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, u_smem(TN));
+  if (e != cudaSuccess) return (int)e;
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (!enc) return IFX_ERR_UNSUPPORTED;
+  CUtensorMap map_w, map_x = {};
+  {
+    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N};
+    cuuint64_t strides[1] = {(cuuint64_t)K * 4};
+    cuuint32_t box[2] = {32, 128}, estr[2] = {1, 1};
+    if (enc(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return IFX_ERR_UNSUPPORTED;
+  }
+  if (TN > 64) {
+    const int pitch = (K + 7) / 8 * 8;
+    cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)M, 3};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)M * pitch * 2};
+    cuuint32_t box[3] = {FK64, (cuuint32_t)tn, 3}, estr[3] = {1, 1, 1};
+    if (enc(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, scratch, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return IFX_ERR_UNSUPPORTED;
+    const long long items = (long long)M * (pitch / 8);
+    int rc = launch_pdl(split_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, A, (uint4*)scratch, M, K, lda, pitch, (int)vec_a);
+    if (rc) return rc;
+  }
+  const int rc = launch_pdl_cluster(kern, dim3(count, (N + 127) / 128, slices), dim3(U_THREADS), (size_t)u_smem(TN), stream, dim3(1, 1, slices),
+                                    map_w, map_x, A, W, bias, C, M, N, K, lda, ldc, tn, steps, (int)vec_a, w_fixed, error_flag);
+  return rc ? rc : IFX_LAUNCH_CHECK();
+}
+}  // namespace
+
+bool gemm_f32_umma_takes(const float* W, int N, int K) { return K % 4 == 0 && !((uintptr_t)W & 15) && N >= 256 && K >= 256; }
+
+int gemm_f32_umma(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
+                  void* scratch, int w_fixed, int* error_flag, cudaStream_t stream) {
+  if (!error_flag) return IFX_ERR_UNSUPPORTED;
+  if (M > 64 && (!scratch || ((uintptr_t)scratch & 15))) return IFX_ERR_ALIGNMENT;
+  int sms = 0;
+  const int rc = u_sm_count(&sms);
+  if (rc) return rc;
+  const int slices = umma_slices(N, K), steps_all = (K + FK64 - 1) / FK64, steps = (steps_all + slices - 1) / slices;
+  const TokenTiles t = token_tiles(M, N, slices, steps, sms);
+  const bool vec_a = lda % 4 == 0 && !((uintptr_t)A & 15);
+#define IFX_TILE(TN) launch_umma_f32<TN>(A, W, bias, C, M, N, K, lda, ldc, t.tn, t.count, slices, steps, vec_a, scratch, w_fixed, error_flag, stream)
+  return t.tn <= 16 ? IFX_TILE(16) : t.tn <= 32 ? IFX_TILE(32) : t.tn <= 64 ? IFX_TILE(64) : t.tn <= 96 ? IFX_TILE(96) : t.tn <= 128 ? IFX_TILE(128) : IFX_TILE(160);
+#undef IFX_TILE
+}

@@ -32,40 +32,12 @@
 // Every mbarrier wait is bounded: if one runs out the thread sets *error_flag and the block's abort
 // word, the other warps leave their loops, the block waits a moment for TMA copies in flight, and the
 // pair frees its tensor memory and returns.
-#include "common.cuh"
-#include <cuda.h>
-#include <cudaTypedefs.h>
+#include "umma.cuh"
 
 namespace {
 
 constexpr int TK = 64;                  // K per stage: one 128-byte swizzled row of bfloat16
-constexpr int G_WAIT_LIMIT = 1 << 20;   // tries of at most 2 microseconds each
 
-__device__ __forceinline__ unsigned g_smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// false: the wait ran out, or (abort_flag given) another warp of the block gave up
-__device__ __forceinline__ bool g_wait(unsigned bar, unsigned parity, const volatile int* abort_flag) {
-  for (int i = 0; i < G_WAIT_LIMIT; ++i) {
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");   // a try sleeps 2 microseconds at most
-    if (ok) return true;
-    if (abort_flag && (i & 255) == 255 && *abort_flag) return false;
-  }
-  return false;
-}
-__device__ __forceinline__ void g_expect_tx(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ unsigned long long g_desc(unsigned saddr) {      // K-major, 128-byte swizzle, 8-row groups of 1024 bytes
-  unsigned long long d = 0;
-  d |= (unsigned long long)((saddr & 0x3FFFF) >> 4);
-  d |= (unsigned long long)(16 >> 4) << 16;
-  d |= (unsigned long long)(1024 >> 4) << 32;
-  d |= 1ull << 46;
-  d |= 2ull << 61;
-  return d;
-}
 __device__ __forceinline__ void g_tmem_ld32(unsigned taddr, float (&v)[32]) {
   unsigned r[32];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
@@ -493,18 +465,6 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   __syncthreads();
   p_cluster_sync();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
-  return fn;
 }
 
 // [rows, K] bfloat16, row stride ld elements; boxes of box_rows rows x 64 elements, 128-byte swizzle, zeros outside

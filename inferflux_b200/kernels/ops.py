@@ -51,7 +51,7 @@ def _load():
         lib.ifx_qkv_rope_kv_write.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                               c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                               c_int, c_void_p]
-        lib.ifx_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p]
+        lib.ifx_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_void_p, c_int, c_void_p, c_void_p]
         lib.ifx_attn_paged_generic.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_int,
                                                c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p]
@@ -416,7 +416,9 @@ def qkv_rope_kv_write(qkv: torch.Tensor, bias: Optional[torch.Tensor], cos: torc
 # before it has waited itself); a copy, a kernel of torch or a synchronisation after the write settles it.  Without the flag
 # ``w`` may be anything, the output of the kernel just before included.
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, w_fixed: bool = False) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32, plain FFMA (``w_fixed``: see above; up to 16 rows use it)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32 and to float32's precision: exact thirds of the operands on the
+    tensor cores, or plain FFMA for small matrices (``w_fixed``: see above).  A bounded wait that runs out sets the device's
+    error flag (see :func:`check_device_errors`)."""
     m, k = a.shape
     n = w.shape[0]
     _need(a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32, "gemm_f32: float32")
@@ -424,8 +426,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     _need(a.stride(1) == 1 and out.stride(1) == 1, "gemm_f32: unit inner strides")
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm_f32: bias float32 [N]")
+    scratch = torch.empty((6 * m * ((k + 7) // 8 * 8),), dtype=torch.uint8, device=a.device) if m > 64 and k % 4 == 0 else None
     _check(_lib().ifx_gemm_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0) if m > 1 else k,
-                               out.stride(0) if m > 1 else n, w_fixed, _stream()), "gemm_f32")
+                               out.stride(0) if m > 1 else n, _ptr(scratch), w_fixed, error_flag(a.device).data_ptr(), _stream()), "gemm_f32")
     return out
 
 
