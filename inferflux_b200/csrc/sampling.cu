@@ -313,14 +313,16 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, float* __r
 // nor on how many blocks share the row.
 constexpr int SC_THREADS = 1024, SC_BINS = 1024, SC_MAX_CL = 8;
 constexpr int SC_MAX_SLICE = 51200;                     // floats of a row one block keeps (200 KB)
+constexpr int SC_LIST = 1024;                           // weights that a block can note down for the later levels, behind its slice
 
 struct SampleShared {
-  unsigned limb[3][SC_BINS];                            // counts, or masses in three 13-bit limbs: 32-bit shared-memory adds
+  unsigned limb[3][SC_BINS];                            // counts, or masses in three 16-bit limbs: 32-bit shared-memory adds
   unsigned long long hist[2][SC_BINS];                  // the limbs put together; two buffers: one is read by the cluster
                                                         // while the next fills
   unsigned long long warp_tot[32];
   unsigned long long part_total, bcast;                 // what this block tells the others; what lies above the chosen bin
   int chosen;
+  int listed;                                           // weights noted; more than there is room for: they did not fit
   ArgPair best;
   ArgPair ascratch[32];
 };
@@ -371,10 +373,10 @@ __device__ __forceinline__ void radix_add(SampleShared& sh, unsigned key, float 
     atomicAdd(&sh.limb[0][key], 1u);
   } else {                                              // a slice has at most 51,200 entries: no limb's sum passes 2^32
     const unsigned long long q = weight_fix(v);
-    const unsigned l0 = (unsigned)(q & 0x1FFFu), l1 = (unsigned)((q >> 13) & 0x1FFFu), l2 = (unsigned)(q >> 26);
+    const unsigned l0 = (unsigned)(q & 0xFFFFu), l1 = (unsigned)(q >> 16) & 0xFFFFu, l2 = (unsigned)(q >> 32);
     if (l0) atomicAdd(&sh.limb[0][key], l0);
-    if (l1) atomicAdd(&sh.limb[1][key], l1);
-    if (l2) atomicAdd(&sh.limb[2][key], l2);            // most weights are below 2^-13
+    if (l1) atomicAdd(&sh.limb[1][key], l1);            // none below 2^-23
+    if (l2) atomicAdd(&sh.limb[2][key], l2);            // few weights are as large as 2^-7
   }
 }
 template <bool COUNT> __device__ __forceinline__ void radix_clear(SampleShared& sh) {      // counts leave the other two limbs alone
@@ -398,10 +400,13 @@ template <typename F> __device__ __forceinline__ void for_weights(const float* w
 // The largest threshold T >= floor_bits such that the entries with bits >= T number (COUNT) or weigh (fixed point) at least
 // a target; floor_bits if even that does not reach it.  w: this block's n weights.  The target is `count` or, of masses, the
 // share p of all that the histogram's first level holds (the entries from floor_bits on).  The caller has cleared the limbs
-// and filled the first level (bits 20 to 29 as the key).
+// and filled the first level (bits 20 to 29 as the key).  The second level's walk over the weights notes down those that can
+// still matter (of counts all from the first level's bin on, for the masses that may be asked for next; of masses those in the
+// bin), and what follows walks that short list; where it overflows, all weights again.  list: room for list_room weights;
+// `noted`: those of a call before are there.
 template <bool COUNT>
-__device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, unsigned floor_bits, unsigned long long count, float p,
-                                    int& buffer, int cl) {
+__device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, float* list, int list_room, unsigned floor_bits,
+                                    unsigned long long count, float p, int& buffer, int cl, bool& noted) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned prefix = 0;                                  // the bits above the level's ten, once decided
   unsigned long long above = 0, target = count;         // count / mass of the entries above the prefix's range
@@ -411,17 +416,34 @@ __device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, uns
     unsigned long long* h = sh.hist[buffer & 1];
     ++buffer;
     if (lev > 0) {
-      for_weights(w, n, [&](float v) {
+      auto add = [&](float v) {
         const unsigned b = __float_as_uint(v);
         if ((b >> (shift + 10)) == prefix && b >= floor_bits) radix_add<COUNT>(sh, (b >> shift) & (SC_BINS - 1), v);
-      });
+      };
+      if (noted) {
+        for (int i = tid; i < sh.listed; i += SC_THREADS) add(list[i]);
+      } else {
+        for_weights(w, n, [&](float v) {
+          const unsigned b = __float_as_uint(v);
+          if (lev == 1 && (COUNT ? (b >> 20) >= prefix : (b >> 20) == prefix && b >= floor_bits)) {
+            const int at = atomicAdd(&sh.listed, 1);
+            if (at < list_room) list[at] = v;
+          }
+          add(v);
+        });
+      }
     }
     __syncthreads();
+    if (lev == 1 && !noted) noted = sh.listed <= list_room;
     h[tid] = COUNT ? (unsigned long long)sh.limb[0][tid]
-                   : (unsigned long long)sh.limb[0][tid] + ((unsigned long long)sh.limb[1][tid] << 13) +
-                         ((unsigned long long)sh.limb[2][tid] << 26);
+                   : (unsigned long long)sh.limb[0][tid] + ((unsigned long long)sh.limb[1][tid] << 16) +
+                         ((unsigned long long)sh.limb[2][tid] << 32);
     radix_clear<COUNT>(sh);                             // (every thread its own bins) for the next level
-    if (tid == 0) { sh.chosen = 0; sh.bcast = above; }
+    if (tid == 0) {
+      sh.chosen = 0;
+      sh.bcast = above;
+      if (lev == 0 && !noted) sh.listed = 0;
+    }
     cluster_sync_all();
     const int bin = SC_BINS - 1 - tid;                  // thread order = bins from the top
     unsigned long long part[SC_MAX_CL];
@@ -468,9 +490,10 @@ __global__ void __launch_bounds__(SC_THREADS, 2)        // two blocks per SM: 32
 sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, const float* __restrict__ temperature,
                       const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
                       const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
-                      int* __restrict__ out, int vocab, int cl, int slice) {
+                      int* __restrict__ out, int vocab, int cl, int slice, int list_room) {
   pdl_enter();
-  extern __shared__ __align__(16) float w_s[];          // this block's slice of the row: logits, then weights
+  extern __shared__ __align__(16) float w_s[];          // this block's slice of the row: logits, then weights; then the list
+  float* list = w_s + slice;
   __shared__ SampleShared sh;
   const int tid = threadIdx.x;
   const int row = blockIdx.x / cl;
@@ -539,17 +562,23 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
   }
   __syncthreads();
   int buffer = 0;
+  bool noted = false;
   unsigned thr = 0u;                                    // keep entries with weight bits >= thr
-  if (by_count) thr = radix_threshold<true>(sh, w_s, n, 0u, (unsigned long long)k, 0.0f, buffer, cl);
+  if (by_count) thr = radix_threshold<true>(sh, w_s, n, list, list_room, 0u, (unsigned long long)k, 0.0f, buffer, cl, noted);
   thr = max(thr, thr_min);
   if (by_mass) {                                        // the largest threshold whose kept mass is >= p of the mass kept so far
     if (by_count) {
-      for_weights(w_s, n, [&](float v) {
+      auto add = [&](float v) {
         const unsigned b = __float_as_uint(v);
         if (b >= thr) radix_add<false>(sh, (b >> 20) & (SC_BINS - 1), v);
-      });
+      };
+      if (noted) {
+        for (int i = tid; i < sh.listed; i += SC_THREADS) add(list[i]);
+      } else {
+        for_weights(w_s, n, add);
+      }
     }
-    thr = radix_threshold<false>(sh, w_s, n, thr, 0ull, p, buffer, cl);
+    thr = radix_threshold<false>(sh, w_s, n, list, list_room, thr, 0ull, p, buffer, cl, noted);
   }
   // inverse CDF over the kept entries in index order: first the block that holds the target, then the thread, then the entry
   const int seg = ((n + SC_THREADS - 1) / SC_THREADS) | 1;      // odd: the threads' entries lie in different banks
@@ -597,11 +626,14 @@ int launch_sample_cluster(const float* logits, long long row_stride, const float
                           const float* top_p, const float* min_p, const unsigned long long* seeds,
                           const unsigned long long* counters, int* out, int n_rows, int vocab, int cl, cudaStream_t stream) {
   const int slice = ((vocab + cl - 1) / cl + 3) / 4 * 4;
-  const size_t smem = (size_t)slice * sizeof(float);
+  // the list takes what a slice leaves of 227 KB
+  const int left = (227 * 1024 - (int)sizeof(SampleShared)) / (int)sizeof(float) - slice - 16;
+  const int list_room = left < 0 ? 0 : left < SC_LIST ? left : SC_LIST;
+  const size_t smem = (size_t)(slice + list_room) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int rc = launch_pdl_cluster(sample_cluster_kernel, dim3(n_rows * cl), dim3(SC_THREADS), smem, stream, dim3(cl, 1, 1),
-                                    logits, row_stride, temperature, top_k, top_p, min_p, seeds, counters, out, vocab, cl, slice);
+                                    logits, row_stride, temperature, top_k, top_p, min_p, seeds, counters, out, vocab, cl, slice, list_room);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
 }  // namespace
