@@ -17,6 +17,7 @@ from ..config.registry import part_class
 from ..config.spec import ModelSpec
 from ..parts.base import KVNeed, RunInfo, StateNeed
 from ..weights.loader import WeightSpec, load_weights
+from .prenorm_run import PrenormRun
 
 
 class Model:
@@ -41,6 +42,7 @@ class Model:
         self._plan_cache()
         self._describers = self._collect_describers()
         self._keeps_embedding = any(getattr(b, "needs_embedding_output", False) for b in self.blocks)
+        self._prenorm_run = PrenormRun.of(self)
 
     @staticmethod
     def _roles(layer) -> Dict[str, str]:
@@ -179,8 +181,11 @@ class Model:
         if self._keeps_embedding:
             ctx.embedding_output = residual.clone()      # a block reads the stream as the embedding left it
         delta = None
-        for info in self.runs:
-            delta = self.blocks[self.spec.schedule[info.run_index].layer].forward(residual, delta, ctx, info)
+        if self._prenorm_run is not None and self._prenorm_run.takes(ctx):
+            delta = self._prenorm_run.forward(residual, ctx, self.runs)      # (None: not for these weights)
+        if delta is None:
+            for info in self.runs:
+                delta = self.blocks[self.spec.schedule[info.run_index].layer].forward(residual, delta, ctx, info)
         if ctx.n_want == 0:
             return torch.empty((0, self.spec.vocab_size), dtype=torch.float32, device=self.device)
         x = self.final_norm.forward(residual, delta, rows=ctx.want_rows)

@@ -1,0 +1,119 @@
+"""A step's pre-norm layers launched by one native call.
+
+A step that brings a prompt portion is launched kernel by kernel from the host, and with few rows the host is what it waits
+for: at the 3B sizes 77 rows take the GPU 60 to 90 us a layer and the host, from Python, 110 to 140.  Where a model's layers are
+all of the common kind (:class:`~inferflux_b200.parts.block.PreNormBlock` of grouped-query attention and SwiGLU with RMSNorm,
+bfloat16, head size 128, no window) such a step's layers are launched by ``ops.prenorm_layers``: the same kernels with the same
+arguments, so the same results.  Everything else goes through the blocks.
+"""
+from __future__ import annotations
+
+from typing import Optional
+
+import numpy as np
+import torch
+
+from ..kernels import ops
+from ..parts.attention import GQAttention, prefill_plan
+from ..parts.base import PartialSums
+from ..parts.block import PreNormBlock
+from ..parts.feed_forward import SwiGLU
+from ..parts.norm import RMSNorm
+
+
+class PrenormRun:
+    """The layers of a model that one call can launch: all of its runs or none."""
+
+    def __init__(self, blocks):
+        self.blocks = blocks                            # one per run, in schedule order
+
+    @staticmethod
+    def of(model) -> Optional["PrenormRun"]:
+        blocks = [model.blocks[r.layer] for r in model.spec.schedule]
+        if model.dtype != torch.bfloat16 or not blocks:
+            return None
+        shapes = set()
+        for block, info in zip(blocks, model.runs):
+            if type(block) is not PreNormBlock or type(block.mixer) is not GQAttention or type(block.feed_forward) is not SwiGLU:
+                return None
+            if type(block.mixer_norm) is not RMSNorm or type(block.feed_forward_norm) is not RMSNorm:
+                return None
+            a = block.mixer
+            if a.window or a.kv_shared or not info.writes_kv or a.head_dim != ops.UMMA_ATTENTION_HEAD_DIM or a.params.get("o_bias"):
+                return None
+            shapes.add((info.kv_group, block.position_name, a.hidden, a.n_heads, a.n_kv, a.scale, block.feed_forward.intermediate))
+        if len(shapes) != 1 or blocks[0].mixer.hidden % 8 or blocks[0].feed_forward.intermediate % 8:
+            return None
+        return PrenormRun(blocks)
+
+    def takes(self, ctx) -> bool:
+        step = ctx.extras[GQAttention.describe_key]
+        return ops.PRENORM_MIN_ROWS <= ctx.n_tokens <= ops.PRENORM_MAX_ROWS and step.n_decode != ctx.n_tokens
+
+    def forward(self, residual: torch.Tensor, ctx, runs) -> Optional[PartialSums]:
+        """All layers; the last one's pending delta.  None (nothing done): weights or angles that the kernels do not take."""
+        first, n, dev = self.blocks[0].mixer, ctx.n_tokens, residual.device
+        hidden, inter, nh, nkv, hd = first.hidden, self.blocks[0].feed_forward.intermediate, first.n_heads, first.n_kv, first.head_dim
+        position = ctx.position_tables.get(self.blocks[0].position_name) if self.blocks[0].position_name else None
+        if not isinstance(position, (tuple, list)) or len(position) != 2 or 2 * position[0].shape[1] != hd:
+            return None
+        cos, sin = position
+        words, matrices = [], 0
+        for block, info in zip(self.blocks, runs):
+            a, f = block.mixer, block.feed_forward
+            k, v, page_stride = ctx.kv.layer_views(info.kv_group, info.kv_index)
+            mats = (a.qkv.weight, a.o.weight, f.gate_up.weight, f.down.weight)
+            at = [m.data_ptr() for m in mats]
+            if any(m.dtype != torch.bfloat16 for m in mats) or any(p & 15 for p in at):
+                return None
+            if a.qkv.bias is not None or a.o.bias is not None or f.down.bias is not None:
+                return None
+            words.append((block.mixer_norm.weight.data_ptr(), at[0], 0 if a.qkv_bias is None else a.qkv_bias.data_ptr(),
+                          k.data_ptr(), v.data_ptr(), at[1], block.feed_forward_norm.weight.data_ptr(), at[2], at[3], 0, 0))
+        layers = np.array(words, dtype=np.int64)
+        eps = layers.view(np.float64)
+        eps[:, 9] = [b.mixer_norm.eps for b in self.blocks]
+        eps[:, 10] = [b.feed_forward_norm.eps for b in self.blocks]
+
+        step, width = ctx.extras[GQAttention.describe_key], (nh + 2 * nkv) * hd
+        g = runs[0].kv_group
+        s = ops.PrenormStep()
+        keep = []                                       # scratch stays until the kernels are launched (then the stream orders its reuse)
+
+        def scratch(dtype, count):
+            t = torch.empty(count, dtype=dtype, device=dev)
+            keep.append(t)
+            return t.data_ptr()
+        bf16, f32 = torch.bfloat16, torch.float32
+        s.rows, s.hidden, s.inter, s.n_heads, s.n_kv, s.page_size = n, hidden, inter, nh, nkv, ctx.page_size
+        s.qkv_parts = ops.gemm_umma_skinny_parts(width, hidden, n)
+        s.o_parts = ops.gemm_umma_skinny_parts(hidden, nh * hd, n)
+        s.down_parts = ops.gemm_umma_skinny_parts(hidden, inter, n)
+        delta = torch.empty((max(s.o_parts, s.down_parts), n, hidden), dtype=f32, device=dev)
+        s.residual, s.delta = residual.data_ptr(), delta.data_ptr()
+        s.x, s.qkv, s.attn, s.act = (scratch(bf16, n * w) for w in (hidden, width, nh * hd, inter))
+        s.qkv_sums = scratch(f32, s.qkv_parts * n * width)
+        s.cos_t, s.sin_t, s.slot_map = cos.data_ptr(), sin.data_ptr(), ctx.slot_maps[g].data_ptr()
+        tables = ctx.block_tables[g]
+        s.block_tables, s.bt_stride, s.page_stride = tables.data_ptr(), tables.stride(0), page_stride
+        s.entry_q_start, s.entry_q_len, s.entry_ctx_start = (t.data_ptr() for t in (ctx.entry_q_start, ctx.entry_q_len, ctx.entry_ctx_start))
+        s.num_pages = ops.paged_pool_pages(k, v, page_stride, nkv * ctx.page_size * hd)
+        s.scale = first.scale
+        s.n_tiles, s.tile_rows = step.n_umma_tiles, step.umma_tile_rows
+        s.tile_entry, s.tile_q0 = step.umma_tile_entry.data_ptr(), step.umma_tile_q0.data_ptr()
+        s.n_splits = prefill_plan(ctx, 2, step.umma_tile_rows, nh, ctx.max_ctx_len, 0)[0]
+        if s.n_splits > 1:
+            rows = ops.attn_prefill_cut_units(s.n_tiles, nh) * s.n_splits * ops.UMMA_ATTENTION_TILE
+            s.part_o, s.part_ml = scratch(f32, rows * hd), scratch(f32, rows * 2)
+        s.n_dec, s.dec_splits = step.n_decode, 1
+        if step.n_decode:
+            s.dec_entries = step.decode_entries.data_ptr()
+            if first._share_by_tiles(step):
+                s.dec_pieces = ops.attn_decode_pieces(nh, nkv, hd, ctx.max_ctx_len)
+                s.piece_count = scratch(torch.int32, step.n_decode * nh)
+            else:
+                s.dec_splits = ops.attn_decode_splits(step.n_decode, nh, nkv, hd, ctx.max_ctx_len)
+            rows = step.n_decode * nh * max(s.dec_pieces, s.dec_splits)
+            s.dec_o, s.dec_ml = scratch(f32, rows * hd), scratch(f32, rows * 2)
+        ops.prenorm_layers(s, layers, dev)
+        return PartialSums(delta[:s.down_parts])

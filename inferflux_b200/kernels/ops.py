@@ -99,6 +99,8 @@ def _load():
         lib.ifx_attn_prefill_plan.restype = c_int
         lib.ifx_attn_prefill_umma_cut_units.argtypes = [c_int, c_int]
         lib.ifx_attn_prefill_umma_cut_units.restype = c_int
+        lib.ifx_prenorm_layers.argtypes = [c_void_p, c_void_p, c_int, c_void_p]
+        lib.ifx_prenorm_layers.restype = c_int
         lib.ifx_argmax.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p]
         lib.ifx_apply_penalties.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                             c_void_p, c_int, c_int, c_void_p]
@@ -732,14 +734,12 @@ def attn_prefill_umma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_layer
     _need(block_tables.dtype == torch.int32 and block_tables.stride(1) == 1, "attn: block_tables int32 [R, B]")
     # The kernel reads the cache through a TMA tensor map, which wants to know how many pages lie behind page 0:
     # as many as fit between the view's start and the end of the storage it is a view of.
-    n_elems = k_layer.untyped_storage().nbytes() // k_layer.element_size()
-    last = max(k_layer.storage_offset(), v_layer.storage_offset()) + n_kv * page_size * head_dim
-    num_pages = (n_elems - last) // page_stride + 1 if n_elems >= last else 0
+    num_pages = paged_pool_pages(k_layer, v_layer, page_stride, n_kv * page_size * head_dim)
     _need(num_pages >= 1, "attn_prefill_umma: k_layer / v_layer are not views of page 0 of a paged pool")
     part_o = part_ml = None
     global launch_count
     if n_splits > 1:
-        rows = int(_lib().ifx_attn_prefill_umma_cut_units(n_tiles, n_heads)) * n_splits * UMMA_ATTENTION_TILE
+        rows = attn_prefill_cut_units(n_tiles, n_heads) * n_splits * UMMA_ATTENTION_TILE
         part_o = torch.empty(rows * head_dim, dtype=torch.float32, device=q.device)
         part_ml = torch.empty(rows * 2, dtype=torch.float32, device=q.device)
         launch_count += 1          # the merge kernel
@@ -925,6 +925,49 @@ def attn_decode_even_bf16(q: torch.Tensor, out: torch.Tensor, k_layer: torch.Ten
                                             n_kv, head_dim, float(scale), int(window), int(max_pieces),
                                             error_flag(q.device).data_ptr(), _stream()), "attn_decode_even_bf16")
     return out
+
+
+# ------------------------------------------------------------- whole layers
+class PrenormStep(ctypes.Structure):
+    """``PrenormStep`` of csrc/prenorm_layers.cu: what the layers of one call share."""
+
+    _fields_ = ([(n, c_void_p) for n in ("residual", "x", "qkv", "attn", "act", "qkv_sums", "delta", "cos_t", "sin_t", "slot_map",
+                                         "block_tables", "entry_q_start", "entry_q_len", "entry_ctx_start", "tile_entry", "tile_q0",
+                                         "dec_entries", "part_o", "part_ml", "dec_o", "dec_ml", "piece_count", "error_flag", "stream")]
+                + [("page_stride", c_ll)]
+                + [(n, c_int) for n in ("rows", "hidden", "inter", "n_heads", "n_kv", "page_size", "bt_stride", "num_pages", "qkv_parts",
+                                        "o_parts", "down_parts", "n_tiles", "tile_rows", "n_splits", "n_dec", "dec_splits", "dec_pieces")]
+                + [("scale", c_float)])
+
+
+PRENORM_MIN_ROWS, PRENORM_MAX_ROWS = 9, 128
+
+
+def attn_prefill_cut_units(n_tiles: int, n_heads: int) -> int:
+    """(tile, head) units that :func:`attn_prefill_umma` cuts with more than one part: scratch for so many."""
+    return int(_lib().ifx_attn_prefill_umma_cut_units(n_tiles, n_heads))
+
+
+def paged_pool_pages(k_layer: torch.Tensor, v_layer: torch.Tensor, page_stride: int, page_elements: int) -> int:
+    """How many pages lie behind page 0, of which the two are views: as many as fit before the end of their storage."""
+    n_elems = k_layer.untyped_storage().nbytes() // k_layer.element_size()
+    last = max(k_layer.storage_offset(), v_layer.storage_offset()) + page_elements
+    return (n_elems - last) // page_stride + 1 if n_elems >= last else 0
+
+
+def prenorm_layers(step: PrenormStep, layers: np.ndarray, device) -> None:
+    """The kernels of ``len(layers)`` pre-norm layers (norm, grouped-query attention over the paged cache, norm, SwiGLU; head size
+    128, bfloat16) launched by one call.  ``layers``: [n, 11] 64-bit words, a row as ``PrenormLayer`` of
+    csrc/prenorm_layers.cu.  ``step.stream`` and ``step.error_flag`` are filled in here."""
+    _need(layers.dtype == np.int64 and layers.ndim == 2 and layers.shape[1] == 11 and layers.flags.c_contiguous,
+          "prenorm_layers: int64 [n, 11] layers")
+    _need(PRENORM_MIN_ROWS <= step.rows <= PRENORM_MAX_ROWS, "prenorm_layers: 9 to 128 rows")
+    step.stream, step.error_flag = _stream(), error_flag(device).data_ptr()
+    launched = c_int(0)
+    rc = _lib().ifx_prenorm_layers(ctypes.byref(step), layers.ctypes.data, layers.shape[0], ctypes.byref(launched))
+    global launch_count
+    launch_count += launched.value - 1                    # (_check counts one)
+    _check(rc, "prenorm_layers")
 
 
 # --------------------------------------------------------------------- sampling
