@@ -15,7 +15,7 @@
 // multiply-adds in index order, so infinities and NaN come out as they do there.
 //
 // A block takes 128 rows of W, the tile's M rows of the MMA, and tile_n tokens, its N columns.  W arrives as float32 by TMA
-// (128-byte swizzle, K 64 a stage); a thread of eight warps reads half a row's 64 values, cuts them up with bit masks and
+// (128-byte swizzle, K 64 a stage); a thread of sixteen warps reads a quarter of a row's 64 values, cuts them up with bit masks and
 // subtractions (exact) and writes the three parts into tensor memory, where the MMA takes its A operand from: the parts never go
 // back to shared memory, whose bandwidth the MMA's B operand (the tokens' three parts) needs.  Up to 64 tokens the same
 // threads cut the tokens' values up as well; for more, split_kernel has done it once for all blocks and TMA brings the parts.
@@ -32,7 +32,7 @@ namespace {
 
 constexpr int FK64 = 64;                        // K per step
 constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
-constexpr int U_WORKERS = 256, U_THREADS = U_WORKERS + 96;   // 8 warps of workers, a warp each for W's copies, the MMAs and the tokens' copies
+constexpr int U_WORKERS = 512, U_THREADS = U_WORKERS + 96;   // 16 warps of workers, a warp each for W's copies, the MMAs and the tokens' copies
 constexpr unsigned U_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // D float32, A and B bfloat16, K-major, M 128; N (in eighths) at bit 17
 
 __host__ __device__ constexpr int u_w_stages(int tn) { return tn == 16 ? 3 : tn <= 64 ? 5 : tn <= 128 ? 4 : 3; }
@@ -72,16 +72,21 @@ __device__ __forceinline__ void u_tmem_st8(unsigned taddr, const unsigned (&r)[8
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
+__device__ __forceinline__ void u_tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+}
 __device__ __forceinline__ void u_tmem_ld8(unsigned taddr, unsigned (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-__device__ __forceinline__ void u_mma(unsigned d, unsigned a_tmem, unsigned long long db, unsigned idesc, unsigned accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(d), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+// The warp that issues runs as one, and one lane of it (elected != 0) issues: its operands can then stand in uniform registers, where
+// the instruction wants them (from inside a branch of one lane an MMA took 75 cycles to issue, more than it takes to run).
+__device__ __forceinline__ void u_mma(unsigned elected, unsigned d, unsigned a_tmem, unsigned long long db, unsigned idesc, unsigned accumulate) {
+  asm volatile("{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 e, %5, 0;\n @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(d), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
 }
-__device__ __forceinline__ void u_commit(unsigned bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+__device__ __forceinline__ void u_commit(unsigned elected, unsigned bar) {
+  asm volatile("{\n .reg .pred e;\n setp.ne.b32 e, %1, 0;\n @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar), "r"(elected) : "memory");
 }
 
 // TN: token columns a block can hold.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W, slices of K), the slices of a tile a
@@ -92,13 +97,13 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                      const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K, long long lda,
                      long long ldc, int tile_n, int slice_steps, int vec_a, int w_fixed, int* __restrict__ error_flag) {
   constexpr bool OWN_X = TN <= 64;
-  constexpr int STAGES = u_w_stages(TN), HALF = TN / 2, X_PER = OWN_X ? TN / 16 : 1;   // X_PER: float4 of the tokens a worker cuts up
+  constexpr int STAGES = u_w_stages(TN), COLS = TN / 4, X_PER = OWN_X && TN > 32 ? TN / 32 : 1;   // columns, and float4 of the tokens, of a worker
   extern __shared__ unsigned char u_smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 6];   // w_full[s], w_empty[s], x_full[2], parts_full[2], mma_done[2]
   __shared__ unsigned tmem_slot;
   __shared__ int abort_s;
   const unsigned sbase = (g_smem_addr(u_smem_raw) + 1023u) & ~1023u, sx = sbase + STAGES * W_STAGE;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (shuffled: known to be uniform)
   const unsigned w_full = g_smem_addr(&bars[0]), w_empty = g_smem_addr(&bars[STAGES]), x_full = g_smem_addr(&bars[2 * STAGES]);
   const unsigned parts_full = x_full + 16, mma_done = x_full + 32;
   volatile int* abort_flag = &abort_s;
@@ -116,7 +121,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
-  if (warp == 9) {
+  if (warp == 17) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(g_smem_addr(&tmem_slot)), "n"(u_columns(TN)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
@@ -124,17 +129,17 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   pdl_launch_dependents();                       // behind the allocation: no block of the next kernel can be ahead of it at the tensor memory
-  const unsigned tmem = tmem_slot;
+  const unsigned tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const int m0 = blockIdx.x * tile_n, n0 = blockIdx.y * 128;
   const int steps_all = (K + FK64 - 1) / FK64, step0 = min(steps_all, (int)blockIdx.z * slice_steps);
   const int steps = min(steps_all, step0 + slice_steps) - step0;
   bool gave_up = false;
-  float acc[HALF];
+  float acc[COLS];
 #pragma unroll
-  for (int i = 0; i < HALF; ++i) acc[i] = 0.0f;
-  const int quarter = warp & 3, half = warp >> 2;                      // of a worker: its lanes of tensor memory, its half of K and of the columns
+  for (int i = 0; i < COLS; ++i) acc[i] = 0.0f;
+  const int quarter = warp & 3, part = warp >> 2;                      // of a worker: its lanes of tensor memory, its fourth of K and of the columns
 
-  if (warp == 8) {                                                     // W's copies
+  if (warp == 16) {                                                    // W's copies
     if (lane == 0) {
       if (!w_fixed) pdl_wait();
       for (int c = 0; c < steps; ++c) {
@@ -148,7 +153,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                        ::"r"(sbase + st * W_STAGE + h * (W_STAGE / 2)), "l"(&map_w), "r"((step0 + c) * FK64 + 32 * h), "r"(n0), "r"(w_full + 8 * st) : "memory");
       }
     }
-  } else if (warp == 10) {                                             // the tokens' copies
+  } else if (warp == 18) {                                             // the tokens' copies
     if (!OWN_X && lane == 0) {
       pdl_wait();
       for (int c = 0; c < steps; ++c) {
@@ -159,26 +164,26 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                      ::"r"(sx + b * 3 * TN * 128), "l"(&map_x), "r"((step0 + c) * FK64), "r"(m0), "r"(0), "r"(x_full + 8 * b) : "memory");
       }
     }
-  } else if (warp == 9) {                                              // the MMAs
-    if (lane == 0) {
-      pdl_wait();
-      const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17);
-      for (int c = 0; c < steps; ++c) {
-        const int b = c & 1;
-        const unsigned par = (unsigned)((c >> 1) & 1);
-        if (!g_wait(parts_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
-        if (!OWN_X && !g_wait(x_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const unsigned d = tmem + 192 + b * TN, wp = tmem + b * 96, xp = sx + b * 3 * TN * 128;
-        // (W's part, the tokens' part), 0 the highest: the small products first
-        constexpr int order[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
+  } else if (warp == 17) {                                             // the MMAs
+    pdl_wait();
+    const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17), elected = lane == 0;
+    for (int c = 0; c < steps; ++c) {
+      const int b = c & 1;
+      const unsigned par = (unsigned)((c >> 1) & 1);
+      bool ok = g_wait(parts_full + 8 * b, par, abort_flag);
+      if (!OWN_X) ok = ok && g_wait(x_full + 8 * b, par, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) { gave_up = true; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const unsigned d = tmem + 192 + b * TN, wp = tmem + b * 96;
+      const unsigned long long xd = g_desc(sx + b * 3 * TN * 128);
+      // (W's part, the tokens' part), 0 the highest: the small products first
+      constexpr int order[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-        for (int p = 0; p < 6; ++p)
+      for (int p = 0; p < 6; ++p)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            u_mma(d, wp + order[p][0] * 32 + k * 8, g_desc(xp + order[p][1] * tile_n * 128 + k * 32), idesc, (p | k) != 0);
-        u_commit(mma_done + 8 * b);
-      }
+        for (int k = 0; k < 4; ++k)                                    // (a descriptor's address counts 16 bytes)
+          u_mma(elected, d, wp + order[p][0] * 32 + k * 8, xd + (unsigned)(order[p][1] * tile_n * 8 + k * 2), idesc, (p | k) != 0);
+      u_commit(elected, mma_done + 8 * b);
     }
   } else {
     const unsigned lanes = tmem + ((unsigned)(quarter * 32) << 16);
@@ -187,13 +192,22 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       if (!__all_sync(0xffffffffu, g_wait(mma_done + 8 * (c & 1), (unsigned)((c >> 1) & 1), abort_flag))) return false;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
-      for (int i = 0; i < HALF / 8; ++i) {
-        if (half * HALF + i * 8 >= tile_n) break;                      // (the same for the warp)
-        unsigned r[8];
-        u_tmem_ld8(lanes + 192 + (c & 1) * TN + half * HALF + i * 8, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      for (int i = 0; i < (COLS + 7) / 8; ++i) {
+        if (part * COLS + i * 8 >= tile_n) break;                      // (the same for the warp)
+        const unsigned at = lanes + 192 + (c & 1) * TN + part * COLS + i * 8;
+        if constexpr (COLS == 4) {
+          unsigned r[4];
+          u_tmem_ld4(at, r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i * 8 + j] += __uint_as_float(r[j]);
+          for (int j = 0; j < 4; ++j) acc[j] += __uint_as_float(r[j]);
+        } else {
+          unsigned r[8];
+          u_tmem_ld8(at, r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[i * 8 + j] += __uint_as_float(r[j]);
+        }
       }
       return true;
     };
@@ -202,7 +216,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       const int k = (step0 + c) * FK64 + (tid & 15) * 4;
 #pragma unroll
       for (int i = 0; i < X_PER; ++i) {
-        const int t = (tid >> 4) + 16 * i, m = m0 + t;
+        const int t = (tid >> 4) + 32 * i, m = m0 + t;
         xr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < tile_n && m < M && k < K && c < steps) {               // K is a multiple of 4
           const float* p = A + (size_t)m * lda + k;
@@ -218,27 +232,24 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       bool ok = c < 2 || add_sums(c - 2);                              // (and its parts' places are free)
       ok = ok && g_wait(w_full + 8 * st, (unsigned)((c / STAGES) & 1), abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { gave_up = true; break; }
-      const unsigned wrow = sbase + st * W_STAGE + half * (W_STAGE / 2) + row * 128;
+      const unsigned wrow = sbase + st * W_STAGE + (part >> 1) * (W_STAGE / 2) + row * 128;
+      unsigned hi[8], mid[8], lo[8];
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {                                    // 16 values at a time
-        unsigned hi[8], mid[8], lo[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float x, y, z, w;
-          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(wrow + (((g * 4 + j) ^ (row & 7)) << 4)) : "memory");
-          cut(x, y, hi[2 * j], mid[2 * j], lo[2 * j]);
-          cut(z, w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
-        }
-        const unsigned at = lanes + b * 96 + half * 16 + g * 8;
-        u_tmem_st8(at, hi);
-        u_tmem_st8(at + 32, mid);
-        u_tmem_st8(at + 64, lo);
+      for (int j = 0; j < 4; ++j) {
+        float x, y, z, w;
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(wrow + ((((part & 1) * 4 + j) ^ (row & 7)) << 4)) : "memory");
+        cut(x, y, hi[2 * j], mid[2 * j], lo[2 * j]);
+        cut(z, w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
       }
+      const unsigned at = lanes + b * 96 + part * 8;
+      u_tmem_st8(at, hi);
+      u_tmem_st8(at + 32, mid);
+      u_tmem_st8(at + 64, lo);
       u_arrive_warp(w_empty + 8 * st, lane);
       if (OWN_X) {
 #pragma unroll
         for (int i = 0; i < X_PER; ++i) {
-          const int t = (tid >> 4) + 16 * i, q = tid & 15;
+          const int t = (tid >> 4) + 32 * i, q = tid & 15;
           if (t >= tile_n) break;
           unsigned h0, m0_, l0, h1, m1, l1;
           cut(xr[i].x, xr[i].y, h0, m0_, l0);
@@ -275,29 +286,29 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.0f);
   };
   if (slices == 1) {
-    if (warp < 8) {
+    if (warp < 16) {
       const int n = n0 + quarter * 32 + lane;
       if (n < N)
 #pragma unroll
-        for (int i = 0; i < HALF; ++i) {
-          const int t = half * HALF + i;
+        for (int i = 0; i < COLS; ++i) {
+          const int t = part * COLS + i;
           if (t < tile_n && m0 + t < M) put(m0 + t, n, acc[i]);
         }
     }
   } else {
     __syncthreads();
-    if (warp < 8) {
+    if (warp < 16) {
 #pragma unroll
-      for (int i = 0; i < HALF; ++i) {
-        const int t = half * HALF + i;
+      for (int i = 0; i < COLS; ++i) {
+        const int t = part * COLS + i;
         if (t < tile_n) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sbase + (t * 128 + quarter * 32 + lane) * 4), "f"(acc[i]) : "memory");
       }
     }
     u_cluster_sync();
     const int rank = (int)u_cluster_rank();
-    if (warp < 8) {
+    if (warp < 16) {
       const int n = n0 + (tid & 127);
-      for (int t = rank * 2 + (tid >> 7); t < tile_n && m0 + t < M; t += 2 * slices) {
+      for (int t = rank * 4 + (tid >> 7); t < tile_n && m0 + t < M; t += 4 * slices) {
         float s = 0.0f;
         for (int z = 0; z < slices; ++z) s += u_read_peer(sbase + (t * 128 + (tid & 127)) * 4, z);
         if (n < N) put(m0 + t, n, s);
@@ -307,7 +318,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(u_columns(TN)) : "memory");
+  if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(u_columns(TN)) : "memory");
 }
 
 // A's values cut into their parts [3][M][pitch] (zeros behind K), eight a thread.
