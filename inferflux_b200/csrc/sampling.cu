@@ -40,24 +40,21 @@ __device__ __forceinline__ ArgPair better(ArgPair a, ArgPair b) {
   if (b.i >= 0 && (a.i < 0 || b.v > a.v || (b.v == a.v && b.i < a.i))) return b;
   return a;
 }
-// The best pair of the block; every thread of warp 0 gets it.  `scratch` holds 32 pairs.
+// The best pair of the warp / of the block, for every thread.  `scratch` holds 32 pairs.
+__device__ __forceinline__ ArgPair warp_best(ArgPair best) {
+  // values as integers of the same order (both zeros alike), 0 for none
+  const unsigned bits = __float_as_uint(best.v + 0.0f), key = best.i < 0 ? 0u : bits ^ ((bits >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+  const unsigned top = __reduce_max_sync(0xffffffffu, key);
+  const unsigned at = __reduce_min_sync(0xffffffffu, key == top ? (unsigned)best.i : 0xFFFFFFFFu);      // (an index of -1 is the largest)
+  return ArgPair{__uint_as_float(top ^ ((top >> 31) ? 0x80000000u : 0xFFFFFFFFu)), (int)at};
+}
 __device__ ArgPair block_best(ArgPair best, ArgPair* scratch) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ArgPair other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
-    best = better(best, other);
-  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+  best = warp_best(best);
   __syncthreads();
   if (lane == 0) scratch[warp] = best;
   __syncthreads();
-  best = lane < nwarps ? scratch[lane] : ArgPair{-INFINITY, -1};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ArgPair other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
-    best = better(best, other);
-  }
-  return best;
+  return warp_best(lane < nwarps ? scratch[lane] : ArgPair{-INFINITY, -1});
 }
 __device__ ArgPair block_argmax(const float* row, int n, ArgPair* scratch) {
   ArgPair best{-INFINITY, -1};
@@ -314,6 +311,8 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, float* __r
 constexpr int SC_THREADS = 1024, SC_BINS = 1024, SC_MAX_CL = 8;
 constexpr int SC_MAX_SLICE = 51200;                     // floats of a row one block keeps (200 KB)
 constexpr int SC_LIST = 1024;                           // weights that a block can note down for the later levels, behind its slice
+constexpr int SC_GATHER = 4096;                         // weights of all blocks that one can gather, in the histograms' place
+constexpr int SC_MASS_KEY = (127 - 39) << 3;            // weights below this first-level key are below 2^-39: their mass is 0
 
 struct SampleShared {
   unsigned limb[3][SC_BINS];                            // counts, or masses in three 16-bit limbs: 32-bit shared-memory adds
@@ -323,6 +322,9 @@ struct SampleShared {
   unsigned long long part_total, bcast;                 // what this block tells the others; what lies above the chosen bin
   int chosen;
   int listed;                                           // weights noted; more than there is room for: they did not fit
+  float temp, top_p, min_p;                             // the row's numbers, asked for while the row is
+  int top_k;
+  float uniform;
   ArgPair best;
   ArgPair ascratch[32];
 };
@@ -400,58 +402,102 @@ template <typename F> __device__ __forceinline__ void for_weights(const float* w
 // The largest threshold T >= floor_bits such that the entries with bits >= T number (COUNT) or weigh (fixed point) at least
 // a target; floor_bits if even that does not reach it.  w: this block's n weights.  The target is `count` or, of masses, the
 // share p of all that the histogram's first level holds (the entries from floor_bits on).  The caller has cleared the limbs
-// and filled the first level (bits 20 to 29 as the key).  The second level's walk over the weights notes down those that can
-// still matter (of counts all from the first level's bin on, for the masses that may be asked for next; of masses those in the
-// bin), and what follows walks that short list; where it overflows, all weights again.  list: room for list_room weights;
-// `noted`: those of a call before are there.
+// and filled the first level (bits 20 to 29 as the key).
+//
+// A level that the cluster's blocks make together costs a barrier of the cluster and eight reads of the others' shared memory a
+// thread, some 4 us.  So the second level's walk over the weights notes down those that can still matter (of counts all from the
+// first level's bin on, for the masses that may be asked for next; of masses those in the bin) in `list` (room for list_room);
+// where they are few enough every block gathers those of all blocks and makes the rest of the search by itself.  gathered: how
+// many a call has gathered (they stand in sh.hist), -1: none; with some from a call before, the whole search is local.
 template <bool COUNT>
 __device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, float* list, int list_room, unsigned floor_bits,
-                                    unsigned long long count, float p, int& buffer, int cl, bool& noted) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                                    unsigned long long count, float p, int& buffer, int cl, int& gathered) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bin = SC_BINS - 1 - tid;    // thread order = bins from the top
+  float* all = reinterpret_cast<float*>(sh.hist);
   unsigned prefix = 0;                                  // the bits above the level's ten, once decided
   unsigned long long above = 0, target = count;         // count / mass of the entries above the prefix's range
 #pragma unroll 1
   for (int lev = 0; lev < 3; ++lev) {
     const int shift = 20 - 10 * lev;
-    unsigned long long* h = sh.hist[buffer & 1];
-    ++buffer;
-    if (lev > 0) {
-      auto add = [&](float v) {
-        const unsigned b = __float_as_uint(v);
-        if ((b >> (shift + 10)) == prefix && b >= floor_bits) radix_add<COUNT>(sh, (b >> shift) & (SC_BINS - 1), v);
-      };
-      if (noted) {
-        for (int i = tid; i < sh.listed; i += SC_THREADS) add(list[i]);
-      } else {
+    auto add = [&](float v) {
+      const unsigned b = __float_as_uint(v);
+      if ((b >> (shift + 10)) == prefix && b >= floor_bits) radix_add<COUNT>(sh, (b >> shift) & (SC_BINS - 1), v);
+    };
+    auto own = [&](int k) {
+      return COUNT ? (unsigned long long)sh.limb[0][k]
+                   : (unsigned long long)sh.limb[0][k] + ((unsigned long long)sh.limb[1][k] << 16) + ((unsigned long long)sh.limb[2][k] << 32);
+    };
+    auto clear = [&](int k) {                           // (a thread its own bins; counts leave the other two limbs alone)
+      sh.limb[0][k] = 0;
+      if (!COUNT) { sh.limb[1][k] = 0; sh.limb[2][k] = 0; }
+    };
+    unsigned long long tot = 0;
+    if (gathered < 0) {
+      unsigned long long* h = sh.hist[buffer & 1];
+      ++buffer;
+      if (lev == 1) {
         for_weights(w, n, [&](float v) {
           const unsigned b = __float_as_uint(v);
-          if (lev == 1 && (COUNT ? (b >> 20) >= prefix : (b >> 20) == prefix && b >= floor_bits)) {
+          if (COUNT ? (b >> 20) >= prefix : (b >> 20) == prefix && b >= floor_bits) {
             const int at = atomicAdd(&sh.listed, 1);
             if (at < list_room) list[at] = v;
           }
           add(v);
         });
+      } else if (lev == 2) {
+        for_weights(w, n, add);
       }
-    }
-    __syncthreads();
-    if (lev == 1 && !noted) noted = sh.listed <= list_room;
-    h[tid] = COUNT ? (unsigned long long)sh.limb[0][tid]
-                   : (unsigned long long)sh.limb[0][tid] + ((unsigned long long)sh.limb[1][tid] << 16) +
-                         ((unsigned long long)sh.limb[2][tid] << 32);
-    radix_clear<COUNT>(sh);                             // (every thread its own bins) for the next level
-    if (tid == 0) {
-      sh.chosen = 0;
-      sh.bcast = above;
-      if (lev == 0 && !noted) sh.listed = 0;
-    }
-    cluster_sync_all();
-    const int bin = SC_BINS - 1 - tid;                  // thread order = bins from the top
-    unsigned long long part[SC_MAX_CL];
+      __syncthreads();
+      if (COUNT) reinterpret_cast<unsigned*>(h)[tid] = sh.limb[0][tid];
+      else h[tid] = own(tid);
+      clear(tid);
+      if (tid == 0) {
+        sh.chosen = 0;
+        sh.bcast = above;
+        if (lev == 0) sh.listed = 0;
+      }
+      cluster_sync_all();
+      if (lev == 1) {                                   // how many the blocks have noted, the same in each of them
+        const int theirs = lane < cl ? *cluster_peer(&sh.listed, lane) : 0;
+        const bool fit = __all_sync(0xffffffffu, theirs <= list_room);
+        int end = theirs;
 #pragma unroll
-    for (int r = 0; r < SC_MAX_CL; ++r) part[r] = r < cl ? cluster_peer(h, r)[bin] : 0ull;   // all loads in flight together
-    unsigned long long tot = 0;
+        for (int o = 1; o < SC_MAX_CL; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, end, o);
+          if (lane >= o) end += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, end, SC_MAX_CL - 1);
+        if (fit && total <= SC_GATHER) {
+          gathered = total;
+          int from = 0;
+          for (int r = 0; r < cl; ++r) {
+            const int to = __shfl_sync(0xffffffffu, end, r);
+            for (int i = from + tid; i < to; i += SC_THREADS) all[i] = cluster_peer(list, r)[i - from];
+            from = to;
+          }
+          __syncthreads();
+          for (int i = tid; i < gathered; i += SC_THREADS) add(all[i]);
+          __syncthreads();
+          tot = own(bin);
+          clear(bin);
+        }
+      }
+      if (gathered < 0 && (COUNT || lev > 0 || bin >= SC_MASS_KEY)) {
+        unsigned long long part[SC_MAX_CL];
 #pragma unroll
-    for (int r = 0; r < SC_MAX_CL; ++r) tot += part[r];
+        for (int r = 0; r < SC_MAX_CL; ++r)             // all loads in flight together
+          part[r] = r >= cl ? 0ull : COUNT ? (unsigned long long)cluster_peer(reinterpret_cast<unsigned*>(h), r)[bin] : cluster_peer(h, r)[bin];
+#pragma unroll
+        for (int r = 0; r < SC_MAX_CL; ++r) tot += part[r];
+      }
+    } else {
+      if (lev > 0)
+        for (int i = tid; i < gathered; i += SC_THREADS) add(all[i]);
+      __syncthreads();                                  // (and the level before has been read)
+      if (tid == 0) { sh.chosen = 0; sh.bcast = above; }
+      tot = own(bin);
+      clear(bin);
+    }
     unsigned long long reach = tot;                     // the entries in this bin and above it: within the warp, then what
 #pragma unroll                                          // the warps before hold
     for (int o = 1; o < 32; o <<= 1) {
@@ -500,6 +546,13 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
   const int rank = (int)cluster_rank();
   const int begin = min(vocab, rank * slice), n = min(vocab, begin + slice) - begin;
   const float* lg = logits + (size_t)row * row_stride + begin;
+  if (tid == 0) {
+    sh.temp = temperature[row];
+    sh.top_k = top_k[row];
+    sh.top_p = top_p[row];
+    sh.min_p = min_p[row];
+    sh.uniform = uniform01(seeds[row], counters[row]);
+  }
   // the slice into shared memory, and its best logit
   radix_clear<false>(sh);
   ArgPair best{-INFINITY, -1};
@@ -530,7 +583,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
 #pragma unroll
     for (int r = 0; r < SC_MAX_CL; ++r) top = better(top, peer[r]);                 // in rank order: the lowest index among equals
   }
-  const float temp = temperature[row];
+  const float temp = sh.temp;
   if (temp <= 0.0f || top.i < 0) {
     if (rank == 0 && tid == 0) out[row] = top.i < 0 ? 0 : top.i;
     cluster_sync_all();                                 // no block leaves while another may still read its shared memory
@@ -538,8 +591,8 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
   }
   const float inv_t = 1.0f / temp;
   const float mx = top.v * inv_t;
-  const int k = top_k[row];
-  const float mp = min_p[row], p = top_p[row];
+  const int k = sh.top_k;
+  const float mp = sh.min_p, p = sh.top_p;
   const bool by_count = k > 0 && k < vocab, by_mass = p > 0.0f && p < 1.0f;
   const unsigned thr_min = mp > 0.0f ? __float_as_uint(fminf(mp, 1.0f)) : 0u;
   auto weight = [&](float v) { return (v == v) ? expf(v * inv_t - mx) : 0.0f; };      // in [0, 1], the maximum is exactly 1
@@ -561,10 +614,9 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
     first_level(w);
   }
   __syncthreads();
-  int buffer = 0;
-  bool noted = false;
+  int buffer = 0, gathered = -1;
   unsigned thr = 0u;                                    // keep entries with weight bits >= thr
-  if (by_count) thr = radix_threshold<true>(sh, w_s, n, list, list_room, 0u, (unsigned long long)k, 0.0f, buffer, cl, noted);
+  if (by_count) thr = radix_threshold<true>(sh, w_s, n, list, list_room, 0u, (unsigned long long)k, 0.0f, buffer, cl, gathered);
   thr = max(thr, thr_min);
   if (by_mass) {                                        // the largest threshold whose kept mass is >= p of the mass kept so far
     if (by_count) {
@@ -572,13 +624,13 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
         const unsigned b = __float_as_uint(v);
         if (b >= thr) radix_add<false>(sh, (b >> 20) & (SC_BINS - 1), v);
       };
-      if (noted) {
-        for (int i = tid; i < sh.listed; i += SC_THREADS) add(list[i]);
-      } else {
+      if (gathered < 0) {
         for_weights(w_s, n, add);
+      } else {
+        for (int i = tid; i < gathered; i += SC_THREADS) add(reinterpret_cast<float*>(sh.hist)[i]);
       }
     }
-    thr = radix_threshold<false>(sh, w_s, n, list, list_room, thr, 0ull, p, buffer, cl, noted);
+    thr = radix_threshold<false>(sh, w_s, n, list, list_room, thr, 0ull, p, buffer, cl, gathered);
   }
   // inverse CDF over the kept entries in index order: first the block that holds the target, then the thread, then the entry
   const int seg = ((n + SC_THREADS - 1) / SC_THREADS) | 1;      // odd: the threads' entries lie in different banks
@@ -596,7 +648,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
     if (r == rank) block_total = t;
     total += t;
   }
-  const unsigned long long target = (unsigned long long)((double)uniform01(seeds[row], counters[row]) * (double)total);   // < total
+  const unsigned long long target = (unsigned long long)((double)sh.uniform * (double)total);   // < total
   if (target >= offset && target - offset < block_total) {                    // block-uniform
     const unsigned long long local = target - offset;
     if (s > 0 && before <= local && local < incl) {     // exactly one thread
