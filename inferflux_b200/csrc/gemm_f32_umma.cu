@@ -32,6 +32,7 @@ namespace {
 
 constexpr int FK64 = 64;                        // K per step
 constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
+constexpr int U_MAX_SLICES = 8;                  // of K: the largest portable cluster
 constexpr int U_WORKERS = 512, U_THREADS = U_WORKERS + 96;   // 16 warps of workers, a warp each for W's copies, the MMAs and the tokens' copies
 constexpr unsigned U_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // D float32, A and B bfloat16, K-major, M 128; N (in eighths) at bit 17
 
@@ -44,11 +45,11 @@ __device__ __forceinline__ void u_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
-__device__ __forceinline__ float u_read_peer(unsigned saddr, int rank) {
+__device__ __forceinline__ float4 u_read_peer4(unsigned saddr, int rank) {
   unsigned ra;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(saddr), "r"(rank));
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
   return v;
 }
 // one arrival for the warp, once all its lanes have come here
@@ -79,14 +80,12 @@ __device__ __forceinline__ void u_tmem_ld8(unsigned taddr, unsigned (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-// The warp that issues runs as one, and one lane of it (elected != 0) issues: its operands can then stand in uniform registers, where
-// the instruction wants them (from inside a branch of one lane an MMA took 75 cycles to issue, more than it takes to run).
-__device__ __forceinline__ void u_mma(unsigned elected, unsigned d, unsigned a_tmem, unsigned long long db, unsigned idesc, unsigned accumulate) {
-  asm volatile("{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 e, %5, 0;\n @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(d), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
+__device__ __forceinline__ void u_mma(unsigned d, unsigned a_tmem, unsigned long long db, unsigned idesc, unsigned accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(d), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void u_commit(unsigned elected, unsigned bar) {
-  asm volatile("{\n .reg .pred e;\n setp.ne.b32 e, %1, 0;\n @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar), "r"(elected) : "memory");
+__device__ __forceinline__ void u_commit(unsigned bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
 
 // TN: token columns a block can hold.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W, slices of K), the slices of a tile a
@@ -165,25 +164,27 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       }
     }
   } else if (warp == 17) {                                             // the MMAs
-    pdl_wait();
-    const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17), elected = lane == 0;
-    for (int c = 0; c < steps; ++c) {
-      const int b = c & 1;
-      const unsigned par = (unsigned)((c >> 1) & 1);
-      bool ok = g_wait(parts_full + 8 * b, par, abort_flag);
-      if (!OWN_X) ok = ok && g_wait(x_full + 8 * b, par, abort_flag);
-      if (!__all_sync(0xffffffffu, ok)) { gave_up = true; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const unsigned d = tmem + 192 + b * TN, wp = tmem + b * 96;
-      const unsigned long long xd = g_desc(sx + b * 3 * TN * 128);
-      // (W's part, the tokens' part), 0 the highest: the small products first
-      constexpr int order[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
+    if (lane == 0) {
+      pdl_wait();
+      const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17);
+      for (int c = 0; c < steps; ++c) {
+        const int b = c & 1;
+        const unsigned par = (unsigned)((c >> 1) & 1);
+        if (!g_wait(parts_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
+        if (!OWN_X && !g_wait(x_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const unsigned d = tmem + 192 + b * TN, wp = tmem + b * 96;
+        // One thread issues an MMA in 46 cycles if it only adds to a descriptor, in 75 if it makes each anew; the MMA takes tile_n / 2.
+        const unsigned long long xd = g_desc(sx + b * 3 * TN * 128);
+        // (W's part, the tokens' part), 0 the highest: the small products first
+        constexpr int order[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-      for (int p = 0; p < 6; ++p)
+        for (int p = 0; p < 6; ++p)
 #pragma unroll
-        for (int k = 0; k < 4; ++k)                                    // (a descriptor's address counts 16 bytes)
-          u_mma(elected, d, wp + order[p][0] * 32 + k * 8, xd + (unsigned)(order[p][1] * tile_n * 8 + k * 2), idesc, (p | k) != 0);
-      u_commit(elected, mma_done + 8 * b);
+          for (int k = 0; k < 4; ++k)                                  // (a descriptor's address counts 16 bytes)
+            u_mma(d, wp + order[p][0] * 32 + k * 8, xd + (unsigned)(order[p][1] * tile_n * 8 + k * 2), idesc, (p | k) != 0);
+        u_commit(mma_done + 8 * b);
+      }
     }
   } else {
     const unsigned lanes = tmem + ((unsigned)(quarter * 32) << 16);
@@ -306,12 +307,21 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     }
     u_cluster_sync();
     const int rank = (int)u_cluster_rank();
-    if (warp < 16) {
-      const int n = n0 + (tid & 127);
-      for (int t = rank * 4 + (tid >> 7); t < tile_n && m0 + t < M; t += 4 * slices) {
-        float s = 0.0f;
-        for (int z = 0; z < slices; ++z) s += u_read_peer(sbase + (t * 128 + (tid & 127)) * 4, z);
-        if (n < N) put(m0 + t, n, s);
+    if (warp < 16) {                                                   // a warp a token's 128 sums, all slices asked for together
+      const int n = n0 + 4 * lane;
+      for (int t = rank * 16 + warp; t < tile_n && m0 + t < M; t += 16 * slices) {
+        float4 v[U_MAX_SLICES];
+#pragma unroll
+        for (int z = 0; z < U_MAX_SLICES; ++z)
+          if (z < slices) v[z] = u_read_peer4(sbase + (t * 128 + 4 * lane) * 4, z);
+        float4 o = v[0];
+#pragma unroll
+        for (int z = 1; z < U_MAX_SLICES; ++z)
+          if (z < slices) { o.x += v[z].x; o.y += v[z].y; o.z += v[z].z; o.w += v[z].w; }
+        if (n < N) put(m0 + t, n, o.x);
+        if (n + 1 < N) put(m0 + t, n + 1, o.y);
+        if (n + 2 < N) put(m0 + t, n + 2, o.z);
+        if (n + 3 < N) put(m0 + t, n + 3, o.w);
       }
     }
     u_cluster_sync();                                                  // no block leaves while another still reads its sums
@@ -349,13 +359,13 @@ split_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, int 
 int umma_slices(int N, int K) {
   const int rows = (N + 127) / 128;
   int s = 1;
-  while (s < 8 && rows * s < 128 && K / (2 * s) >= 256) s *= 2;
+  while (s < U_MAX_SLICES && rows * s < 128 && K / (2 * s) >= 256) s *= 2;
   return s;
 }
 
 struct TokenTiles { int tn, count; };
-// Tiles of tokens: as few rounds of blocks over the SMs as the widths allow.  A step's cycles go by its MMAs (6 a token) or by
-// the workers (cutting up W, adding sums, and up to 64 tokens cutting these up too); a block has some 4,000 of its own.
+// Tiles of tokens: as few rounds of blocks over the SMs as the widths allow.  A step's cycles go by its 24 MMAs, half a cycle a
+// token each and 46 at least; a block has some 6,000 of its own.
 TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
   TokenTiles best{16, 1};
   long long best_cost = -1;
@@ -363,8 +373,8 @@ TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
   for (int count = (M + 159) / 160; count <= (M + 15) / 16; ++count) {
     const int tn = ((M + count - 1) / count + 15) / 16 * 16;
     const long long per_sm = tn <= 16 ? 2 : 1, rounds = (blocks * count + sms * per_sm - 1) / (sms * per_sm);
-    const int workers = 600 + (tn <= 64 ? 7 : 3) * tn, mma = 6 * tn;
-    const long long cost = rounds * ((long long)steps * (workers > mma ? workers : mma) * per_sm + 4000);
+    const int mma = 24 * (tn / 2 > 46 ? tn / 2 : 46);
+    const long long cost = rounds * ((long long)steps * mma + 6000);
     if (best_cost < 0 || cost < best_cost) { best = TokenTiles{tn, count}; best_cost = cost; }
   }
   return best;
