@@ -15,7 +15,7 @@
 // multiply-adds in index order, so infinities and NaN come out as they do there.
 //
 // A block takes 128 rows of W, the tile's M rows of the MMA, and tile_n tokens, its N columns.  W arrives as float32 by TMA
-// (128-byte swizzle, K 64 a stage); a thread of sixteen warps reads a quarter of a row's 64 values, cuts them up with bit masks and
+// (128-byte swizzle, K 64 a stage); a worker thread reads its part of a row's 64 values, cuts them up with bit masks and
 // subtractions (exact) and writes the three parts into tensor memory, where the MMA takes its A operand from: the parts never go
 // back to shared memory, whose bandwidth the MMA's B operand (the tokens' three parts) needs.  Up to 64 tokens the same
 // threads cut the tokens' values up as well; for more, split_kernel has done it once for all blocks and TMA brings the parts.
@@ -33,7 +33,14 @@ namespace {
 constexpr int FK64 = 64;                        // K per step
 constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int U_MAX_SLICES = 8;                  // of K: the largest portable cluster
-constexpr int U_WORKERS = 512, U_THREADS = U_WORKERS + 96;   // 16 warps of workers, a warp each for W's copies, the MMAs and the tokens' copies
+#ifndef IFX_PARTS16
+#define IFX_PARTS16 2
+#define IFX_PARTS64 4
+#define IFX_PARTS160 4
+#endif
+// Into how many parts K and the columns are dealt out to the workers, four warps each; a warp each for W's copies, the MMAs and the tokens' copies.
+__host__ __device__ constexpr int u_parts(int tn) { return tn == 16 ? IFX_PARTS16 : tn <= 64 ? IFX_PARTS64 : IFX_PARTS160; }
+__host__ __device__ constexpr int u_threads(int tn) { return 128 * u_parts(tn) + 96; }
 constexpr unsigned U_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // D float32, A and B bfloat16, K-major, M 128; N (in eighths) at bit 17
 
 __host__ __device__ constexpr int u_w_stages(int tn) { return tn == 16 ? 3 : tn <= 64 ? 5 : tn <= 128 ? 4 : 3; }
@@ -91,12 +98,13 @@ __device__ __forceinline__ void u_commit(unsigned bar) {
 // TN: token columns a block can hold.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W, slices of K), the slices of a tile a
 // cluster.  Up to TN 64 A is read here; above, map_x describes split_kernel's parts [3][M][K].
 template <int TN>
-__global__ void __launch_bounds__(U_THREADS, TN == 16 ? 2 : 1)
+__global__ void __launch_bounds__(u_threads(TN), TN == 16 ? 2 : 1)
 gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ A,
                      const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K, long long lda,
                      long long ldc, int tile_n, int slice_steps, int vec_a, int w_fixed, int* __restrict__ error_flag) {
   constexpr bool OWN_X = TN <= 64;
-  constexpr int STAGES = u_w_stages(TN), COLS = TN / 4, X_PER = OWN_X && TN > 32 ? TN / 32 : 1;   // columns, and float4 of the tokens, of a worker
+  constexpr int STAGES = u_w_stages(TN), PARTS = u_parts(TN), WARPS = 4 * PARTS, COLS = TN / PARTS, UNITS = 16 / PARTS;   // a worker's columns, and float4 of W
+  constexpr int X_ROWS = 2 * WARPS, X_PER = OWN_X && TN > X_ROWS ? TN / X_ROWS : 1;                                          // and float4 of the tokens
   extern __shared__ unsigned char u_smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 6];   // w_full[s], w_empty[s], x_full[2], parts_full[2], mma_done[2]
   __shared__ unsigned tmem_slot;
@@ -110,17 +118,17 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     abort_s = 0;
     for (int s = 0; s < STAGES; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(w_full + 8 * s));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(w_empty + 8 * s), "r"(U_WORKERS / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(w_empty + 8 * s), "r"(WARPS));
     }
     for (int b = 0; b < 2; ++b) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(x_full + 8 * b));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(parts_full + 8 * b), "r"(U_WORKERS / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(parts_full + 8 * b), "r"(WARPS));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mma_done + 8 * b));
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
-  if (warp == 17) {
+  if (warp == WARPS + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(g_smem_addr(&tmem_slot)), "n"(u_columns(TN)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
@@ -136,9 +144,9 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   float acc[COLS];
 #pragma unroll
   for (int i = 0; i < COLS; ++i) acc[i] = 0.0f;
-  const int quarter = warp & 3, part = warp >> 2;                      // of a worker: its lanes of tensor memory, its fourth of K and of the columns
+  const int quarter = warp & 3, part = warp >> 2;                      // of a worker: its lanes of tensor memory, its part of K and of the columns
 
-  if (warp == 16) {                                                    // W's copies
+  if (warp == WARPS) {                                                    // W's copies
     if (lane == 0) {
       if (!w_fixed) pdl_wait();
       for (int c = 0; c < steps; ++c) {
@@ -152,7 +160,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                        ::"r"(sbase + st * W_STAGE + h * (W_STAGE / 2)), "l"(&map_w), "r"((step0 + c) * FK64 + 32 * h), "r"(n0), "r"(w_full + 8 * st) : "memory");
       }
     }
-  } else if (warp == 18) {                                             // the tokens' copies
+  } else if (warp == WARPS + 2) {                                             // the tokens' copies
     if (!OWN_X && lane == 0) {
       pdl_wait();
       for (int c = 0; c < steps; ++c) {
@@ -163,7 +171,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                      ::"r"(sx + b * 3 * TN * 128), "l"(&map_x), "r"((step0 + c) * FK64), "r"(m0), "r"(0), "r"(x_full + 8 * b) : "memory");
       }
     }
-  } else if (warp == 17) {                                             // the MMAs
+  } else if (warp == WARPS + 1) {                                             // the MMAs
     if (lane == 0) {
       pdl_wait();
       const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17);
@@ -217,7 +225,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       const int k = (step0 + c) * FK64 + (tid & 15) * 4;
 #pragma unroll
       for (int i = 0; i < X_PER; ++i) {
-        const int t = (tid >> 4) + 32 * i, m = m0 + t;
+        const int t = (tid >> 4) + X_ROWS * i, m = m0 + t;
         xr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < tile_n && m < M && k < K && c < steps) {               // K is a multiple of 4
           const float* p = A + (size_t)m * lda + k;
@@ -233,24 +241,29 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       bool ok = c < 2 || add_sums(c - 2);                              // (and its parts' places are free)
       ok = ok && g_wait(w_full + 8 * st, (unsigned)((c / STAGES) & 1), abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { gave_up = true; break; }
-      const unsigned wrow = sbase + st * W_STAGE + (part >> 1) * (W_STAGE / 2) + row * 128;
-      unsigned hi[8], mid[8], lo[8];
+      const unsigned wrow = sbase + st * W_STAGE + row * 128;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float x, y, z, w;
-        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(wrow + ((((part & 1) * 4 + j) ^ (row & 7)) << 4)) : "memory");
-        cut(x, y, hi[2 * j], mid[2 * j], lo[2 * j]);
-        cut(z, w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
+      for (int g = 0; g < UNITS / 4; ++g) {                            // 16 values at a time
+        unsigned hi[8], mid[8], lo[8];
+        const int u = part * UNITS + g * 4;                            // among the row's 16 units of 16 bytes, eight in each box
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float x, y, z, w;
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w)
+                       : "r"(wrow + (u >> 3) * (W_STAGE / 2) + ((((u & 7) + j) ^ (row & 7)) << 4)) : "memory");
+          cut(x, y, hi[2 * j], mid[2 * j], lo[2 * j]);
+          cut(z, w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
+        }
+        const unsigned at = lanes + b * 96 + u * 2;
+        u_tmem_st8(at, hi);
+        u_tmem_st8(at + 32, mid);
+        u_tmem_st8(at + 64, lo);
       }
-      const unsigned at = lanes + b * 96 + part * 8;
-      u_tmem_st8(at, hi);
-      u_tmem_st8(at + 32, mid);
-      u_tmem_st8(at + 64, lo);
       u_arrive_warp(w_empty + 8 * st, lane);
       if (OWN_X) {
 #pragma unroll
         for (int i = 0; i < X_PER; ++i) {
-          const int t = (tid >> 4) + 32 * i, q = tid & 15;
+          const int t = (tid >> 4) + X_ROWS * i, q = tid & 15;
           if (t >= tile_n) break;
           unsigned h0, m0_, l0, h1, m1, l1;
           cut(xr[i].x, xr[i].y, h0, m0_, l0);
@@ -287,7 +300,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.0f);
   };
   if (slices == 1) {
-    if (warp < 16) {
+    if (warp < WARPS) {
       const int n = n0 + quarter * 32 + lane;
       if (n < N)
 #pragma unroll
@@ -298,7 +311,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     }
   } else {
     __syncthreads();
-    if (warp < 16) {
+    if (warp < WARPS) {
 #pragma unroll
       for (int i = 0; i < COLS; ++i) {
         const int t = part * COLS + i;
@@ -307,9 +320,9 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     }
     u_cluster_sync();
     const int rank = (int)u_cluster_rank();
-    if (warp < 16) {                                                   // a warp a token's 128 sums, all slices asked for together
+    if (warp < WARPS) {                                                // a warp a token's 128 sums, all slices asked for together
       const int n = n0 + 4 * lane;
-      for (int t = rank * 16 + warp; t < tile_n && m0 + t < M; t += 16 * slices) {
+      for (int t = rank * WARPS + warp; t < tile_n && m0 + t < M; t += WARPS * slices) {
         float4 v[U_MAX_SLICES];
 #pragma unroll
         for (int z = 0; z < U_MAX_SLICES; ++z)
@@ -328,7 +341,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(u_columns(TN)) : "memory");
+  if (warp == WARPS + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(u_columns(TN)) : "memory");
 }
 
 // A's values cut into their parts [3][M][pitch] (zeros behind K), eight a thread.
@@ -416,7 +429,7 @@ int launch_umma_f32(const float* A, const float* W, const float* bias, float* C,
     int rc = launch_pdl(split_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, A, (uint4*)scratch, M, K, lda, pitch, (int)vec_a);
     if (rc) return rc;
   }
-  const int rc = launch_pdl_cluster(kern, dim3(count, (N + 127) / 128, slices), dim3(U_THREADS), (size_t)u_smem(TN), stream, dim3(1, 1, slices),
+  const int rc = launch_pdl_cluster(kern, dim3(count, (N + 127) / 128, slices), dim3(u_threads(TN)), (size_t)u_smem(TN), stream, dim3(1, 1, slices),
                                     map_w, map_x, A, W, bias, C, M, N, K, lda, ldc, tn, steps, (int)vec_a, w_fixed, error_flag);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
