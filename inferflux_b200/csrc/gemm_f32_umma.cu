@@ -33,13 +33,13 @@ namespace {
 constexpr int FK64 = 64;                        // K per step
 constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int U_MAX_SLICES = 8;                  // of K: the largest portable cluster
-#ifndef IFX_PARTS16
-#define IFX_PARTS16 2
-#define IFX_PARTS64 4
-#define IFX_PARTS160 4
+#ifndef IFX_SL
+#define IFX_SL 256
 #endif
-// Into how many parts K and the columns are dealt out to the workers, four warps each; a warp each for W's copies, the MMAs and the tokens' copies.
-__host__ __device__ constexpr int u_parts(int tn) { return tn == 16 ? IFX_PARTS16 : tn <= 64 ? IFX_PARTS64 : IFX_PARTS160; }
+// Into how many parts K and the columns are dealt out to the workers, four warps each.  (With twice as many warps of workers 1 row x N 22,016
+// K 2,048 took 46 us instead of 43, 301 rows x N 2,048 K 11,008 105 instead of 103: they are in the issuing thread's way.)
+__host__ __device__ constexpr int u_parts(int tn) { return tn == 16 ? 1 : 2; }
+// the workers, and a warp each for W's copies, the MMAs and the tokens' copies
 __host__ __device__ constexpr int u_threads(int tn) { return 128 * u_parts(tn) + 96; }
 constexpr unsigned U_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // D float32, A and B bfloat16, K-major, M 128; N (in eighths) at bit 17
 
@@ -372,13 +372,13 @@ split_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, int 
 int umma_slices(int N, int K) {
   const int rows = (N + 127) / 128;
   int s = 1;
-  while (s < U_MAX_SLICES && rows * s < 128 && K / (2 * s) >= 256) s *= 2;
+  while (s < U_MAX_SLICES && rows * s < IFX_SL && K / (2 * s) >= 256) s *= 2;
   return s;
 }
 
 struct TokenTiles { int tn, count; };
-// Tiles of tokens: as few rounds of blocks over the SMs as the widths allow.  A step's cycles go by its 24 MMAs, half a cycle a
-// token each and 46 at least; a block has some 6,000 of its own.
+// Tiles of tokens: as few rounds of blocks over the SMs as the widths allow.  A step's cycles go by its 24 MMAs: 97 each with
+// 160 tokens, 76 with up to 120 (issuing one beside the workers takes that long); a block has some 6,000 of its own.
 TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
   TokenTiles best{16, 1};
   long long best_cost = -1;
@@ -386,7 +386,7 @@ TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
   for (int count = (M + 159) / 160; count <= (M + 15) / 16; ++count) {
     const int tn = ((M + count - 1) / count + 15) / 16 * 16;
     const long long per_sm = tn <= 16 ? 2 : 1, rounds = (blocks * count + sms * per_sm - 1) / (sms * per_sm);
-    const int mma = 24 * (tn / 2 > 46 ? tn / 2 : 46);
+    const int mma = 24 * (tn * 3 / 5 > 76 ? tn * 3 / 5 : 76);
     const long long cost = rounds * ((long long)steps * mma + 6000);
     if (best_cost < 0 || cost < best_cost) { best = TokenTiles{tn, count}; best_cost = cost; }
   }
