@@ -22,8 +22,10 @@
 // Parts and sums are double-buffered: while the MMAs of one step run, the threads add the sums of the step before it and
 // cut up the values of the step behind it.
 //
-// What bounds it: six MMAs a product, so 2,250 / 6 = 375 TFLOP/s at most; with few tokens reading W.  301 rows: N 22,016 K 2,048
-// 155 us (623 by multiply-adds), N 2,048 K 11,008 106 us (373), N 2,560 K 2,048 44 us (94); 16 rows 49 us (111), 35 (76), 10 (17).
+// What bounds it: six MMAs a product, so 2,250 / 6 = 375 TFLOP/s at most, and the thread that issues them (78 cycles each beside
+// the workers, while an MMA takes half a cycle a token); with few tokens reading W.  Us here (by multiply-adds), 301 rows: N 22,016
+// K 2,048 150 (623), N 2,048 K 11,008 103 (372), N 2,560 K 2,048 41 (93); 16 rows 48 (111), 32 (76), 10 (17); 1 row 44 (42), 32 (26),
+// 9.0 (7.4), N 151,936 K 2,048 202 (208): a single row's blocks wait for one another's steps, and stay here for the sake of its bits.
 #include "gemm_f32_umma.h"
 #include "umma.cuh"
 #include <float.h>
@@ -33,9 +35,6 @@ namespace {
 constexpr int FK64 = 64;                        // K per step
 constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int U_MAX_SLICES = 8;                  // of K: the largest portable cluster
-#ifndef IFX_SL
-#define IFX_SL 256
-#endif
 // Into how many parts K and the columns are dealt out to the workers, four warps each.  (With twice as many warps of workers 1 row x N 22,016
 // K 2,048 took 46 us instead of 43, 301 rows x N 2,048 K 11,008 105 instead of 103: they are in the issuing thread's way.)
 __host__ __device__ constexpr int u_parts(int tn) { return tn == 16 ? 1 : 2; }
@@ -368,11 +367,12 @@ split_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, int 
   for (int q = 0; q < 3; ++q) parts[(long long)q * M * groups + i] = o[q];
 }
 
-// Slices of K, from N and K alone (1, 2, 4 or 8): a narrow product's blocks fill the SMs, each slice at least 256 long.
+// Slices of K, from N and K alone (1, 2, 4 or 8), each at least 256 long: blocks enough that their last round is a small part of
+// all (N 22,016 K 2,048 in two slices instead of one: 160 rows 99 -> 88 us, 77 rows 80 -> 71, 1 row 44 in both).
 int umma_slices(int N, int K) {
   const int rows = (N + 127) / 128;
   int s = 1;
-  while (s < U_MAX_SLICES && rows * s < IFX_SL && K / (2 * s) >= 256) s *= 2;
+  while (s < U_MAX_SLICES && rows * s < 256 && K / (2 * s) >= 256) s *= 2;
   return s;
 }
 
