@@ -21,8 +21,8 @@
 //
 // Barriers (same offsets in both blocks): full[s] counts the bytes of both blocks' copies and lives in
 // the leader (the other block's TMA completes on it; no multicast); empty[s] and acc_full[a] are
-// arrived on in both blocks by one tcgen05.commit; acc_empty[a] in the leader counts the 256 epilogue
-// threads of both blocks.  The pair synchronises as a cluster after set-up and before it frees tensor
+// arrived on in both blocks by one tcgen05.commit; acc_empty[a] in the leader counts the epilogue
+// warps of both blocks.  The pair synchronises as a cluster after set-up and before it frees tensor
 // memory, so neither block leaves while the other may still signal it.
 //
 // A block sets itself up before it waits for the kernel ahead of it in the stream.  Where the caller says that W is fixed
@@ -85,7 +85,11 @@ constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + 1024;
 // Modes 2 and 6 (few tokens): a stage is as small as the tile's rows and the tokens allow, and there are as many as fit.
 constexpr int S_MAX_STAGES = 12;
 constexpr int S_SMEM = 212 * 1024;                    // with 1 KB for alignment and 16 KB behind the last stage, which the MMA may read (see below)
-constexpr int P_THREADS = 192;                        // producer warp, MMA warp, 4 epilogue warps
+// Producer warp, MMA warp, and the warps of the epilogue: four, or with few tokens, where a pair has a tile or two and nothing
+// runs beside the last one's epilogue, sixteen, which take 16 of the columns in turn (gate and up of the 3B sizes, 23 / 77 / 128
+// rows: EPI_FIGURES).
+__host__ __device__ constexpr int epilogue_warps(int mode) { return mode == 2 || mode == 6 ? 16 : 4; }
+__host__ __device__ constexpr int pair_threads(int mode) { return 64 + 32 * epilogue_warps(mode); }
 constexpr unsigned LEADER_MASK = 0xFEFFFFFFu;         // a shared-memory address of this block -> the same place in the pair's leader
 // kind::f16 instruction descriptor: D float32, A and B bfloat16, both K-major, M 256 (over the pair), N 256
 constexpr unsigned P_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(256 >> 4) << 24);   // N (in eighths) goes to bits 17-22
@@ -122,6 +126,12 @@ __device__ __forceinline__ void g_tmem_ld16(unsigned taddr, float (&v)[32]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) { v[i] = __uint_as_float(r[i]); v[16 + i] = 0.0f; }
 }
+__device__ __forceinline__ void g_tmem_ld16(unsigned taddr, float (&v)[16]) {
+  float w[32];
+  g_tmem_ld16(taddr, w);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = w[i];
+}
 __device__ __forceinline__ void p_commit_both(unsigned bar) {      // arrives on this barrier in both blocks of the pair
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
                ::"r"(bar), "h"((unsigned short)3) : "memory");
@@ -154,7 +164,7 @@ struct QkvEpilogue {
 // silu(gate) * up.  In both a tile has tile_h <= 256 rows (a multiple of 16) of which each block loads half: the MMA still
 // works on 128 rows a block, and what the others hold is never read.
 template <int MODE, typename TOut>
-__global__ void __launch_bounds__(P_THREADS, 1)
+__global__ void __launch_bounds__(pair_threads(MODE), 1)
 gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       TOut* __restrict__ out, long long ldo, const float* __restrict__ bias, int M, int n_out, int K,
                       int tile_n, int* __restrict__ error_flag, int k_parts, long long part_stride, QkvEpilogue qe,
@@ -187,7 +197,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     for (int a = 0; a < 2; ++a) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_acc_full + 8 * a));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;\n" ::"r"(bar_acc_empty + 8 * a));   // epilogue threads of both blocks
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar_acc_empty + 8 * a), "r"(2 * epilogue_warps(MODE)));   // epilogue warps of both blocks
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -283,10 +293,11 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           if (!g_wait(bar_full + 8 * stage, phase, abort_flag)) { gave_up = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           const unsigned sa = sbase + stage * stage_bytes, sw = sa + w_at;
+          const unsigned long long da = g_desc(sa), dw = g_desc(sw), du = g_desc(sa + a_bytes);   // an address counts 16 bytes
 #pragma unroll
           for (int k = 0; k < TK / 16; ++k) {
-            p_mma(d, g_desc(sa + k * 32), g_desc(sw + k * 32), idesc, ks != ks0 || k != 0);
-            if (SKINNY_GLU) p_mma(d + 128, g_desc(sa + a_bytes + k * 32), g_desc(sw + k * 32), idesc, ks != ks0 || k != 0);
+            p_mma(d, da + 2 * k, dw + 2 * k, idesc, ks != ks0 || k != 0);
+            if (SKINNY_GLU) p_mma(d + 128, du + 2 * k, dw + 2 * k, idesc, ks != ks0 || k != 0);
           }
           p_commit_both(bar_empty + 8 * stage);                  // both blocks' stage is free once these MMAs have read it
           if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -295,7 +306,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, group = (warp - 2) >> 2;       // group: of the warps with the same quarter of the lanes
     const int row_in_tile = (int)rank * half_h + quarter * 32 + lane;
     const bool row_there = quarter * 32 + lane < half_h;         // (modes 2 and 6: tiles of fewer than 256 rows)
     pdl_wait();
@@ -314,14 +325,14 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       TOut* orow = out + (size_t)(row < M ? row : 0) * (SKINNY ? 1 : ldo);
       if (SKINNY_GLU) {                                          // this lane's row of gate and up is a column of the output
 #pragma unroll 1
-        for (int c = 0; c * 32 < tile_n; ++c) {
-          float g[32], u[32];
-          if (tile_n - c * 32 >= 32) { g_tmem_ld32(taddr + c * 32, g); g_tmem_ld32(taddr + 128 + c * 32, u); }
-          else { g_tmem_ld16(taddr + c * 32, g); g_tmem_ld16(taddr + 128 + c * 32, u); }
+        for (int c = group; c * 16 < tile_n; c += epilogue_warps(MODE) / 4) {
+          float g[16], u[16];
+          g_tmem_ld16(taddr + c * 16, g);
+          g_tmem_ld16(taddr + 128 + c * 16, u);
           if (row < M && row_there) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int token = c * 32 + i;
+            for (int i = 0; i < 16; ++i) {
+              const int token = c * 16 + i;
               if (token < n_out) orow[(size_t)token * ldo] = Num<TOut>::from_f(g[i] / (1.0f + __expf(-g[i])) * u[i]);
             }
           }
@@ -329,14 +340,13 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       } else if (SKINNY) {                                       // this lane's row of the weights is a column of the output
         TOut* opart = orow + (size_t)(t / m_tiles) * part_stride;
 #pragma unroll 1
-        for (int c = 0; c * 32 < tile_n; ++c) {
-          float v[32];
-          if (tile_n - c * 32 >= 32) g_tmem_ld32(taddr + c * 32, v);
-          else g_tmem_ld16(taddr + c * 32, v);                   // warp-uniform: the tile's last 16 columns
+        for (int c = group; c * 16 < tile_n; c += epilogue_warps(MODE) / 4) {
+          float v[16];
+          g_tmem_ld16(taddr + c * 16, v);
           if (row < M && row_there) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int token = c * 32 + i;
+            for (int i = 0; i < 16; ++i) {
+              const int token = c * 16 + i;
               if (token < n_out) opart[(size_t)token * ldo] = (TOut)v[i];   // a warp's lanes write 32 neighbours
             }
           }
@@ -453,7 +463,8 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-      p_arrive_leader(bar_acc_empty + 8 * acc);                  // this thread has read its part of the accumulator
+      __syncwarp();
+      if (lane == 0) p_arrive_leader(bar_acc_empty + 8 * acc);   // this warp has read its part of the accumulator
     }
   }
   if (gave_up) {                                                 // a wait ran out: tell everyone, let copies in flight land
@@ -517,7 +528,7 @@ int launch_gemm_pair(const void* A, long long lda, const void* W, const float* b
   if (rc) return rc;
   const int tiles = ((M + 255) / 256) * ((n_out + out_cols - 1) / out_cols);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
+  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(pair_threads(MODE)), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
                           ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, (const int*)nullptr, 0, glu, 256, P_STAGES, w_fixed);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
@@ -546,7 +557,7 @@ int launch_gemm_grouped(const void* A, long long lda, const void* W, void* out, 
   if (rc) return rc;
   const int tiles = ((M + 255) / 256) * ((n_out + out_cols - 1) / out_cols);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
+  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(pair_threads(MODE)), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, (TOut*)out,
                           ldo, (const float*)nullptr, M, n_out, K, tile_n, error_flag, 1, 0ll, QkvEpilogue{}, tile_expert, expert_rows, glu, 256, P_STAGES, 0);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
@@ -607,7 +618,7 @@ int launch_gemm_qkv(const void* A, long long lda, const void* W, const float* bi
   if (rc) return rc;
   const int tiles = ((M + 255) / 256) * ((n_out + tile_n - 1) / tile_n);
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, q_out,
+  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(pair_threads(3)), (size_t)P_SMEM, stream, dim3(2, 1, 1), map_a, map_w, q_out,
                           ldo, bias, M, n_out, K, tile_n, error_flag, 1, 0ll, qe, (const int*)nullptr, 0, GluShape{}, 256, P_STAGES, w_fixed);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
@@ -637,7 +648,7 @@ int launch_gemm_skinny(const void* X, long long ldx, const void* W, TOut* out, l
   if (rc) return rc;
   const int tiles = ((n_out + plan.h - 1) / plan.h) * plan.parts;
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)S_SMEM, stream, dim3(2, 1, 1), map_w, map_x, out, ldo,
+  rc = launch_pdl_cluster(kern, dim3(2 * pairs), dim3(pair_threads(MODE)), (size_t)S_SMEM, stream, dim3(2, 1, 1), map_w, map_x, out, ldo,
                           (const float*)nullptr, n_out, tokens, K, tile_n, error_flag, plan.parts, part_stride, QkvEpilogue{},
                           (const int*)nullptr, 0, GluShape{}, plan.h, stages, w_fixed);
   return rc ? rc : IFX_LAUNCH_CHECK();
