@@ -85,10 +85,11 @@ constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + 1024;
 // Modes 2 and 6 (few tokens): a stage is as small as the tile's rows and the tokens allow, and there are as many as fit.
 constexpr int S_MAX_STAGES = 12;
 constexpr int S_SMEM = 212 * 1024;                    // with 1 KB for alignment and 16 KB behind the last stage, which the MMA may read (see below)
-// Producer warp, MMA warp, and the warps of the epilogue: four, or with few tokens, where a pair has a tile or two and nothing
-// runs beside the last one's epilogue, sixteen, which take 16 of the columns in turn (gate and up of the 3B sizes, 23 / 77 / 128
-// rows: EPI_FIGURES).
-__host__ __device__ constexpr int epilogue_warps(int mode) { return mode == 2 || mode == 6 ? 16 : 4; }
+// Producer warp, MMA warp, and the warps of the epilogue: four, or for gate and up of few tokens sixteen, which take 16 of the columns
+// in turn: a pair has a tile or two there, so nothing runs beside the last one's activation, which took four warps 4 to 9 us (16 / 4
+// warps: 3B sizes 23, 64 and 128 rows 20.0 / 20.9, 21.2 / 24.8 and 23.4 / 30.6 us, 7B 44.8 / 45.5, 45.7 / 49.4 and 49.6 / 56.8; without
+// an activation the stores are the time and four warps are ahead by 0.5 us).
+__host__ __device__ constexpr int epilogue_warps(int mode) { return mode == 6 ? 16 : 4; }
 __host__ __device__ constexpr int pair_threads(int mode) { return 64 + 32 * epilogue_warps(mode); }
 constexpr unsigned LEADER_MASK = 0xFEFFFFFFu;         // a shared-memory address of this block -> the same place in the pair's leader
 // kind::f16 instruction descriptor: D float32, A and B bfloat16, both K-major, M 256 (over the pair), N 256
@@ -340,13 +341,14 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       } else if (SKINNY) {                                       // this lane's row of the weights is a column of the output
         TOut* opart = orow + (size_t)(t / m_tiles) * part_stride;
 #pragma unroll 1
-        for (int c = group; c * 16 < tile_n; c += epilogue_warps(MODE) / 4) {
-          float v[16];
-          g_tmem_ld16(taddr + c * 16, v);
+        for (int c = 0; c * 32 < tile_n; ++c) {
+          float v[32];
+          if (tile_n - c * 32 >= 32) g_tmem_ld32(taddr + c * 32, v);
+          else g_tmem_ld16(taddr + c * 32, v);                   // warp-uniform: the tile's last 16 columns
           if (row < M && row_there) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const int token = c * 16 + i;
+            for (int i = 0; i < 32; ++i) {
+              const int token = c * 32 + i;
               if (token < n_out) opart[(size_t)token * ldo] = (TOut)v[i];   // a warp's lanes write 32 neighbours
             }
           }

@@ -67,10 +67,8 @@ class SwiGLU(Part):
             ops.gemm_umma(x, w, None, act, swiglu=True, w_fixed=True)       # many rows: tcgen05 product, activation in its epilogue
         elif fused and x.is_contiguous() and x.data_ptr() % 16 == 0:
             # 17 to 128 rows: the weights as the tiles' rows, one rounding from float32 sums.  us at 17 / 64 / 128 rows, against library
-            # product and activation kernel (which round to bfloat16 in between): 7B sizes 43.7 / 48.2 / 55.0 against 46.9 / 49.6 / 54.2,
-            # 14B 46.6 / 51.1 / 57.5 against 48.3 / 50.1 / 59.1, 3B 19.9 / 24.0 / 29.6 against 18.2 / 19.5 / 22.0; a whole captured step
-            # (6 layers) takes 0.96 to 1.00 of the time at the 7B and 14B sizes and 1.00 to 1.06 at the 3B ones (1.02 at 64 rows), a
-            # step that the host launches 0.87 to 0.89 at the 3B sizes, 0.87 to 0.96 at the 7B, 0.98 to 1.01 at the 14B.
+            # product and activation kernel (which round to bfloat16 in between): 7B sizes 44.7 / 45.7 / 49.6 against 46.9 / 49.6 / 54.2,
+            # 14B 47.8 / 49.0 / 52.3 against 48.3 / 50.1 / 59.1, 3B 20.1 / 21.2 / 23.4 against 18.2 / 19.5 / 22.0.
             ops.gemm_umma_skinny_glu(x, w, act, True)
         else:
             ops.swiglu(self.gate_up.forward(x), act)
