@@ -432,17 +432,21 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           float gate[32], up[32];
           g_tmem_ld32(taddr + c * 32, gate);
           g_tmem_ld32(taddr + 128 + c * 32, up);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (MODE == 5) {
-              const float g = fminf(gate[i], glu.limit), u = fminf(fmaxf(up[i], -glu.limit), glu.limit);
-              gate[i] = g / (1.0f + __expf(-glu.alpha * g)) * (u + glu.shift);
-            } else {
-              gate[i] = gate[i] / (1.0f + __expf(-gate[i])) * up[i];
-            }
-          }
+          // Rows beyond M hold zeros, and a division of 0 leaves the short way through the divide: with their activations worked out
+          // as well 540 rows of the 7B sizes took 150 us and 129 rows of the 3B ones 71, more than 768 and 256 rows do.
           const int col = n0 + c * 32;
-          if (row < M && col < n_out) store_row32<TOut>(orow + col, gate, min(32, n_out - col), vec && (col % 8 == 0));
+          if (row < M && col < n_out) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (MODE == 5) {
+                const float g = fminf(gate[i], glu.limit), u = fminf(fmaxf(up[i], -glu.limit), glu.limit);
+                gate[i] = g / (1.0f + __expf(-glu.alpha * g)) * (u + glu.shift);
+              } else {
+                gate[i] = gate[i] / (1.0f + __expf(-gate[i])) * up[i];
+              }
+            }
+            store_row32<TOut>(orow + col, gate, min(32, n_out - col), vec && (col % 8 == 0));
+          }
         }
       } else {
 #pragma unroll 1
