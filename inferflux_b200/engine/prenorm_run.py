@@ -99,9 +99,12 @@ class PrenormRun:
         s.entry_q_start, s.entry_q_len, s.entry_ctx_start = (t.data_ptr() for t in (ctx.entry_q_start, ctx.entry_q_len, ctx.entry_ctx_start))
         s.num_pages = ops.paged_pool_pages(k, v, page_stride, nkv * ctx.page_size * hd)
         s.scale = first.scale
-        s.n_tiles, s.tile_rows = step.n_umma_tiles, step.umma_tile_rows
-        s.tile_entry, s.tile_q0 = step.umma_tile_entry.data_ptr(), step.umma_tile_q0.data_ptr()
-        s.n_splits = prefill_plan(ctx, 2, step.umma_tile_rows, nh, ctx.max_ctx_len, 0)[0]
+        splits, umma_us, mma_us = prefill_plan(ctx, 2, step.umma_tile_rows, nh, ctx.max_ctx_len, 0)
+        if mma_us < umma_us:
+            s.n_tiles, s.tile_entry, s.tile_q0 = step.n_chunk_tiles, step.chunk_tile_entry.data_ptr(), step.chunk_tile_q0.data_ptr()
+        else:
+            s.n_tiles, s.tile_rows, s.n_splits = step.n_umma_tiles, step.umma_tile_rows, splits
+            s.tile_entry, s.tile_q0 = step.umma_tile_entry.data_ptr(), step.umma_tile_q0.data_ptr()
         if s.n_splits > 1:
             rows = ops.attn_prefill_cut_units(s.n_tiles, nh) * s.n_splits * ops.UMMA_ATTENTION_TILE
             s.part_o, s.part_ml = scratch(f32, rows * hd), scratch(f32, rows * 2)
