@@ -29,11 +29,6 @@ IFX_API int ifx_attn_prefill_umma(const void* q, long long q_stride, void* out, 
                                   float scale, int window, int* error_flag, float* part_o, float* part_ml, int n_splits,
                                   int num_pages, int tile_rows, const float* gate, int gate_parts, long long gate_part_stride,
                                   int gate_stride, cudaStream_t stream);
-IFX_API int ifx_attn_prefill_bf16(const void* q, long long q_stride, void* out, long long out_stride, void* k_layer, void* v_layer,
-                                  long long page_stride, int page_size, const int* block_tables, int bt_stride,
-                                  const int* tile_entry, const int* tile_q0, int n_tiles, const int* entry_q_start,
-                                  const int* entry_q_len, const int* entry_ctx_start, int n_heads, int n_kv, int head_dim,
-                                  float scale, int window, cudaStream_t stream);
 IFX_API int ifx_attn_decode_bf16(const void* q, long long q_stride, void* out, long long out_stride, void* k_layer, void* v_layer,
                                  long long page_stride, int page_size, const int* block_tables, int bt_stride,
                                  const int* dec_entries, int n_dec, const int* entry_q_start, const int* entry_q_len,
@@ -60,7 +55,7 @@ struct PrenormStep {
   long long page_stride;
   int rows, hidden, inter, n_heads, n_kv, page_size, bt_stride, num_pages;
   int qkv_parts, o_parts, down_parts;
-  int n_tiles, tile_rows, n_splits;                 // of the prompt portions; n_splits 0: the mma.sync kernel, tiles of 64
+  int n_tiles, tile_rows, n_splits;                 // of the prompt portions
   int n_dec, dec_splits, dec_pieces;                // single tokens: dec_pieces > 0: shared out by tiles, else dec_splits parts of the keys
   float scale;
 };
@@ -87,12 +82,7 @@ IFX_API int ifx_prenorm_layers(const PrenormStep* step, const PrenormLayer* laye
     if (!rc) rc = ifx_qkv_rope_kv_write(s.qkv, IFX_BF16, l.qkv_bias, s.cos_t, s.sin_t, hd, s.slot_map, l.k_layer, l.v_layer, s.page_stride,
                                         s.page_size, s.rows, s.n_heads, s.n_kv, hd, s.qkv_sums, s.qkv_parts, s.stream);
     n += 3;
-    if (!rc && s.n_tiles && !s.n_splits) {
-      rc = ifx_attn_prefill_bf16(s.qkv, width, s.attn, nq, l.k_layer, l.v_layer, s.page_stride, s.page_size, s.block_tables, s.bt_stride,
-                                 s.tile_entry, s.tile_q0, s.n_tiles, s.entry_q_start, s.entry_q_len, s.entry_ctx_start, s.n_heads, s.n_kv, hd,
-                                 s.scale, 0, s.stream);
-      n += 1;
-    } else if (!rc && s.n_tiles) {
+    if (!rc && s.n_tiles) {
       rc = ifx_attn_prefill_umma(s.qkv, width, s.attn, nq, l.k_layer, l.v_layer, s.page_stride, s.page_size, s.block_tables, s.bt_stride,
                                  s.tile_entry, s.tile_q0, s.n_tiles, s.entry_q_start, s.entry_q_len, s.entry_ctx_start, s.n_heads, s.n_kv, hd,
                                  s.scale, 0, s.error_flag, s.part_o, s.part_ml, s.n_splits, s.num_pages, s.tile_rows, nullptr, 0, 0, 0, s.stream);

@@ -18,6 +18,7 @@ from ..parts.attention import GQAttention, prefill_plan
 from ..parts.base import PartialSums
 from ..parts.block import PreNormBlock
 from ..parts.feed_forward import SwiGLU
+from ..parts.linear import FEW_ROWS_MIN_K
 from ..parts.norm import RMSNorm
 
 
@@ -42,7 +43,8 @@ class PrenormRun:
             if a.window or a.kv_shared or not info.writes_kv or a.head_dim != ops.UMMA_ATTENTION_HEAD_DIM or a.params.get("o_bias"):
                 return None
             shapes.add((info.kv_group, block.position_name, a.hidden, a.n_heads, a.n_kv, a.scale, block.feed_forward.intermediate))
-        if len(shapes) != 1 or blocks[0].mixer.hidden % 8 or blocks[0].feed_forward.intermediate % 8:
+        # (a shorter down projection goes to the library, which the call does not reach)
+        if len(shapes) != 1 or blocks[0].mixer.hidden % 8 or blocks[0].feed_forward.intermediate % 8 or blocks[0].feed_forward.intermediate < FEW_ROWS_MIN_K:
             return None
         return PrenormRun(blocks)
 
@@ -99,12 +101,9 @@ class PrenormRun:
         s.entry_q_start, s.entry_q_len, s.entry_ctx_start = (t.data_ptr() for t in (ctx.entry_q_start, ctx.entry_q_len, ctx.entry_ctx_start))
         s.num_pages = ops.paged_pool_pages(k, v, page_stride, nkv * ctx.page_size * hd)
         s.scale = first.scale
-        splits, umma_us, mma_us = prefill_plan(ctx, 2, step.umma_tile_rows, nh, ctx.max_ctx_len, 0)
-        if mma_us < umma_us:
-            s.n_tiles, s.tile_entry, s.tile_q0 = step.n_chunk_tiles, step.chunk_tile_entry.data_ptr(), step.chunk_tile_q0.data_ptr()
-        else:
-            s.n_tiles, s.tile_rows, s.n_splits = step.n_umma_tiles, step.umma_tile_rows, splits
-            s.tile_entry, s.tile_q0 = step.umma_tile_entry.data_ptr(), step.umma_tile_q0.data_ptr()
+        s.n_tiles, s.tile_rows = step.n_umma_tiles, step.umma_tile_rows
+        s.tile_entry, s.tile_q0 = step.umma_tile_entry.data_ptr(), step.umma_tile_q0.data_ptr()
+        s.n_splits = prefill_plan(ctx, 2, step.umma_tile_rows, nh, ctx.max_ctx_len, 0)[0]
         if s.n_splits > 1:
             rows = ops.attn_prefill_cut_units(s.n_tiles, nh) * s.n_splits * ops.UMMA_ATTENTION_TILE
             s.part_o, s.part_ml = scratch(f32, rows * hd), scratch(f32, rows * 2)

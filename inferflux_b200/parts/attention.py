@@ -257,8 +257,8 @@ class GQAttention(Part):
 
     def attend(self, qkv, attn, ctx, step, g, k_layer, v_layer, page_stride) -> None:
         """bfloat16 with a head size the tensor-core kernels take: prompt
-        portions go to the tcgen05 kernel (head size 128, but for short ones) or the mma.sync
-        kernel, single tokens to the split decode kernel; anything else (float32,
+        portions go to the tcgen05 kernel (head size 128) or the mma.sync kernel
+        (64), single tokens to the split decode kernel; anything else (float32,
         other head sizes) to the generic kernel."""
         common = (ctx.entry_q_start, ctx.entry_q_len, ctx.entry_ctx_start)
         if qkv.dtype != torch.bfloat16 or self.head_dim not in ops.FAST_ATTENTION_HEAD_DIMS:
@@ -266,15 +266,9 @@ class GQAttention(Part):
                                    ctx.block_tables[g], step.tile_entry, step.tile_q0, step.n_tiles, *common,
                                    self.n_heads, self.n_kv, self.head_dim, self.scale, self.window)
             return
-        # Of the two kernels the one whose expected time is the shorter: the mma.sync kernel for prompts of up to 128 tokens or so
-        # (16 heads, us, mma.sync / tcgen05: 20 tokens 4.8 / 6.8, 77 6.0 / 8.2, 128 6.6 / 8.2, 150 7.4 / 8.5 but planned as tcgen05, 256
-        # 9.3 / 9.4, 509 16.4 / 11.6; 3 x 100 tokens 6.9 / 8.3; 64 behind 1,000 25.3 / 17.5).
-        umma = step.n_chunk_tiles > 0 and self.head_dim == ops.UMMA_ATTENTION_HEAD_DIM
-        if umma:
+        if step.n_chunk_tiles and self.head_dim == ops.UMMA_ATTENTION_HEAD_DIM:
             max_keys = min(ctx.max_ctx_len, self.window + 128) if self.window else ctx.max_ctx_len
-            splits, umma_us, mma_us = prefill_plan(ctx, 2, step.umma_tile_rows, self.n_heads, max_keys, self.window)
-            umma = umma_us <= mma_us
-        if umma:
+            splits = prefill_plan(ctx, 2, step.umma_tile_rows, self.n_heads, max_keys, self.window)[0]
             ops.attn_prefill_umma(qkv, qkv.stride(0), attn, k_layer, v_layer, page_stride, ctx.page_size,
                                   ctx.block_tables[g], step.umma_tile_entry, step.umma_tile_q0, step.n_umma_tiles,
                                   *common, self.n_heads, self.n_kv, self.head_dim, self.scale, self.window, splits,
