@@ -2,8 +2,8 @@
 
 The reference issues one cuBLAS call per projection with float32 accumulation
 (runtime/backends/cuda/native/cublas_gemm.cpp:84-102, ``C[M,N] = A[M,K] *
-B[N,K]^T``).  Here a float32 weight goes through the FFMA kernel of the 32-bit
-path; a bfloat16 weight goes through the library (cuBLAS via ``torch.mm``) for
+B[N,K]^T``).  Here a float32 weight goes through the products of the 32-bit
+path (gemm_f32.cu, gemm_f32_umma.cu); a bfloat16 weight goes through the library (cuBLAS via ``torch.mm``) for
 many rows, through the weight-streaming kernel (gemv_bf16.cu) for up to 8
 rows, and through the tcgen05 kernel with the operands' places changed
 (gemm_umma.cu) for 9 to 128 rows where the consumer adds partial sums and K is
