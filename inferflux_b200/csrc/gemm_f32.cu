@@ -25,6 +25,8 @@
 // the blocks; the same sums): 64 rows x N 300 x K 96 6.2 us against 9.9, 17 x 1,000 x 333 16.6 / 24.6, 64 x 512 x 512
 // 14.4 / 24.6 (8.2, 20.1 and 34.4 by 64 x 64 blocks of 4 x 4 a thread).
 //
+// (These sizes go to the tensor cores now, but with rows of W off the 16-byte boundaries or K no multiple of 4.)
+//
 // Up to 16 rows (few_kernel; from 9 on only where ifx_gemm_f32 says so): bound by reading W.  A thread owns one output column and
 // runs along its row of W, which arrives through a ring of cp.async copies.  One row
 // against N 151,936 K 2,048: 205 us, 6.0 TB/s (1,406 us by 64 x 64 blocks).

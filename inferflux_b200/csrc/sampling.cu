@@ -529,7 +529,8 @@ __device__ unsigned radix_threshold(SampleShared& sh, const float* w, int n, flo
   return prefix > floor_bits ? prefix : floor_bits;
 }
 
-// Bound by latency: a row goes through its blocks' shared memory a few times, with a barrier of the cluster between.  So the
+// Bound by latency: a row goes through its blocks' shared memory a few times, with a barrier of the cluster between (152,064 logits, 8 / 64
+// rows: temperature alone 15.5 / 43 us, top-p 27 / 82, top-k and top-p 28 / 85, where each level was made by the whole cluster 31 / 105 and 44 / 144).  So the
 // first level of the first histogram is made while the weights are, the mass that top-p refers to is the histogram's own sum,
 // and the masses for the draw are added once, by the segments that the draw then looks into.
 __global__ void __launch_bounds__(SC_THREADS, 2)        // two blocks per SM: 32 registers a thread
