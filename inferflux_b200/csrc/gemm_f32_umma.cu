@@ -1,9 +1,10 @@
 // float32 matrix product C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) on the tcgen05 tensor cores, for matrices that are not small.
 //
-// The tensor cores have no float32 operands.  A float32 number is the exact sum of three bfloat16 numbers, its 24 bits cut
-// into eights from the top (the exponent ranges are the same, so nothing overflows), and the product of two such numbers is
-// exact in float32.  Of the nine products of parts the six largest are taken; the three others together are below 2^-23 of
-// the product.  The tensor core rounds its running sum towards zero at each step of 16 along K, which over a long K would cost
+// The tensor cores have no float32 operands.  A float32 number is the exact sum of three bfloat16 numbers, each the one nearest to
+// what the ones before it leave (the exponent ranges are the same), and the product of two such numbers is exact in float32.  Of the
+// nine products of parts the six largest are taken; the second part is at most 2^-8 of the number and the third 2^-17, so the three others together
+// are at most 2^-24 of the product, of either sign.  (Parts cut off instead of rounded leave out up to 2^-21, always towards
+// zero.)  The tensor core rounds its running sum towards zero at each step of 16 along K, which over a long K would cost
 // more than plain float32 sums do.  So it sums 64 along K at a time, the small products first, and CUDA cores add these sums
 // up in registers, in order and rounded to nearest.  Error against 64 bits (2-norm over 2-norm, normal operands; in brackets the
 // fused multiply-adds in index order that gemm_f32.cu makes): K 256 1.3e-7 (2.9e-7), N 2,560 K 2,048 1.4e-7 (2.9e-7), N 22,016
@@ -15,7 +16,7 @@
 // multiply-adds in index order, so infinities and NaN come out as they do there.
 //
 // A block takes 128 rows of W, the tile's M rows of the MMA, and tile_n tokens, its N columns.  W arrives as float32 by TMA
-// (128-byte swizzle, K 64 a stage); a worker thread reads its part of a row's 64 values, cuts them up with bit masks and
+// (128-byte swizzle, K 64 a stage); a worker thread reads its part of a row's 64 values, cuts them up by conversions and
 // subtractions (exact) and writes the three parts into tensor memory, where the MMA takes its A operand from: the parts never go
 // back to shared memory, whose bandwidth the MMA's B operand (the tokens' three parts) needs.  Up to 64 tokens the same
 // threads cut the tokens' values up as well; for more, split_kernel has done it once for all blocks and TMA brings the parts.
@@ -64,15 +65,17 @@ __device__ __forceinline__ void u_arrive_warp(unsigned bar, int lane) {
   if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 
-// Two floats into their three bfloat16 parts each, packed (the first in the low half): x = hi + mid + lo exactly.
+// Two floats into their three bfloat16 parts each, packed (the first in the low half): x = hi + mid + lo exactly, each part what
+// the parts before it leave, rounded to nearest (hi to the largest finite one at most).  Below 2^-110 lo's last bits are below
+// bfloat16's least number.  Infinities and NaN leave a NaN in lo.
 __device__ __forceinline__ void cut(float x0, float x1, unsigned& hi, unsigned& mid, unsigned& lo) {
-  const unsigned a0 = __float_as_uint(x0), a1 = __float_as_uint(x1);
-  hi = __byte_perm(a0, a1, 0x7632);
-  const float r0 = x0 - __uint_as_float(a0 & 0xFFFF0000u), r1 = x1 - __uint_as_float(a1 & 0xFFFF0000u);
-  const unsigned b0 = __float_as_uint(r0), b1 = __float_as_uint(r1);
-  mid = __byte_perm(b0, b1, 0x7632);
-  const float s0 = r0 - __uint_as_float(b0 & 0xFFFF0000u), s1 = r1 - __uint_as_float(b1 & 0xFFFF0000u);
-  lo = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;\n" : "=r"(hi) : "f"(x1), "f"(x0));
+  x0 -= __uint_as_float(hi << 16);
+  x1 -= __uint_as_float(hi & 0xFFFF0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(mid) : "f"(x1), "f"(x0));
+  x0 -= __uint_as_float(mid << 16);
+  x1 -= __uint_as_float(mid & 0xFFFF0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(lo) : "f"(x1), "f"(x0));
 }
 
 __device__ __forceinline__ void u_tmem_st8(unsigned taddr, const unsigned (&r)[8]) {
