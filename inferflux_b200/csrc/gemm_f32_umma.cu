@@ -12,8 +12,10 @@
 //
 // How an output element is summed depends on N and K alone, as in gemm_f32.cu: K is cut into umma_slices(N, K) slices, a slice
 // into steps of 64, whatever M is and whichever tile width runs, so a row's result does not depend on what else is in
-// the batch.  A result that is not finite (an operand was not, or a sum overflowed on the way) is computed again by fused
-// multiply-adds in index order, so infinities and NaN come out as they do there.
+// the batch.  A slice's sum that is not finite (an operand was not, or a sum overflowed on the way), and one below 2^-64 that is not
+// zero (operands so small that bfloat16 does not reach to their last bits), is made again by fused multiply-adds in index order,
+// as gemm_f32.cu makes them.  So infinities and NaN come out as there, and for sums of 2^-64 and more what small operands lose,
+// 2^-134 of the other operand a product, is below float32's rounding unless that other operand is beyond 2^32.
 //
 // A block takes 128 rows of W, the tile's M rows of the MMA, and tile_n tokens, its N columns.  W arrives as float32 by TMA
 // (128-byte swizzle, K 64 a stage); a worker thread reads its part of a row's 64 values, cuts them up by conversions and
@@ -29,7 +31,6 @@
 // 9.0 (7.4), N 151,936 K 2,048 202 (208): a single row's blocks wait for one another's steps, and stay here for the sake of its bits.
 #include "gemm_f32_umma.h"
 #include "umma.cuh"
-#include <float.h>
 
 namespace {
 
@@ -97,6 +98,81 @@ __device__ __forceinline__ void u_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
 
+constexpr unsigned U_SMALL = 0x1F800000u;        // 2^-64
+// A sum that is to be made again: not finite, or below 2^-64 and not zero.
+__device__ __forceinline__ bool odd_sum(float v) {
+  const unsigned u = __float_as_uint(v) & 0x7FFFFFFFu;
+  return u >= 0x7F800000u || (u < U_SMALL && u != 0);
+}
+// Makes the odd ones among sums [TN][128] again over k_begin .. k_end, called by all workers: the tokens that have any 16 a part at a time, W
+// and the tokens through the shared memory behind the sums, the next 32 along K on their way meanwhile.  In a function of its own and
+// with the sums in memory it leaves the kernel's registers alone (inlined it cost up to 7 %).
+// (One NaN among 301 rows, N 22,016 K 2,048: 330 us where the product alone takes 147; in every row 1,760.  A thread a sum by itself took
+// 2,600 and 55,800.)
+template <int TN>
+__device__ __noinline__ void sums_again(float* sums, unsigned* odd_tokens, const float* __restrict__ A, const float* __restrict__ W, long long lda,
+                                        int M, int N, int K, int m0, int n0, int tile_n, int k_begin, int k_end) {
+  constexpr int PARTS = u_parts(TN), THREADS = 128 * PARTS, COLS = TN / PARTS, PITCH = 36;   // 36: 16-byte reads of eight rows meet no bank twice
+  constexpr int W_EACH = 128 * 8 / THREADS;
+  float *ws = sums + TN * 128, *xs = ws + 128 * PITCH;                 // [128][PITCH], [16 * PARTS][32]
+  const int tid = threadIdx.x, row = tid & 127, part = tid >> 7, kc = (tid & 7) * 4;
+  for (int i = 0; i < COLS; ++i) {
+    const int t = part * COLS + i;
+    if (odd_sum(sums[t * 128 + row]) && t < tile_n && m0 + t < M && n0 + row < N) atomicOr(&odd_tokens[t >> 5], 1u << (t & 31));
+  }
+  asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+#pragma unroll 1
+  for (int g = 0; g < COLS / 16; ++g) {
+    auto flags = [&](int p) { const int t = p * COLS + g * 16; return odd_tokens[t >> 5] >> (t & 31) & 0xFFFFu; };
+    if (!(flags(0) | flags(PARTS - 1))) continue;                      // (the same for all workers)
+    const unsigned mine = flags(part);
+    const int at = tid >> 3, xt = (at >> 4) * COLS + g * 16 + (at & 15);   // of the tokens' copies
+    float4 wv[W_EACH], xv;
+    auto load = [&](int k0) {
+      const int k = k0 + kc;                                           // K is a multiple of 4
+#pragma unroll
+      for (int i = 0; i < W_EACH; ++i) {
+        const int r = at + i * (THREADS / 8);
+        wv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n0 + r < N && k < k_end) wv[i] = *reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * K + k);
+      }
+      xv = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (xt < tile_n && m0 + xt < M && k < k_end) {
+        const float* p = A + (size_t)(m0 + xt) * lda + k;
+        xv = make_float4(p[0], p[1], p[2], p[3]);
+      }
+    };
+    float r[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = 0.0f;
+    load(k_begin);
+#pragma unroll 1
+    for (int k0 = k_begin; k0 < k_end; k0 += 32) {
+      asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+#pragma unroll
+      for (int i = 0; i < W_EACH; ++i) *reinterpret_cast<float4*>(ws + (at + i * (THREADS / 8)) * PITCH + kc) = wv[i];
+      *reinterpret_cast<float4*>(xs + at * 32 + kc) = xv;
+      asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+      load(k0 + 32);
+#pragma unroll 2
+      for (int c = 0; c < 32; c += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(ws + row * PITCH + c);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (mine >> i & 1) {
+            const float4 x = *reinterpret_cast<const float4*>(xs + (part * 16 + i) * 32 + c);
+            r[i] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, r[i]))));
+          }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float& v = sums[(part * COLS + g * 16 + i) * 128 + row];
+      if (mine >> i & 1 && odd_sum(v)) v = r[i];
+    }
+  }
+}
+
 // TN: token columns a block can hold.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W, slices of K), the slices of a tile a
 // cluster.  Up to TN 64 A is read here; above, map_x describes split_kernel's parts [3][M][K].
 template <int TN>
@@ -111,6 +187,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 6];   // w_full[s], w_empty[s], x_full[2], parts_full[2], mma_done[2]
   __shared__ unsigned tmem_slot;
   __shared__ int abort_s;
+  __shared__ unsigned odd_tokens[(TN + 31) / 32];                      // tokens with sums that are to be made again
   const unsigned sbase = (g_smem_addr(u_smem_raw) + 1023u) & ~1023u, sx = sbase + STAGES * W_STAGE;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (shuffled: known to be uniform)
   const unsigned w_full = g_smem_addr(&bars[0]), w_empty = g_smem_addr(&bars[STAGES]), x_full = g_smem_addr(&bars[2 * STAGES]);
@@ -118,6 +195,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   volatile int* abort_flag = &abort_s;
   if (tid == 0) {
     abort_s = 0;
+    for (int i = 0; i < (TN + 31) / 32; ++i) odd_tokens[i] = 0;
     for (int s = 0; s < STAGES; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(w_full + 8 * s));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(w_empty + 8 * s), "r"(WARPS));
@@ -291,16 +369,25 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     __nanosleep(2000000);
   }
   // Every MMA has been waited for, every copy has landed: the ring's memory can take the slices' sums.
+  // Whether there are sums to be made again, three instructions a sum: zero times it is not zero, or the least of the numbers that
+  // are not zero (zeros come out largest) is below 2^-64.
+  float zero = 0.0f;
+  unsigned least = 0xFFFFFFFFu;
+#pragma unroll
+  for (int i = 0; i < COLS; ++i) {
+    zero = fmaf(acc[i], 0.0f, zero);
+    least = min(least, 2u * __float_as_uint(acc[i]) - 1u);
+  }
+  if (__syncthreads_or(!(zero == 0.0f) || least < 2u * U_SMALL - 1u) && !*abort_flag && warp < WARPS) {
+    float* sums = reinterpret_cast<float*>(u_smem_raw + (sbase - g_smem_addr(u_smem_raw)));
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) sums[(part * COLS + i) * 128 + (tid & 127)] = acc[i];
+    sums_again<TN>(sums, odd_tokens, A, W, lda, M, N, K, m0, n0, tile_n, step0 * FK64, min(K, (step0 + steps) * FK64));
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) acc[i] = sums[(part * COLS + i) * 128 + (tid & 127)];
+  }
   const int slices = gridDim.z;
-  auto put = [&](int m, int n, float v) {
-    if (!(fabsf(v) <= FLT_MAX)) {
-      const float *a = A + (size_t)m * lda, *w = W + (size_t)n * K;
-      v = 0.0f;
-#pragma unroll 1
-      for (int k = 0; k < K; ++k) v = fmaf(a[k], w[k], v);
-    }
-    C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.0f);
-  };
+  auto put = [&](int m, int n, float v) { C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.0f); };
   if (slices == 1) {
     if (warp < WARPS) {
       const int n = n0 + quarter * 32 + lane;
