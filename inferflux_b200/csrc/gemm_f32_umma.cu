@@ -60,6 +60,13 @@ __device__ __forceinline__ float4 u_read_peer4(unsigned saddr, int rank) {
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
   return v;
 }
+// True for one lane of the warp, chosen in a way that the compiler knows to be one.  An MMA issued behind it takes the tensor core's time, 21
+// cycles with 16 columns, 39 with 64, 80 with 160; behind lane == 0 it takes at least 61 (measured with one block).
+__device__ __forceinline__ bool u_elect() {
+  unsigned r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+  return r != 0;
+}
 // one arrival for the warp, once all its lanes have come here
 __device__ __forceinline__ void u_arrive_warp(unsigned bar, int lane) {
   __syncwarp();
@@ -252,7 +259,7 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       }
     }
   } else if (warp == WARPS + 1) {                                             // the MMAs
-    if (lane == 0) {
+    if (u_elect()) {
       pdl_wait();
       const unsigned idesc = U_IDESC | ((unsigned)(tile_n >> 3) << 17);
       for (int c = 0; c < steps; ++c) {
@@ -262,15 +269,14 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         if (!OWN_X && !g_wait(x_full + 8 * b, par, abort_flag)) { gave_up = true; break; }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const unsigned d = tmem + 192 + b * TN, wp = tmem + b * 96;
-        // One thread issues an MMA in 46 cycles if it only adds to a descriptor, in 75 if it makes each anew; the MMA takes tile_n / 2.
-        const unsigned long long xd = g_desc(sx + b * 3 * TN * 128);
+        const unsigned long long xd0 = g_desc(sx + b * 3 * TN * 128), xd[3] = {xd0, xd0 + (unsigned)(tile_n * 8), xd0 + (unsigned)(tile_n * 16)};
         // (W's part, the tokens' part), 0 the highest: the small products first
         constexpr int order[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
         for (int p = 0; p < 6; ++p)
 #pragma unroll
           for (int k = 0; k < 4; ++k)                                  // (a descriptor's address counts 16 bytes)
-            u_mma(d, wp + order[p][0] * 32 + k * 8, xd + (unsigned)(order[p][1] * tile_n * 8 + k * 2), idesc, (p | k) != 0);
+            u_mma(d, wp + order[p][0] * 32 + k * 8, xd[order[p][1]] + k * 2, idesc, (p | k) != 0);
         u_commit(mma_done + 8 * b);
       }
     }
