@@ -7,28 +7,33 @@
 // zero.)  The tensor core rounds its running sum towards zero at each step of 16 along K, which over a long K would cost
 // more than plain float32 sums do.  So it sums 64 along K at a time, the small products first, and CUDA cores add these sums
 // up in registers, in order and rounded to nearest.  Error against 64 bits (2-norm over 2-norm, normal operands; in brackets the
-// fused multiply-adds in index order that gemm_f32.cu makes): K 256 1.3e-7 (2.9e-7), N 2,560 K 2,048 1.4e-7 (2.9e-7), N 22,016
-// K 2,048 1.6e-7 (8.1e-7), N 2,048 K 11,008 1.6e-7 (6.7e-7).
+// fused multiply-adds in index order that gemm_f32.cu makes): K 256 0.9e-7 (2.9e-7), N 2,560 K 2,048 1.0e-7 (2.9e-7), N 22,016
+// K 2,048 1.1e-7 (8.1e-7), N 2,048 K 11,008 1.3e-7 (6.7e-7), N 3,584 K 18,944 1.5e-7 (8.7e-7).
 //
 // How an output element is summed depends on N and K alone, as in gemm_f32.cu: K is cut into umma_slices(N, K) slices, a slice
-// into steps of 64, whatever M is and whichever tile width runs, so a row's result does not depend on what else is in
+// into steps of 64, and the slices' sums are added two by two, then the pairs in order, whatever M is, whichever tile width runs and
+// whether a block makes one slice or two, so a row's result does not depend on what else is in
 // the batch.  A slice's sum that is not finite (an operand was not, or a sum overflowed on the way), and one below 2^-64 that is not
-// zero (operands so small that bfloat16 does not reach to their last bits), is made again by fused multiply-adds in index order,
-// as gemm_f32.cu makes them.  So infinities and NaN come out as there, and for sums of 2^-64 and more what small operands lose,
-// 2^-134 of the other operand a product, is below float32's rounding unless that other operand is beyond 2^32.
+// zero (operands so small that bfloat16 does not reach to their last bits), is made again by fused multiply-adds in index
+// order.  So infinities and NaN are what these give (a sum that they would take beyond the range on the way and the tensor cores do
+// not stays as it is), and for sums of 2^-64 and more what small operands lose, 2^-134 of the other operand a product, is below
+// float32's rounding unless that other operand is beyond 2^32.
 //
 // A block takes 128 rows of W, the tile's M rows of the MMA, and tile_n tokens, its N columns.  W arrives as float32 by TMA
 // (128-byte swizzle, K 64 a stage); a worker thread reads its part of a row's 64 values, cuts them up by conversions and
 // subtractions (exact) and writes the three parts into tensor memory, where the MMA takes its A operand from: the parts never go
 // back to shared memory, whose bandwidth the MMA's B operand (the tokens' three parts) needs.  Up to 64 tokens the same
-// threads cut the tokens' values up as well; for more, split_kernel has done it once for all blocks and TMA brings the parts.
+// threads cut the tokens' values up as well (a warp of its own for them is ahead with one row and behind with eight); for more,
+// split_kernel has done it once for all blocks and TMA brings the parts.
 // Parts and sums are double-buffered: while the MMAs of one step run, the threads add the sums of the step before it and
 // cut up the values of the step behind it.
 //
-// What bounds it: six MMAs a product, so 2,250 / 6 = 375 TFLOP/s at most, and the thread that issues them (78 cycles each beside
-// the workers, while an MMA takes half a cycle a token); with few tokens reading W.  Us here (by multiply-adds), 301 rows: N 22,016
-// K 2,048 150 (623), N 2,048 K 11,008 103 (372), N 2,560 K 2,048 41 (93); 16 rows 48 (111), 32 (76), 10 (17); 1 row 44 (42), 32 (26),
-// 9.0 (7.4), N 151,936 K 2,048 202 (208): a single row's blocks wait for one another's steps, and stay here for the sake of its bits.
+// What bounds it: six MMAs a product, so 2,250 / 6 = 375 TFLOP/s at most; with few tokens the workers, of whose step (0.7 us alone on an
+// SM, 1.2 beside another block) the MMAs fill a quarter, and reading W.  Us here (by multiply-adds), 301 rows: N 22,016 K 2,048 142
+// (623), N 2,048 K 11,008 94 (373), N 2,560 K 2,048 40 (94); 64 rows 71 (251), 42 (182), 14 (50); 16 rows 41 (111), 28 (76), 8.6 (16.5); 8 rows 40
+// (72), 27 (50), 8.4 (11.5); 4 rows 39 (46), 27 (33), 7.7 (9.7); 2 rows 39 (46), 27 (32), 7.5 (9.5); 1 row 39 (39), 26.5 (27), 7.2 (7.2), N 151,936
+// K 2,048 205 (214).  Behind multiply-adds is one row of a square matrix of up to 2,048, whose blocks have few steps: 2,048 6.8 us (6.2), 1,024
+// 5.7 (4.5), 512 5.3 (4.1), 256 4.2 (3.2); it stays here for the sake of its bits, which are those of every batch.
 #include "gemm_f32_umma.h"
 #include "umma.cuh"
 
@@ -37,11 +42,9 @@ namespace {
 constexpr int FK64 = 64;                        // K per step
 constexpr int W_STAGE = 128 * FK64 * 4;         // 32 KB: two boxes of 128 rows x 32 floats
 constexpr int U_MAX_SLICES = 8;                  // of K: the largest portable cluster
-// Into how many parts K and the columns are dealt out to the workers, four warps each.  (With twice as many warps of workers 1 row x N 22,016
-// K 2,048 took 46 us instead of 43, 301 rows x N 2,048 K 11,008 105 instead of 103: they are in the issuing thread's way.)
-__host__ __device__ constexpr int u_parts(int tn) { return tn == 16 ? 1 : 2; }
+constexpr int U_PARTS = 2;                       // into so many K and the columns are dealt out to the workers, four warps each
 // the workers, and a warp each for W's copies, the MMAs and the tokens' copies
-__host__ __device__ constexpr int u_threads(int tn) { return 128 * u_parts(tn) + 96; }
+constexpr int U_THREADS = 128 * U_PARTS + 96;
 constexpr unsigned U_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // D float32, A and B bfloat16, K-major, M 128; N (in eighths) at bit 17
 
 __host__ __device__ constexpr int u_w_stages(int tn) { return tn == 16 ? 3 : tn <= 64 ? 5 : tn <= 128 ? 4 : 3; }
@@ -73,16 +76,19 @@ __device__ __forceinline__ void u_arrive_warp(unsigned bar, int lane) {
   if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 
+// Takes two packed parts off two floats.
+__device__ __forceinline__ void take_off(float& x0, float& x1, unsigned part) {
+  asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n sub.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}\n"
+      : "+f"(x0), "+f"(x1) : "r"(part << 16), "r"(part & 0xFFFF0000u));
+}
 // Two floats into their three bfloat16 parts each, packed (the first in the low half): x = hi + mid + lo exactly, each part what
 // the parts before it leave, rounded to nearest (hi to the largest finite one at most).  Below 2^-110 lo's last bits are below
 // bfloat16's least number.  Infinities and NaN leave a NaN in lo.
 __device__ __forceinline__ void cut(float x0, float x1, unsigned& hi, unsigned& mid, unsigned& lo) {
   asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;\n" : "=r"(hi) : "f"(x1), "f"(x0));
-  x0 -= __uint_as_float(hi << 16);
-  x1 -= __uint_as_float(hi & 0xFFFF0000u);
+  take_off(x0, x1, hi);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(mid) : "f"(x1), "f"(x0));
-  x0 -= __uint_as_float(mid << 16);
-  x1 -= __uint_as_float(mid & 0xFFFF0000u);
+  take_off(x0, x1, mid);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(lo) : "f"(x1), "f"(x0));
 }
 
@@ -111,84 +117,89 @@ __device__ __forceinline__ bool odd_sum(float v) {
   const unsigned u = __float_as_uint(v) & 0x7FFFFFFFu;
   return u >= 0x7F800000u || (u < U_SMALL && u != 0);
 }
-// Makes the odd ones among sums [TN][128] again over k_begin .. k_end, called by all workers: the tokens that have any 16 a part at a time, W
+// Makes the odd ones among sums [BOTH][TN][128] again, of slices slice_len long from k_begin on, called by all workers: the tokens that have any 16 a part at a time, W
 // and the tokens through the shared memory behind the sums, the next 32 along K on their way meanwhile.  In a function of its own and
 // with the sums in memory it leaves the kernel's registers alone (inlined it cost up to 7 %).
-// (One NaN among 301 rows, N 22,016 K 2,048: 330 us where the product alone takes 147; in every row 1,760.  A thread a sum by itself took
-// 2,600 and 55,800.)
-template <int TN>
+// (One NaN among 301 rows, N 22,016 K 2,048: 325 us where the product alone takes 142; in every row 1,750; 1 row 170 and 39.  A
+// thread a sum by itself took 2,600, 55,800 and 1,780.)
+template <int TN, int BOTH>
 __device__ __noinline__ void sums_again(float* sums, unsigned* odd_tokens, const float* __restrict__ A, const float* __restrict__ W, long long lda,
-                                        int M, int N, int K, int m0, int n0, int tile_n, int k_begin, int k_end) {
-  constexpr int PARTS = u_parts(TN), THREADS = 128 * PARTS, COLS = TN / PARTS, PITCH = 36;   // 36: 16-byte reads of eight rows meet no bank twice
-  constexpr int W_EACH = 128 * 8 / THREADS;
-  float *ws = sums + TN * 128, *xs = ws + 128 * PITCH;                 // [128][PITCH], [16 * PARTS][32]
+                                        int M, int N, int K, int m0, int n0, int tile_n, int k_begin, int slice_len, int k_last) {
+  constexpr int PARTS = U_PARTS, THREADS = 128 * PARTS, COLS = TN / PARTS, PITCH = 36;   // 36: 16-byte reads of eight rows meet no bank twice
+  constexpr int W_EACH = 128 * 8 / THREADS, G = COLS < 16 ? COLS : 16;
+  float *ws = sums + BOTH * TN * 128, *xs = ws + 128 * PITCH;          // [128][PITCH], [16 * PARTS][32]
   const int tid = threadIdx.x, row = tid & 127, part = tid >> 7, kc = (tid & 7) * 4;
-  for (int i = 0; i < COLS; ++i) {
-    const int t = part * COLS + i;
-    if (odd_sum(sums[t * 128 + row]) && t < tile_n && m0 + t < M && n0 + row < N) atomicOr(&odd_tokens[t >> 5], 1u << (t & 31));
-  }
-  asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
 #pragma unroll 1
-  for (int g = 0; g < COLS / 16; ++g) {
-    auto flags = [&](int p) { const int t = p * COLS + g * 16; return odd_tokens[t >> 5] >> (t & 31) & 0xFFFFu; };
-    if (!(flags(0) | flags(PARTS - 1))) continue;                      // (the same for all workers)
-    const unsigned mine = flags(part);
-    const int at = tid >> 3, xt = (at >> 4) * COLS + g * 16 + (at & 15);   // of the tokens' copies
-    float4 wv[W_EACH], xv;
-    auto load = [&](int k0) {
-      const int k = k0 + kc;                                           // K is a multiple of 4
-#pragma unroll
-      for (int i = 0; i < W_EACH; ++i) {
-        const int r = at + i * (THREADS / 8);
-        wv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n0 + r < N && k < k_end) wv[i] = *reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * K + k);
-      }
-      xv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (xt < tile_n && m0 + xt < M && k < k_end) {
-        const float* p = A + (size_t)(m0 + xt) * lda + k;
-        xv = make_float4(p[0], p[1], p[2], p[3]);
-      }
-    };
-    float r[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = 0.0f;
-    load(k_begin);
+  for (int h = 0; h < BOTH; ++h, sums += TN * 128) {
+    const int k_first = min(k_last, k_begin + h * slice_len), k_end = min(k_last, k_first + slice_len);
+    for (int i = 0; i < COLS; ++i) {
+      const int t = part * COLS + i;
+      if (odd_sum(sums[t * 128 + row]) && t < tile_n && m0 + t < M && n0 + row < N) atomicOr(&odd_tokens[t >> 5], 1u << (t & 31));
+    }
+    asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
 #pragma unroll 1
-    for (int k0 = k_begin; k0 < k_end; k0 += 32) {
-      asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+    for (int g = 0; g < (COLS + 15) / 16; ++g) {
+      auto flags = [&](int p) { const int t = p * COLS + g * G; return odd_tokens[t >> 5] >> (t & 31) & ((1u << G) - 1); };
+      if (!(flags(0) | flags(PARTS - 1))) continue;                      // (the same for all workers)
+      const unsigned mine = flags(part);
+      const int at = tid >> 3, xt = (at / G) * COLS + g * G + (at % G);   // of the tokens' copies
+      float4 wv[W_EACH], xv;
+      auto load = [&](int k0) {
+        const int k = k0 + kc;                                           // K is a multiple of 4
 #pragma unroll
-      for (int i = 0; i < W_EACH; ++i) *reinterpret_cast<float4*>(ws + (at + i * (THREADS / 8)) * PITCH + kc) = wv[i];
-      *reinterpret_cast<float4*>(xs + at * 32 + kc) = xv;
-      asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
-      load(k0 + 32);
+        for (int i = 0; i < W_EACH; ++i) {
+          const int r = at + i * (THREADS / 8);
+          wv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (n0 + r < N && k < k_end) wv[i] = *reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * K + k);
+        }
+        xv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (at < G * PARTS && xt < tile_n && m0 + xt < M && k < k_end) {
+          const float* p = A + (size_t)(m0 + xt) * lda + k;
+          xv = make_float4(p[0], p[1], p[2], p[3]);
+        }
+      };
+      float r[G];
+#pragma unroll
+      for (int i = 0; i < G; ++i) r[i] = 0.0f;
+      load(k_first);
+#pragma unroll 1
+      for (int k0 = k_first; k0 < k_end; k0 += 32) {
+        asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+#pragma unroll
+        for (int i = 0; i < W_EACH; ++i) *reinterpret_cast<float4*>(ws + (at + i * (THREADS / 8)) * PITCH + kc) = wv[i];
+        *reinterpret_cast<float4*>(xs + at * 32 + kc) = xv;
+        asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+        load(k0 + 32);
 #pragma unroll 2
-      for (int c = 0; c < 32; c += 4) {
-        const float4 w = *reinterpret_cast<const float4*>(ws + row * PITCH + c);
+        for (int c = 0; c < 32; c += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(ws + row * PITCH + c);
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (mine >> i & 1) {
-            const float4 x = *reinterpret_cast<const float4*>(xs + (part * 16 + i) * 32 + c);
-            r[i] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, r[i]))));
-          }
+          for (int i = 0; i < G; ++i)
+            if (mine >> i & 1) {
+              const float4 x = *reinterpret_cast<const float4*>(xs + (part * G + i) * 32 + c);
+              r[i] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, r[i]))));
+            }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        float& v = sums[(part * COLS + g * G + i) * 128 + row];
+        if (mine >> i & 1 && odd_sum(v)) v = r[i];
       }
     }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float& v = sums[(part * COLS + g * 16 + i) * 128 + row];
-      if (mine >> i & 1 && odd_sum(v)) v = r[i];
-    }
+    asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");      // all have read the flags before the next slice sets some
   }
 }
 
-// TN: token columns a block can hold.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W, slices of K), the slices of a tile a
-// cluster.  Up to TN 64 A is read here; above, map_x describes split_kernel's parts [3][M][K].
-template <int TN>
-__global__ void __launch_bounds__(u_threads(TN), TN == 16 ? 2 : 1)
+// TN: token columns a block can hold.  BOTH: slices of K that it makes.  Grid: (tiles of tile_n tokens, tiles of 128 rows of W,
+// slices of K / BOTH), the blocks of a tile a cluster.  Up to TN 64 A is read here; above, map_x describes split_kernel's parts [3][M][K].
+template <int TN, int BOTH>
+__global__ void __launch_bounds__(U_THREADS, TN == 16 ? 2 : 1)
 gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ A,
                      const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K, long long lda,
                      long long ldc, int tile_n, int slice_steps, int vec_a, int w_fixed, int* __restrict__ error_flag) {
   constexpr bool OWN_X = TN <= 64;
-  constexpr int STAGES = u_w_stages(TN), PARTS = u_parts(TN), WARPS = 4 * PARTS, COLS = TN / PARTS, UNITS = 16 / PARTS;   // a worker's columns, and float4 of W
+  constexpr int STAGES = u_w_stages(TN), PARTS = U_PARTS, WARPS = 4 * PARTS, COLS = TN / PARTS, UNITS = 16 / PARTS;   // a worker's columns, and float4 of W
   constexpr int X_ROWS = 2 * WARPS, X_PER = OWN_X && TN > X_ROWS ? TN / X_ROWS : 1;                                          // and float4 of the tokens
   extern __shared__ unsigned char u_smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 6];   // w_full[s], w_empty[s], x_full[2], parts_full[2], mma_done[2]
@@ -200,7 +211,18 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   const unsigned w_full = g_smem_addr(&bars[0]), w_empty = g_smem_addr(&bars[STAGES]), x_full = g_smem_addr(&bars[2 * STAGES]);
   const unsigned parts_full = x_full + 16, mma_done = x_full + 32;
   volatile int* abort_flag = &abort_s;
-  if (tid == 0) {
+  const int m0 = blockIdx.x * tile_n, n0 = blockIdx.y * 128;
+  const int steps_all = (K + FK64 - 1) / FK64, step0 = min(steps_all, (int)blockIdx.z * BOTH * slice_steps);
+  const int steps = min(steps_all, step0 + BOTH * slice_steps) - step0;
+  auto copy_w = [&](int c) {
+    const int st = c % STAGES;
+    g_expect_tx(w_full + 8 * st, W_STAGE);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+                   ::"r"(sbase + st * W_STAGE + h * (W_STAGE / 2)), "l"(&map_w), "r"((step0 + c) * FK64 + 32 * h), "r"(n0), "r"(w_full + 8 * st) : "memory");
+  };
+  if (tid == 32 * WARPS) {
     abort_s = 0;
     for (int i = 0; i < (TN + 31) / 32; ++i) odd_tokens[i] = 0;
     for (int s = 0; s < STAGES; ++s) {
@@ -214,6 +236,8 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    if (w_fixed)                                                       // the first tiles of W come while the others set up
+      for (int c = 0; c < min(steps, STAGES); ++c) copy_w(c);
   }
   if (warp == WARPS + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(g_smem_addr(&tmem_slot)), "n"(u_columns(TN)) : "memory");
@@ -224,27 +248,23 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   pdl_launch_dependents();                       // behind the allocation: no block of the next kernel can be ahead of it at the tensor memory
   const unsigned tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  const int m0 = blockIdx.x * tile_n, n0 = blockIdx.y * 128;
-  const int steps_all = (K + FK64 - 1) / FK64, step0 = min(steps_all, (int)blockIdx.z * slice_steps);
-  const int steps = min(steps_all, step0 + slice_steps) - step0;
   bool gave_up = false;
-  float acc[COLS];
+  float acc[COLS], first[BOTH == 2 ? COLS : 1];                        // first: of two slices
 #pragma unroll
   for (int i = 0; i < COLS; ++i) acc[i] = 0.0f;
+  if constexpr (BOTH == 2) {
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) first[i] = 0.0f;
+  }
   const int quarter = warp & 3, part = warp >> 2;                      // of a worker: its lanes of tensor memory, its part of K and of the columns
 
   if (warp == WARPS) {                                                    // W's copies
     if (lane == 0) {
       if (!w_fixed) pdl_wait();
-      for (int c = 0; c < steps; ++c) {
-        const int st = c % STAGES;
+      for (int c = w_fixed ? STAGES : 0; c < steps; ++c) {
         if (c == STAGES) pdl_wait();                                   // (bounded waits begin when the kernel ahead has finished)
-        if (c >= STAGES && !g_wait(w_empty + 8 * st, (unsigned)((c / STAGES - 1) & 1), abort_flag)) { gave_up = true; break; }
-        g_expect_tx(w_full + 8 * st, W_STAGE);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-                       ::"r"(sbase + st * W_STAGE + h * (W_STAGE / 2)), "l"(&map_w), "r"((step0 + c) * FK64 + 32 * h), "r"(n0), "r"(w_full + 8 * st) : "memory");
+        if (c >= STAGES && !g_wait(w_empty + 8 * (c % STAGES), (unsigned)((c / STAGES - 1) & 1), abort_flag)) { gave_up = true; break; }
+        copy_w(c);
       }
     }
   } else if (warp == WARPS + 2) {                                             // the tokens' copies
@@ -304,6 +324,11 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
           for (int j = 0; j < 8; ++j) acc[i * 8 + j] += __uint_as_float(r[j]);
         }
       }
+      if constexpr (BOTH == 2)
+        if (c == slice_steps - 1) {
+#pragma unroll
+          for (int i = 0; i < COLS; ++i) { first[i] = acc[i]; acc[i] = 0.0f; }
+        }
       return true;
     };
     float4 xr[X_PER];                                                  // the tokens' values of the step ahead: 16 threads a row, four values each
@@ -383,14 +408,31 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   for (int i = 0; i < COLS; ++i) {
     zero = fmaf(acc[i], 0.0f, zero);
     least = min(least, 2u * __float_as_uint(acc[i]) - 1u);
+    if constexpr (BOTH == 2) {
+      zero = fmaf(first[i], 0.0f, zero);
+      least = min(least, 2u * __float_as_uint(first[i]) - 1u);
+    }
   }
   if (__syncthreads_or(!(zero == 0.0f) || least < 2u * U_SMALL - 1u) && !*abort_flag && warp < WARPS) {
     float* sums = reinterpret_cast<float*>(u_smem_raw + (sbase - g_smem_addr(u_smem_raw)));
+    float* own = sums + part * COLS * 128 + (tid & 127);
+    // (where K ends in the first of two slices its sums are in acc)
+    const int at = BOTH == 2 && steps >= slice_steps ? TN * 128 : 0;
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) sums[(part * COLS + i) * 128 + (tid & 127)] = acc[i];
-    sums_again<TN>(sums, odd_tokens, A, W, lda, M, N, K, m0, n0, tile_n, step0 * FK64, min(K, (step0 + steps) * FK64));
+    for (int i = 0; i < COLS; ++i) {
+      if constexpr (BOTH == 2) own[TN * 128 - at + i * 128] = first[i];
+      own[at + i * 128] = acc[i];
+    }
+    sums_again<TN, BOTH>(sums, odd_tokens, A, W, lda, M, N, K, m0, n0, tile_n, step0 * FK64, slice_steps * FK64, min(K, (step0 + steps) * FK64));
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) acc[i] = sums[(part * COLS + i) * 128 + (tid & 127)];
+    for (int i = 0; i < COLS; ++i) {
+      if constexpr (BOTH == 2) first[i] = own[TN * 128 - at + i * 128];
+      acc[i] = own[at + i * 128];
+    }
+  }
+  if constexpr (BOTH == 2) {
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) acc[i] += first[i];
   }
   const int slices = gridDim.z;
   auto put = [&](int m, int n, float v) { C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.0f); };
@@ -422,10 +464,18 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
         for (int z = 0; z < U_MAX_SLICES; ++z)
           if (z < slices) v[z] = u_read_peer4(sbase + (t * 128 + 4 * lane) * 4, z);
-        float4 o = v[0];
+        auto add = [](float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+        float4 o = v[0];                                               // two by two, then the pairs in order
+        if constexpr (BOTH == 2) {
 #pragma unroll
-        for (int z = 1; z < U_MAX_SLICES; ++z)
-          if (z < slices) { o.x += v[z].x; o.y += v[z].y; o.z += v[z].z; o.w += v[z].w; }
+          for (int z = 1; z < U_MAX_SLICES; ++z)
+            if (z < slices) add(o, v[z]);
+        } else {
+          add(o, v[1]);
+#pragma unroll
+          for (int z = 2; z < U_MAX_SLICES; z += 2)
+            if (z < slices) { add(v[z], v[z + 1]); add(o, v[z]); }
+        }
         if (n < N) put(m0 + t, n, o.x);
         if (n + 1 < N) put(m0 + t, n + 1, o.y);
         if (n + 2 < N) put(m0 + t, n + 2, o.z);
@@ -463,8 +513,9 @@ split_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, int 
   for (int q = 0; q < 3; ++q) parts[(long long)q * M * groups + i] = o[q];
 }
 
-// Slices of K, from N and K alone (1, 2, 4 or 8), each at least 256 long: blocks enough that their last round is a small part of
-// all (N 22,016 K 2,048 in two slices instead of one: 160 rows 99 -> 88 us, 77 rows 80 -> 71, 1 row 44 in both).
+// Slices of K, from N and K alone (1, 2, 4 or 8), each at least 256 long: blocks enough that their last round is a small part of all.
+// (Shorter ones would be ahead for one row of a small matrix, 1,024 x 1,024 in 8 instead of 4 4.3 us instead of 5.6, and behind for
+// many, 2,048 rows 74 instead of 50.)
 int umma_slices(int N, int K) {
   const int rows = (N + 127) / 128;
   int s = 1;
@@ -472,19 +523,29 @@ int umma_slices(int N, int K) {
   return s;
 }
 
-struct TokenTiles { int tn, count; };
-// Tiles of tokens: as few rounds of blocks over the SMs as the widths allow.  A step's cycles go by its 24 MMAs: 97 each with
-// 160 tokens, 76 with up to 120 (issuing one beside the workers takes that long); a block has some 6,000 of its own.
+constexpr int U_TWO_TOKENS = 96;                 // tokens up to which a block can take two slices: it needs registers for two sums of each
+struct TokenTiles { int tn, count, both; };
+// Tiles of tokens, and one slice or two a block, by the time that rounds of blocks over the SMs take.  Clusters of 4 and 8 blocks fit
+// 132 and 120 of 148 SMs only (cudaOccupancyMaxActiveClusters), so two slices a block can save a round: us with two (with one), 1 row
+// N 22,016 K 2,048 38.5 (44), 4,608 x 3,584 19.2 (20.3); 32 rows 2,048 x 2,048 10.6 (15.6); 700 rows 60 (72).  ns, all measured: a step takes 700 with
+// 16 tokens (1,190 with two blocks an SM), 830, 1,000 and 1,090 with 32, 48 and 64, which the workers cut up as well, 800 with 80
+// to 1,110 with 160; a block has 2,000 and 19 a token of its own; two slices with
+// 96 tokens, whose registers spill, a twentieth more; split_kernel takes 2,500.  Over 16 shapes and numbers of rows from
+// 100 to 2,048 the tiles chosen are within 8 % of the best ones, but for 100 rows x 2,048 K 320 (7.2 us, 6.4 with tiles of 32).
 TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
-  TokenTiles best{16, 1};
+  TokenTiles best{16, 1, 1};
   long long best_cost = -1;
-  const long long blocks = (long long)((N + 127) / 128) * slices;
   for (int count = (M + 159) / 160; count <= (M + 15) / 16; ++count) {
     const int tn = ((M + count - 1) / count + 15) / 16 * 16;
-    const long long per_sm = tn <= 16 ? 2 : 1, rounds = (blocks * count + sms * per_sm - 1) / (sms * per_sm);
-    const int mma = 24 * (tn * 3 / 5 > 76 ? tn * 3 / 5 : 76);
-    const long long cost = rounds * ((long long)steps * mma + 6000);
-    if (best_cost < 0 || cost < best_cost) { best = TokenTiles{tn, count}; best_cost = cost; }
+    for (int both = 1; both <= (slices > 1 && tn <= U_TWO_TOKENS ? 2 : 1); ++both) {
+      const int cl = slices / both, fit = sms * (cl == 8 ? 120 : cl == 4 ? 132 : 148) / 148 / cl;   // clusters, at one block an SM
+      const long long clusters = (long long)((N + 127) / 128) * count;
+      const bool pairs = tn == 16 && clusters > fit;
+      const long long rounds = (clusters + fit * (pairs ? 2 : 1) - 1) / (fit * (pairs ? 2 : 1));
+      const int step = tn == 16 ? (pairs ? 1190 : 700) : tn <= 32 ? 830 : tn <= 48 ? 1000 : tn <= 64 ? 1090 : tn <= 96 ? 560 + 3 * tn : 310 + 5 * tn;
+      const long long cost = rounds * ((long long)both * steps * step + 2000 + 19 * tn) * (both == 2 && tn > 64 ? 21 : 20) / 20 + (tn > 64 ? 2500 : 0);
+      if (best_cost < 0 || cost < best_cost) { best = TokenTiles{tn, count, both}; best_cost = cost; }
+    }
   }
   return best;
 }
@@ -496,10 +557,10 @@ int u_sm_count(int* sms) {
   return (int)e;
 }
 
-template <int TN>
+template <int TN, int BOTH>
 int launch_umma_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
                     int tn, int count, int slices, int steps, bool vec_a, void* scratch, int w_fixed, int* error_flag, cudaStream_t stream) {
-  auto kern = gemm_f32_umma_kernel<TN>;
+  auto kern = gemm_f32_umma_kernel<TN, BOTH>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, u_smem(TN));
   if (e != cudaSuccess) return (int)e;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
@@ -525,7 +586,7 @@ int launch_umma_f32(const float* A, const float* W, const float* bias, float* C,
     int rc = launch_pdl(split_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, A, (uint4*)scratch, M, K, lda, pitch, (int)vec_a);
     if (rc) return rc;
   }
-  const int rc = launch_pdl_cluster(kern, dim3(count, (N + 127) / 128, slices), dim3(u_threads(TN)), (size_t)u_smem(TN), stream, dim3(1, 1, slices),
+  const int rc = launch_pdl_cluster(kern, dim3(count, (N + 127) / 128, slices / BOTH), dim3(U_THREADS), (size_t)u_smem(TN), stream, dim3(1, 1, slices / BOTH),
                                     map_w, map_x, A, W, bias, C, M, N, K, lda, ldc, tn, steps, (int)vec_a, w_fixed, error_flag);
   return rc ? rc : IFX_LAUNCH_CHECK();
 }
@@ -543,7 +604,9 @@ int gemm_f32_umma(const float* A, const float* W, const float* bias, float* C, i
   const int slices = umma_slices(N, K), steps_all = (K + FK64 - 1) / FK64, steps = (steps_all + slices - 1) / slices;
   const TokenTiles t = token_tiles(M, N, slices, steps, sms);
   const bool vec_a = lda % 4 == 0 && !((uintptr_t)A & 15);
-#define IFX_TILE(TN) launch_umma_f32<TN>(A, W, bias, C, M, N, K, lda, ldc, t.tn, t.count, slices, steps, vec_a, scratch, w_fixed, error_flag, stream)
-  return t.tn <= 16 ? IFX_TILE(16) : t.tn <= 32 ? IFX_TILE(32) : t.tn <= 64 ? IFX_TILE(64) : t.tn <= 96 ? IFX_TILE(96) : t.tn <= 128 ? IFX_TILE(128) : IFX_TILE(160);
+#define IFX_TILE(TN, BOTH) launch_umma_f32<TN, BOTH>(A, W, bias, C, M, N, K, lda, ldc, t.tn, t.count, slices, steps, vec_a, scratch, w_fixed, error_flag, stream)
+  if (t.both == 2) return t.tn <= 16 ? IFX_TILE(16, 2) : t.tn <= 32 ? IFX_TILE(32, 2) : t.tn <= 64 ? IFX_TILE(64, 2) : IFX_TILE(96, 2);
+  return t.tn <= 16 ? IFX_TILE(16, 1) : t.tn <= 32 ? IFX_TILE(32, 1) : t.tn <= 64 ? IFX_TILE(64, 1)
+         : t.tn <= 96 ? IFX_TILE(96, 1) : t.tn <= 128 ? IFX_TILE(128, 1) : IFX_TILE(160, 1);
 #undef IFX_TILE
 }
