@@ -359,8 +359,11 @@ int many(bool vec, bool narrow, const float* A, const float* W, const float* bia
 
 // A rows lda, C rows ldc elements apart, W contiguous, any K and alignment.  w_fixed: 1 = W is a parameter, which may be read
 // before the kernel has waited for those ahead of it (see common.cuh on what that takes; here up to 16 rows, and the tensor
-// cores, use it).  scratch: 6 M ceil8(K) bytes, 16-byte aligned, used for more than 64 rows; may be null with fewer.
+// cores, use it).  scratch: as many bytes as ifx_gemm_f32_scratch says for the same W, M, N and K, 16-byte aligned; null where that is 0.
 // error_flag: a device word set if a bounded wait inside the kernel runs out.
+IFX_API long long ifx_gemm_f32_scratch(const float* W, int M, int N, int K) {
+  return M > 0 && K > 0 && gemm_f32_umma_takes(W, N, K) ? gemm_f32_umma_scratch(M, K) : 0;
+}
 IFX_API int ifx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                          long long lda, long long ldc, void* scratch, int w_fixed, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;

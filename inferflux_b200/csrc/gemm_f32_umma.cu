@@ -594,6 +594,19 @@ int launch_umma_f32(const float* A, const float* W, const float* bias, float* C,
 
 bool gemm_f32_umma_takes(const float* W, int N, int K) { return K % 4 == 0 && !((uintptr_t)W & 15) && N >= 256 && K >= 256; }
 
+// More rows than this go piece by piece, so that their parts take 64 MB at most (but for K beyond 69,000, where 160 rows take more).  They
+// then stay in the L2 besides: 8,192 rows x N 3,584 K 18,944 in pieces of 32 / 64 / 128 / 256 MB 5.56 / 5.44 / 5.75 / 5.83 ms, whole 5.81; N 2,048 K 11,008
+// 2.34 / 2.17 / 2.18 / 2.23, 2.23; 2,048 rows of these 1.39 / 1.36 / 1.43 / 1.45, 1.45 and 0.60 / 0.56 / 0.56 / 0.55, 0.55.
+constexpr long long U_SCRATCH = 64ll << 20;
+static int piece_rows(int K) {
+  const long long rows = U_SCRATCH / (6ll * ((K + 7) / 8 * 8)) / 160 * 160;
+  return rows < 160 ? 160 : rows > (1 << 30) ? 1 << 30 : (int)rows;
+}
+long long gemm_f32_umma_scratch(int M, int K) {
+  const int rows = M < piece_rows(K) ? M : piece_rows(K);
+  return M > 64 ? 6ll * rows * ((K + 7) / 8 * 8) : 0;
+}
+
 int gemm_f32_umma(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, long long lda, long long ldc,
                   void* scratch, int w_fixed, int* error_flag, cudaStream_t stream) {
   if (!error_flag) return IFX_ERR_UNSUPPORTED;
@@ -601,6 +614,14 @@ int gemm_f32_umma(const float* A, const float* W, const float* bias, float* C, i
   int sms = 0;
   const int rc = u_sm_count(&sms);
   if (rc) return rc;
+  const int most = piece_rows(K);
+  if (M > most) {                                                      // (the parts of a piece are made when the piece before it is done)
+    for (int m = 0; m < M; m += most) {
+      const int r = gemm_f32_umma(A + m * lda, W, bias, C + m * ldc, M - m < most ? M - m : most, N, K, lda, ldc, scratch, w_fixed, error_flag, stream);
+      if (r) return r;
+    }
+    return 0;
+  }
   const int slices = umma_slices(N, K), steps_all = (K + FK64 - 1) / FK64, steps = (steps_all + slices - 1) / slices;
   const TokenTiles t = token_tiles(M, N, slices, steps, sms);
   const bool vec_a = lda % 4 == 0 && !((uintptr_t)A & 15);

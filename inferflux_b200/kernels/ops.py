@@ -52,6 +52,8 @@ def _load():
                                               c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                               c_int, c_void_p]
         lib.ifx_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_void_p, c_int, c_void_p, c_void_p]
+        lib.ifx_gemm_f32_scratch.argtypes = [c_void_p, c_int, c_int, c_int]
+        lib.ifx_gemm_f32_scratch.restype = c_ll
         lib.ifx_attn_paged_generic.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_int,
                                                c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p]
@@ -428,10 +430,17 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     _need(a.stride(1) == 1 and out.stride(1) == 1, "gemm_f32: unit inner strides")
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm_f32: bias float32 [N]")
-    scratch = torch.empty((6 * m * ((k + 7) // 8 * 8),), dtype=torch.uint8, device=a.device) if m > 64 and k % 4 == 0 else None
+    size = gemm_f32_scratch(_ptr(w), m, n, k) if m > 64 else 0
+    scratch = torch.empty(size, dtype=torch.uint8, device=a.device) if size else None
     _check(_lib().ifx_gemm_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0) if m > 1 else k,
                                out.stride(0) if m > 1 else n, _ptr(scratch), w_fixed, error_flag(a.device).data_ptr(), _stream()), "gemm_f32")
     return out
+
+
+def gemm_f32_scratch(w_address: int, m: int, n: int, k: int) -> int:
+    """Bytes of scratch that :func:`gemm_f32` takes from the allocator for a call: the parts of ``a``'s rows, 64 MB at most; none for
+    up to 64 rows and for matrices that go to the FFMA kernels."""
+    return int(_lib().ifx_gemm_f32_scratch(w_address, m, n, k))
 
 
 GEMV_MAX_ROWS = 16

@@ -96,3 +96,13 @@ def test_which_kernel_takes_the_portions(ops, entries, heads, window, tcgen05):
     longest = max(n + c for n, c in entries)
     _, us, mma_us = _plan(ops, entries, heads, 128 if 2 * blocks <= SMS else 256, window, 8, min(longest, abs(window) + 256) if window else longest)
     assert (us < mma_us) == tcgen05
+
+
+@pytest.mark.parametrize("m,n,k,address,size", [
+    (64, 2048, 2048, 256, 0), (65, 2048, 2048, 256, 6 * 65 * 2048), (301, 22016, 2052, 256, 6 * 301 * 2056),
+    (4096, 255, 2048, 256, 0), (4096, 2048, 252, 256, 0), (4096, 2048, 2050, 256, 0), (4096, 2048, 2048, 260, 0),    # to the FFMA kernels
+    (16384, 3584, 18944, 256, None), (100000, 256, 256, 256, None), (1 << 20, 151936, 4096, 256, None)])
+def test_scratch_of_float32_products(ops, m, n, k, address, size):
+    """None where none is used, six bytes a number of the rows, and never more than 64 MB."""
+    got = ops.gemm_f32_scratch(address, m, n, k)
+    assert got == size if size is not None else 32 << 20 < got <= 64 << 20
