@@ -535,8 +535,8 @@ struct TokenTiles { int tn, count, both; };
 TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
   TokenTiles best{16, 1, 1};
   long long best_cost = -1;
-  for (int count = (M + 159) / 160; count <= (M + 15) / 16; ++count) {
-    const int tn = ((M + count - 1) / count + 15) / 16 * 16;
+  for (int widest = 160; widest >= 16; widest -= 16) {                 // (of each width the fewest tiles)
+    const int count = (M + widest - 1) / widest, tn = ((M + count - 1) / count + 15) / 16 * 16;
     for (int both = 1; both <= (slices > 1 && tn <= U_TWO_TOKENS ? 2 : 1); ++both) {
       const int cl = slices / both, fit = sms * (cl == 8 ? 120 : cl == 4 ? 132 : 148) / 148 / cl;   // clusters, at one block an SM
       const long long clusters = (long long)((N + 127) / 128) * count;
