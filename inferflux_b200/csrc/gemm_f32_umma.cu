@@ -96,9 +96,6 @@ __device__ __forceinline__ void u_tmem_st8(unsigned taddr, const unsigned (&r)[8
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-__device__ __forceinline__ void u_tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
-}
 __device__ __forceinline__ void u_tmem_ld8(unsigned taddr, unsigned (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
@@ -138,7 +135,7 @@ __device__ __noinline__ void sums_again(float* sums, unsigned* odd_tokens, const
     }
     asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
 #pragma unroll 1
-    for (int g = 0; g < (COLS + 15) / 16; ++g) {
+    for (int g = 0; g < COLS / G; ++g) {
       auto flags = [&](int p) { const int t = p * COLS + g * G; return odd_tokens[t >> 5] >> (t & 31) & ((1u << G) - 1); };
       if (!(flags(0) | flags(PARTS - 1))) continue;                      // (the same for all workers)
       const unsigned mine = flags(part);
@@ -307,22 +304,14 @@ gemm_f32_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       if (!__all_sync(0xffffffffu, g_wait(mma_done + 8 * (c & 1), (unsigned)((c >> 1) & 1), abort_flag))) return false;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
-      for (int i = 0; i < (COLS + 7) / 8; ++i) {
+      for (int i = 0; i < COLS / 8; ++i) {
         if (part * COLS + i * 8 >= tile_n) break;                      // (the same for the warp)
         const unsigned at = lanes + 192 + (c & 1) * TN + part * COLS + i * 8;
-        if constexpr (COLS == 4) {
-          unsigned r[4];
-          u_tmem_ld4(at, r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        unsigned r[8];
+        u_tmem_ld8(at, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[j] += __uint_as_float(r[j]);
-        } else {
-          unsigned r[8];
-          u_tmem_ld8(at, r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i * 8 + j] += __uint_as_float(r[j]);
-        }
+        for (int j = 0; j < 8; ++j) acc[i * 8 + j] += __uint_as_float(r[j]);
       }
       if constexpr (BOTH == 2)
         if (c == slice_steps - 1) {

@@ -381,9 +381,9 @@ __device__ __forceinline__ void radix_add(SampleShared& sh, unsigned key, float 
     if (l2) atomicAdd(&sh.limb[2][key], l2);            // few weights are as large as 2^-7
   }
 }
-template <bool COUNT> __device__ __forceinline__ void radix_clear(SampleShared& sh) {      // counts leave the other two limbs alone
-  sh.limb[0][threadIdx.x] = 0;
-  if (!COUNT) { sh.limb[1][threadIdx.x] = 0; sh.limb[2][threadIdx.x] = 0; }
+__device__ __forceinline__ void radix_clear(SampleShared& sh) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) sh.limb[i][threadIdx.x] = 0;
 }
 
 // f(w[i]) for this block's n weights, four neighbours a 16-byte read; a short slice one a thread, so that none waits for four
@@ -555,7 +555,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
     sh.uniform = uniform01(seeds[row], counters[row]);
   }
   // the slice into shared memory, and its best logit
-  radix_clear<false>(sh);
+  radix_clear(sh);
   ArgPair best{-INFINITY, -1};
   if ((((uintptr_t)lg) & 15) == 0) {
     for (int i = tid * 4; i < n; i += SC_THREADS * 4) {

@@ -60,7 +60,7 @@ class PrenormRun:
         if not isinstance(position, (tuple, list)) or len(position) != 2 or 2 * position[0].shape[1] != hd:
             return None
         cos, sin = position
-        words, matrices = [], 0
+        words = []
         for block, info in zip(self.blocks, runs):
             a, f = block.mixer, block.feed_forward
             k, v, page_stride = ctx.kv.layer_views(info.kv_group, info.kv_index)
