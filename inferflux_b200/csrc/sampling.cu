@@ -11,7 +11,7 @@
 // maxima, top-k/top-p/min-p become a probability threshold on the float bit
 // pattern, and the uniform comes from a counter-based generator keyed by
 // (seed, counter) so a request's draws do not depend on the batch it is in.
-// A row that fits the shared memory of a thread-block cluster (up to 409,600
+// A row that fits the shared memory of a thread-block cluster (up to 406,912
 // logits) is read once and held there by up to 8 blocks; the threshold is
 // found by a radix search and all masses are added as integers (see
 // sample_cluster_kernel).  Longer rows go to one block of 1024 threads per
@@ -301,7 +301,7 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, float* __r
 }
 
 // ------------------------------------------------------------------ a row on a cluster
-// The same draw for rows that fit the shared memory of a thread-block cluster (8 blocks hold up to 409,600
+// The same draw for rows that fit the shared memory of a thread-block cluster (8 blocks hold up to 406,912
 // logits): every block keeps its slice of the row in shared memory, so the row is read from memory once and
 // every later pass runs on chip.  The threshold for top-k / top-p is found by a radix search over the float
 // bit pattern (three levels of 1,024 bins, histograms added across the cluster through distributed shared
@@ -309,7 +309,6 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, float* __r
 // (weight * 2^39, the maximum weight is exactly 1), so the result does not depend on the order of any sum
 // nor on how many blocks share the row.
 constexpr int SC_THREADS = 1024, SC_BINS = 1024, SC_MAX_CL = 8;
-constexpr int SC_MAX_SLICE = 51200;                     // floats of a row one block keeps (200 KB)
 constexpr int SC_LIST = 1024;                           // weights that a block can note down for the later levels, behind its slice
 constexpr int SC_GATHER = 4096;                         // weights of all blocks that one can gather, in the histograms' place
 constexpr int SC_MASS_KEY = (127 - 39) << 3;            // weights below this first-level key are below 2^-39: their mass is 0
@@ -318,7 +317,10 @@ struct SampleShared {
   unsigned limb[3][SC_BINS];                            // counts, or masses in three 16-bit limbs: 32-bit shared-memory adds
   unsigned long long hist[2][SC_BINS];                  // the limbs put together; two buffers: one is read by the cluster
                                                         // while the next fills
-  unsigned long long warp_tot[32];
+  union {
+    unsigned long long warp_tot[32];
+    ArgPair ascratch[32];                               // of the row's maximum, before the first scan
+  };
   unsigned long long part_total, bcast;                 // what this block tells the others; what lies above the chosen bin
   int chosen;
   int listed;                                           // weights noted; more than there is room for: they did not fit
@@ -326,8 +328,10 @@ struct SampleShared {
   int top_k;
   float uniform;
   ArgPair best;
-  ArgPair ascratch[32];
 };
+constexpr int SC_SHARED = 227 * 1024;                   // bytes a block can have
+constexpr int SC_MAX_SLICE = (SC_SHARED - (int)sizeof(SampleShared)) / 16 * 4;      // floats of a row one block keeps
+static_assert(SC_MAX_SLICE == 50864, "the row's limit above is eight of these");
 
 __device__ __forceinline__ unsigned long long weight_fix(float w) { return __float2ull_rz(w * 549755813888.0f); }   // * 2^39
 
@@ -373,7 +377,7 @@ template <bool COUNT>
 __device__ __forceinline__ void radix_add(SampleShared& sh, unsigned key, float v) {
   if (COUNT) {
     atomicAdd(&sh.limb[0][key], 1u);
-  } else {                                              // a slice has at most 51,200 entries: no limb's sum passes 2^32
+  } else {                                              // a slice has at most SC_MAX_SLICE entries, fewer than 2^16: no limb's sum passes 2^32
     const unsigned long long q = weight_fix(v);
     const unsigned l0 = (unsigned)(q & 0xFFFFu), l1 = (unsigned)(q >> 16) & 0xFFFFu, l2 = (unsigned)(q >> 32);
     if (l0) atomicAdd(&sh.limb[0][key], l0);
@@ -680,7 +684,7 @@ int launch_sample_cluster(const float* logits, long long row_stride, const float
                           const unsigned long long* counters, int* out, int n_rows, int vocab, int cl, cudaStream_t stream) {
   const int slice = ((vocab + cl - 1) / cl + 3) / 4 * 4;
   // the list takes what a slice leaves of 227 KB
-  const int left = (227 * 1024 - (int)sizeof(SampleShared)) / (int)sizeof(float) - slice - 16;
+  const int left = (SC_SHARED - (int)sizeof(SampleShared)) / (int)sizeof(float) - slice - 16;
   const int list_room = left < 0 ? 0 : left < SC_LIST ? left : SC_LIST;
   const size_t smem = (size_t)(slice + list_room) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
