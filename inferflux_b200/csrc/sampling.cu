@@ -672,22 +672,33 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, co
   cluster_sync_all();
 }
 
+inline int sample_slice(int vocab, int cl) { return ((vocab + cl - 1) / cl + 3) / 4 * 4; }
 // Blocks per row for the cluster kernel (a power of two up to 8), or 0 if the row does not fit
 inline int sample_cluster_blocks(int vocab) {
   int cl = 1;
   while (cl < SC_MAX_CL && (vocab + cl - 1) / cl > 8192) cl <<= 1;
-  return ((vocab + cl - 1) / cl + 3) / 4 * 4 <= SC_MAX_SLICE ? cl : 0;
+  return sample_slice(vocab, cl) <= SC_MAX_SLICE ? cl : 0;
+}
+
+// Room for the list: what the slice leaves of a block's shared memory, or, where the blocks are more than the SMs and two fit one SM, of half
+// of that (64 rows of 170,000 with top-p 90.5 us, 142.6 with the whole list and one block an SM).
+inline int sample_list_room(int slice, long long blocks, int sms) {
+  constexpr int PAIR = 228 * 1024 / 2 - 1024 - 64;      // of 228 KB an SM each block takes 1 KB besides its own
+  const int used = (int)sizeof(SampleShared) + slice * (int)sizeof(float);
+  const int left = ((blocks > sms && used <= PAIR ? PAIR : SC_SHARED - 64) - used) / (int)sizeof(float);
+  return left < 0 ? 0 : left < SC_LIST ? left : SC_LIST;
 }
 
 int launch_sample_cluster(const float* logits, long long row_stride, const float* temperature, const int* top_k,
                           const float* top_p, const float* min_p, const unsigned long long* seeds,
                           const unsigned long long* counters, int* out, int n_rows, int vocab, int cl, cudaStream_t stream) {
-  const int slice = ((vocab + cl - 1) / cl + 3) / 4 * 4;
-  // the list takes what a slice leaves of 227 KB
-  const int left = (SC_SHARED - (int)sizeof(SampleShared)) / (int)sizeof(float) - slice - 16;
-  const int list_room = left < 0 ? 0 : left < SC_LIST ? left : SC_LIST;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return (int)e;
+  const int slice = sample_slice(vocab, cl), list_room = sample_list_room(slice, (long long)n_rows * cl, sms);
   const size_t smem = (size_t)(slice + list_room) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int rc = launch_pdl_cluster(sample_cluster_kernel, dim3(n_rows * cl), dim3(SC_THREADS), smem, stream, dim3(cl, 1, 1),
                                     logits, row_stride, temperature, top_k, top_p, min_p, seeds, counters, out, vocab, cl, slice, list_room);
@@ -745,6 +756,14 @@ IFX_API int ifx_ring_append(int* ring, int ring_size, int* totals, const int* sl
   const int ifx_rc = launch_pdl(ring_append_kernel, dim3((n_rows + 127) / 128), dim3(128), 0, stream, ring, ring_size, totals, slots, ids,
                                 n_rows);
   return ifx_rc ? ifx_rc : IFX_LAUNCH_CHECK();
+}
+
+// The shared memory of ifx_sample's blocks: {blocks a row (0: not a cluster's row), bytes without the list, with it}.
+IFX_API void ifx_sample_shared(int vocab, int n_rows, int sms, int* out) {
+  const int cl = sample_cluster_blocks(vocab), slice = cl ? sample_slice(vocab, cl) : 0;
+  out[0] = cl;
+  out[1] = (int)sizeof(SampleShared) + slice * (int)sizeof(float);
+  out[2] = out[1] + (cl ? sample_list_room(slice, (long long)n_rows * cl, sms) : 0) * (int)sizeof(float);
 }
 
 IFX_API int ifx_sample(const float* logits, long long row_stride, float* weights, const float* temperature,

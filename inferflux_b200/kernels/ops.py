@@ -111,6 +111,8 @@ def _load():
         lib.ifx_apply_penalties_ring.restype = c_int
         lib.ifx_ring_append.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         lib.ifx_ring_append.restype = c_int
+        lib.ifx_sample_shared.argtypes = [c_int, c_int, c_int, c_void_p]
+        lib.ifx_sample_shared.restype = None
         lib.ifx_sample.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_int, c_int, c_void_p]
         for name in ("ifx_embed_gather", "ifx_add_rmsnorm", "ifx_swiglu", "ifx_convert", "ifx_rope_table",

@@ -2,6 +2,7 @@
 kernel's (tile, head) units are cut, against a plain list scheduling of the same units."""
 from __future__ import annotations
 
+import ctypes
 import heapq
 import random
 
@@ -106,3 +107,21 @@ def test_scratch_of_float32_products(ops, m, n, k, address, size):
     """None where none is used, six bytes a number of the rows, and never more than 64 MB."""
     got = ops.gemm_f32_scratch(address, m, n, k)
     assert got == size if size is not None else 32 << 20 < got <= 64 << 20
+
+
+def test_a_samplers_list_takes_no_block_off_an_sm(ops):
+    """Two blocks an SM (228 KB, of which each takes 1 KB besides its own) wherever two would fit without the list and are wanted; a list as
+    long as possible otherwise; never more than 227 KB."""
+    out = (ctypes.c_int * 3)()
+    fit = lambda size: 228 * 1024 // (size + 1024)
+    for vocab in [1, 1000, 8193, 32000, 100000, 152064, *range(160000, 176000, 500), 256000, 406400, 406464, 406912]:
+        for rows in (1, 18, 19, 64, 1000):
+            ops._lib().ifx_sample_shared(vocab, rows, SMS, out)
+            blocks, bare, whole = out
+            assert blocks and bare <= whole <= 227 * 1024
+            if rows * blocks > SMS:
+                assert min(2, fit(whole)) == min(2, fit(bare)), (vocab, rows)
+            else:
+                assert whole >= min(bare + 4096, 227 * 1024 - 128), (vocab, rows)
+    ops._lib().ifx_sample_shared(406913, 1, SMS, out)
+    assert out[0] == 0
