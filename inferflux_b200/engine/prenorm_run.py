@@ -4,7 +4,8 @@ A step that brings a prompt portion is launched kernel by kernel from the host, 
 for: at the 3B sizes 77 rows take the GPU 60 to 90 us a layer and the host, from Python, 110 to 140.  Where a model's layers are
 all of the common kind (:class:`~inferflux_b200.parts.block.PreNormBlock` of grouped-query attention and SwiGLU with RMSNorm,
 bfloat16, head size 128, no window) such a step's layers are launched by ``ops.prenorm_layers``: the same kernels with the same
-arguments, so the same results.  Everything else goes through the blocks.
+arguments, so the same results.  Everything else goes through the blocks; so does a model of which a block or one of its parts has
+been given a method of its own since it was made (to watch it, say) or been replaced.
 """
 from __future__ import annotations
 
@@ -18,15 +19,30 @@ from ..parts.attention import GQAttention, prefill_plan
 from ..parts.base import PartialSums
 from ..parts.block import PreNormBlock
 from ..parts.feed_forward import SwiGLU
-from ..parts.linear import FEW_ROWS_MIN_K
+from ..parts.linear import FEW_ROWS_MIN_K, Linear
 from ..parts.norm import RMSNorm
+
+
+#: What the call stands in for: the kinds of a layer's parts with the methods that launch their kernels, as they are here.
+_STANDS_FOR = {cls: {name: getattr(cls, name) for name in names} for cls, names in (
+    (PreNormBlock, ("forward",)), (RMSNorm, ("forward",)), (SwiGLU, ("forward",)), (Linear, ("forward",)),
+    (GQAttention, ("forward", "attend", "decode", "_fused_qkv", "_share_by_tiles")))}
+
+
+_MIXERS_OWN = frozenset(_STANDS_FOR[GQAttention])
+
+
+def _sizes(block) -> tuple:
+    m = block.mixer
+    return block.position_name, m.hidden, m.n_heads, m.n_kv, m.head_dim, m.scale, m.window, m.kv_shared, block.feed_forward.intermediate
 
 
 class PrenormRun:
     """The layers of a model that one call can launch: all of its runs or none."""
 
-    def __init__(self, blocks):
-        self.blocks = blocks                            # one per run, in schedule order
+    def __init__(self, model, blocks):
+        self.model, self.blocks = model, blocks         # one block per run, in schedule order
+        self.sizes = _sizes(blocks[0])
 
     @staticmethod
     def of(model) -> Optional["PrenormRun"]:
@@ -42,15 +58,36 @@ class PrenormRun:
             a = block.mixer
             if a.window or a.kv_shared or not info.writes_kv or a.head_dim != ops.UMMA_ATTENTION_HEAD_DIM or a.params.get("o_bias"):
                 return None
-            shapes.add((info.kv_group, block.position_name, a.hidden, a.n_heads, a.n_kv, a.scale, block.feed_forward.intermediate))
+            shapes.add((info.kv_group, *_sizes(block)))
         # (a shorter down projection goes to the library, which the call does not reach)
         if len(shapes) != 1 or blocks[0].mixer.hidden % 8 or blocks[0].feed_forward.intermediate % 8 or blocks[0].feed_forward.intermediate < FEW_ROWS_MIN_K:
             return None
-        return PrenormRun(blocks)
+        return PrenormRun(model, blocks)
 
     def takes(self, ctx) -> bool:
         step = ctx.extras[GQAttention.describe_key]
-        return ops.PRENORM_MIN_ROWS <= ctx.n_tokens <= ops.PRENORM_MAX_ROWS and step.n_decode != ctx.n_tokens
+        return ops.PRENORM_MIN_ROWS <= ctx.n_tokens <= ops.PRENORM_MAX_ROWS and step.n_decode != ctx.n_tokens and self._as_made()
+
+    def _as_made(self) -> bool:
+        """Whether blocks and parts are still of the kinds that the call stands in for, with these kinds' own methods (a microsecond a
+        layer)."""
+        for cls, methods in _STANDS_FOR.items():
+            if any(getattr(cls, name) is not method for name, method in methods.items()):
+                return False
+        for b, run in zip(self.blocks, self.model.spec.schedule):
+            if self.model.blocks[run.layer] is not b:
+                return False
+            m, f = b.mixer, b.feed_forward
+            if not (type(b) is PreNormBlock and type(m) is GQAttention and type(f) is SwiGLU and type(b.mixer_norm) is RMSNorm
+                    and type(b.feed_forward_norm) is RMSNorm and _MIXERS_OWN.isdisjoint(m.__dict__) and _sizes(b) == self.sizes):
+                return False
+            for linear in (m.qkv, m.o, f.gate_up, f.down):
+                if type(linear) is not Linear or "forward" in linear.__dict__:
+                    return False
+            for part in (b, f, b.mixer_norm, b.feed_forward_norm):
+                if "forward" in part.__dict__:
+                    return False
+        return True
 
     def forward(self, residual: torch.Tensor, ctx, runs) -> Optional[PartialSums]:
         """All layers; the last one's pending delta.  None (nothing done): weights or angles that the kernels do not take."""

@@ -4,6 +4,7 @@ import torch
 
 from inferflux_b200 import Engine, StepEntry
 from inferflux_b200.kernels import ops
+from inferflux_b200.parts.feed_forward import SwiGLU
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +57,57 @@ def test_models_of_another_kind_keep_their_blocks():
     for other in (dict(head_dim=64), dict(intermediate_size=1024), dict(use_sliding_window=True, sliding_window=64, max_window_layers=0)):
         engine = Engine.from_config(dict(CONFIG, **other), seed=3, dtype="bfloat16", kv_cache_tokens=1024, max_seqs=2, max_model_len=512)
         assert PrenormRun.of(engine.runner.model) is None
+
+
+WATCHED = {
+    "block": lambda m: m.blocks[1], "mixer": lambda m: m.blocks[2].mixer, "norm": lambda m: m.blocks[0].mixer_norm,
+    "second norm": lambda m: m.blocks[1].feed_forward_norm, "feed-forward": lambda m: m.blocks[1].feed_forward,
+    "qkv": lambda m: m.blocks[0].mixer.qkv, "down": lambda m: m.blocks[2].feed_forward.down}
+
+
+@pytest.mark.parametrize("of_the_class", [False, True])
+@pytest.mark.parametrize("what", sorted(WATCHED))
+def test_a_method_put_on_a_part_is_called(what, of_the_class, monkeypatch):
+    """A forward that stands on a block or part, or on its class, is called in these steps like in others; when it is gone, one call again."""
+    engine = Engine.from_config(CONFIG, seed=3, dtype="bfloat16", kv_cache_tokens=4096, max_seqs=4, max_model_len=512)
+    model = engine.runner.model
+    part, seen, took = WATCHED[what](model), [], []
+    forward = model._prenorm_run.forward
+    model._prenorm_run.forward = lambda *a: took.append(1) or forward(*a)
+    tokens = torch.randint(0, 1000, (40,), generator=torch.Generator().manual_seed(1)).tolist()
+    want = engine.run_step([StepEntry("a", tokens, [0, 39])]).clone()
+    assert len(took) == 1
+    with monkeypatch.context() as patch:
+        if of_the_class:
+            inner = type(part).forward
+            patch.setattr(type(part), "forward", lambda self, *a, **k: (seen.append(self is part), inner(self, *a, **k))[1])
+        else:
+            inner = part.forward
+            patch.setattr(part, "forward", lambda *a, **k: (seen.append(True), inner(*a, **k))[1], raising=False)
+        got = engine.run_step([StepEntry("b", tokens, [0, 39])]).clone()
+        assert any(seen) and len(took) == 1
+    part.__dict__.pop("forward", None)
+    assert torch.equal(got, want) and torch.equal(engine.run_step([StepEntry("c", tokens, [0, 39])]), want)
+    assert len(took) == 2
+
+
+def test_a_part_put_in_anothers_place_is_called():
+    class Watched(SwiGLU):
+        calls = 0
+
+        def forward(self, x, ctx):
+            Watched.calls += 1
+            return super().forward(x, ctx)
+    engine = Engine.from_config(CONFIG, seed=3, dtype="bfloat16", kv_cache_tokens=4096, max_seqs=4, max_model_len=512)
+    model = engine.runner.model
+    block = model.blocks[1]
+    made = block.feed_forward
+    other = Watched.__new__(Watched)
+    other.__dict__.update(made.__dict__)
+    block.feed_forward = other
+    engine.run_step([StepEntry("a", list(range(40)), [39])])
+    assert Watched.calls == 1
+    block.feed_forward = made
+    model.blocks[1] = type("Block", (), {"forward": lambda self, *a: (setattr(Watched, "calls", 5), block.forward(*a))[1]})()
+    engine.run_step([StepEntry("b", list(range(40)), [39])])
+    assert Watched.calls == 5
