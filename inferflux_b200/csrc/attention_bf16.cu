@@ -17,6 +17,7 @@
 // the 16 rows of an MMA tile are the query heads that share a kv head, so a
 // page is read once for all of them.
 #include "common.cuh"
+#include "launchers.h"
 #include "rope_math.cuh"
 #include <type_traits>
 

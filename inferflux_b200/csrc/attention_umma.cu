@@ -45,6 +45,7 @@
 // since every issued copy is waited for before the MMA that reads it, nothing is
 // in flight when the block frees its tensor memory and returns.
 #include "common.cuh"
+#include "launchers.h"
 #include <cuda.h>
 #include <cudaTypedefs.h>
 

@@ -10,6 +10,7 @@
 // passes, loads are 16 bytes wide where the row length allows, and any row
 // length is taken.
 #include "common.cuh"
+#include "launchers.h"
 
 // ---------------------------------------------------------------- embedding
 template <typename T>

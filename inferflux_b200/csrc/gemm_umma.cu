@@ -33,6 +33,7 @@
 // word, the other warps leave their loops, the block waits a moment for TMA copies in flight, and the
 // pair frees its tensor memory and returns.
 #include "umma.cuh"
+#include "launchers.h"
 
 namespace {
 

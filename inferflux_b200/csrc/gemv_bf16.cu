@@ -24,6 +24,7 @@
 // intermediate [M, 2I] tensor.  With a clamped activation (common.cuh's GluShape) the two meet through that
 // instead: 8 rows of the 7B sizes' gate and up 46.9 us, against 50.1 for float32 sums and 3.5 for a kernel on them.
 #include "common.cuh"
+#include "launchers.h"
 
 namespace {
 

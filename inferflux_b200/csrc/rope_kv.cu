@@ -14,6 +14,7 @@
 // per token, in double precision rounded to float32), and one kernel per layer
 // does bias + rotation + paged write for prompts and decoded tokens alike.
 #include "common.cuh"
+#include "launchers.h"
 #include "rope_math.cuh"
 
 // cos/sin tables [n_tokens, half] from positions and inverse frequencies.
