@@ -22,6 +22,7 @@ struct PrenormStep {
   long long page_stride;
   int rows, hidden, inter, n_heads, n_kv, page_size, bt_stride, num_pages;
   int qkv_parts, o_parts, down_parts;
+  int gate_up_streams;                              // gate and up by the weight-streaming kernel, not the few-row one
   int n_tiles, tile_rows, n_splits;                 // of the prompt portions
   int n_dec, dec_splits, dec_pieces;                // single tokens: dec_pieces > 0: shared out by tiles, else dec_splits parts of the keys
   float scale;
@@ -71,7 +72,7 @@ IFX_API int ifx_prenorm_layers(const PrenormStep* step, const PrenormLayer* laye
     if (!rc) rc = ifx_gemm_umma_skinny(s.attn, nq, l.o_w, s.delta, s.rows, s.hidden, nq, s.o_parts, 1, s.error_flag, s.stream);
     if (!rc) rc = ifx_add_rmsnorm(s.residual, s.delta, IFX_F32, s.o_parts, s.o_parts > 1 ? sum_stride : 0, l.norm2, (float)l.eps2, s.x, IFX_BF16,
                                   nullptr, s.rows, s.hidden, 1, s.stream);
-    if (!rc) rc = s.rows <= 16 ? ifx_gemv_bf16(s.x, l.gate_up_w, nullptr, s.act, IFX_BF16, s.rows, s.inter, s.hidden, s.hidden, s.inter, 1, 1, 0.0f,
+    if (!rc) rc = s.gate_up_streams ? ifx_gemv_bf16(s.x, l.gate_up_w, nullptr, s.act, IFX_BF16, s.rows, s.inter, s.hidden, s.hidden, s.inter, 1, 1, 0.0f,
                                                0.0f, 0.0f, s.stream)
                                : ifx_gemm_umma_skinny_glu(s.x, s.hidden, l.gate_up_w, s.act, s.inter, s.rows, s.inter, s.hidden, 1, s.error_flag, s.stream);
     if (!rc) rc = ifx_gemm_umma_skinny(s.act, s.inter, l.down_w, s.delta, s.rows, s.hidden, s.inter, s.down_parts, 1, s.error_flag, s.stream);

@@ -18,10 +18,12 @@ from ..kernels import ops
 from ..parts.attention import GQAttention, prefill_plan
 from ..parts.base import PartialSums
 from ..parts.block import PreNormBlock
-from ..parts.feed_forward import SwiGLU
-from ..parts.linear import FEW_ROWS_MIN_K, Linear
+from ..parts.feed_forward import FUSED_PRODUCT_ROWS, SwiGLU
+from ..parts.linear import FEW_ROWS, FEW_ROWS_MIN_K, GEMV_ROWS, Linear
 from ..parts.norm import RMSNorm
 
+#: The rows for which the parts take the kernels of the call: more than the weight-streaming product's, no more than the few-row kernels'.
+MIN_ROWS, MAX_ROWS = GEMV_ROWS + 1, min(FEW_ROWS, FUSED_PRODUCT_ROWS)
 
 #: What the call stands in for: the kinds of a layer's parts with the methods that launch their kernels, as they are here.
 _STANDS_FOR = {cls: {name: getattr(cls, name) for name in names} for cls, names in (
@@ -66,7 +68,7 @@ class PrenormRun:
 
     def takes(self, ctx) -> bool:
         step = ctx.extras[GQAttention.describe_key]
-        return ops.PRENORM_MIN_ROWS <= ctx.n_tokens <= ops.PRENORM_MAX_ROWS and step.n_decode != ctx.n_tokens and self._as_made()
+        return MIN_ROWS <= ctx.n_tokens <= MAX_ROWS and step.n_decode != ctx.n_tokens and self._as_made()
 
     def _as_made(self) -> bool:
         """Whether blocks and parts are still of the kinds that the call stands in for, with these kinds' own methods (a microsecond a
@@ -90,32 +92,48 @@ class PrenormRun:
         return True
 
     def forward(self, residual: torch.Tensor, ctx, runs) -> Optional[PartialSums]:
-        """All layers; the last one's pending delta.  None (nothing done): weights or angles that the kernels do not take."""
+        """All layers; the last one's pending delta.  None (nothing done): weights, angles or a cache of which the kernels of the call
+        take no such form; the blocks choose others, or refuse them."""
         first, n, dev = self.blocks[0].mixer, ctx.n_tokens, residual.device
         hidden, inter, nh, nkv, hd = first.hidden, self.blocks[0].feed_forward.intermediate, first.n_heads, first.n_kv, first.head_dim
+        width, g, page = (nh + 2 * nkv) * hd, runs[0].kv_group, nkv * ctx.page_size * hd
         position = ctx.position_tables.get(self.blocks[0].position_name) if self.blocks[0].position_name else None
-        if not isinstance(position, (tuple, list)) or len(position) != 2 or 2 * position[0].shape[1] != hd:
+        if not isinstance(position, (tuple, list)) or len(position) != 2:
             return None
         cos, sin = position
+        if any(t.shape != (n, hd // 2) or t.dtype != torch.float32 or not t.is_contiguous() for t in position):
+            return None
+        if not residual.is_contiguous() or residual.dtype != torch.float32 or ctx.slot_maps[g].dtype != torch.int32 or ctx.slot_maps[g].numel() != n:
+            return None
+        tables = ctx.block_tables[g]
+        if tables.dtype != torch.int32 or tables.stride(1) != 1:
+            return None
+        shapes = ((width, hidden), (hidden, nh * hd), (2 * inter, hidden), (hidden, inter))
         words = []
         for block, info in zip(self.blocks, runs):
             a, f = block.mixer, block.feed_forward
             k, v, page_stride = ctx.kv.layer_views(info.kv_group, info.kv_index)
-            mats = (a.qkv.weight, a.o.weight, f.gate_up.weight, f.down.weight)
-            at = [m.data_ptr() for m in mats]
-            if any(m.dtype != torch.bfloat16 for m in mats) or any(p & 15 for p in at):
+            if k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or (not words and ops.paged_pool_pages(k, v, page_stride, page) < 1):
                 return None
-            if a.qkv.bias is not None or a.o.bias is not None or f.down.bias is not None:
+            at = []
+            for linear, shape in zip((a.qkv, a.o, f.gate_up, f.down), shapes):
+                w = linear.weight
+                at.append(w.data_ptr())
+                if w.dtype != torch.bfloat16 or w.shape != shape or at[-1] & 15 or not w.is_contiguous() or linear.bias is not None:
+                    return None
+            bias, norms = a.qkv_bias, (block.mixer_norm.weight, block.feed_forward_norm.weight)
+            if bias is not None and (bias.dtype != torch.float32 or bias.numel() != width or not bias.is_contiguous()):
                 return None
-            words.append((block.mixer_norm.weight.data_ptr(), at[0], 0 if a.qkv_bias is None else a.qkv_bias.data_ptr(),
-                          k.data_ptr(), v.data_ptr(), at[1], block.feed_forward_norm.weight.data_ptr(), at[2], at[3], 0, 0))
+            if any(w.dtype != torch.float32 or w.numel() != hidden for w in norms):
+                return None
+            words.append((norms[0].data_ptr(), at[0], 0 if bias is None else bias.data_ptr(), k.data_ptr(), v.data_ptr(), at[1],
+                          norms[1].data_ptr(), at[2], at[3], 0, 0))
         layers = np.array(words, dtype=np.int64)
         eps = layers.view(np.float64)
         eps[:, 9] = [b.mixer_norm.eps for b in self.blocks]
         eps[:, 10] = [b.feed_forward_norm.eps for b in self.blocks]
 
-        step, width = ctx.extras[GQAttention.describe_key], (nh + 2 * nkv) * hd
-        g = runs[0].kv_group
+        step = ctx.extras[GQAttention.describe_key]
         s = ops.PrenormStep()
         keep = []                                       # scratch stays until the kernels are launched (then the stream orders its reuse)
 
@@ -133,10 +151,10 @@ class PrenormRun:
         s.x, s.qkv, s.attn, s.act = (scratch(bf16, n * w) for w in (hidden, width, nh * hd, inter))
         s.qkv_sums = scratch(f32, s.qkv_parts * n * width)
         s.cos_t, s.sin_t, s.slot_map = cos.data_ptr(), sin.data_ptr(), ctx.slot_maps[g].data_ptr()
-        tables = ctx.block_tables[g]
         s.block_tables, s.bt_stride, s.page_stride = tables.data_ptr(), tables.stride(0), page_stride
         s.entry_q_start, s.entry_q_len, s.entry_ctx_start = (t.data_ptr() for t in (ctx.entry_q_start, ctx.entry_q_len, ctx.entry_ctx_start))
-        s.num_pages = ops.paged_pool_pages(k, v, page_stride, nkv * ctx.page_size * hd)
+        s.num_pages = ops.paged_pool_pages(k, v, page_stride, page)
+        s.gate_up_streams = n <= ops.GEMV_MAX_ROWS
         s.scale = first.scale
         s.n_tiles, s.tile_rows = step.n_umma_tiles, step.umma_tile_rows
         s.tile_entry, s.tile_q0 = step.umma_tile_entry.data_ptr(), step.umma_tile_q0.data_ptr()

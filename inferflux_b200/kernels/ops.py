@@ -947,7 +947,7 @@ class PrenormStep(ctypes.Structure):
                                          "dec_entries", "part_o", "part_ml", "dec_o", "dec_ml", "piece_count", "error_flag", "stream")]
                 + [("page_stride", c_ll)]
                 + [(n, c_int) for n in ("rows", "hidden", "inter", "n_heads", "n_kv", "page_size", "bt_stride", "num_pages", "qkv_parts",
-                                        "o_parts", "down_parts", "n_tiles", "tile_rows", "n_splits", "n_dec", "dec_splits", "dec_pieces")]
+                                        "o_parts", "down_parts", "gate_up_streams", "n_tiles", "tile_rows", "n_splits", "n_dec", "dec_splits", "dec_pieces")]
                 + [("scale", c_float)])
 
 

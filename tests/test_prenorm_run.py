@@ -13,16 +13,18 @@ CONFIG = dict(architectures=["Qwen2ForCausalLM"], model_type="qwen2", hidden_siz
               tie_word_embeddings=False, max_position_embeddings=8192, use_sliding_window=False, hidden_act="silu", torch_dtype="bfloat16")
 
 
-def _run(native, steps, **config):
+def _run(native, steps, change=None, **config):
     engine = Engine.from_config(dict(CONFIG, **config), seed=3, dtype="bfloat16", kv_cache_tokens=16384, max_seqs=40, max_batch_size=40,
                                 max_batch_tokens=8192, max_model_len=4096)
     model = engine.runner.model
+    if change is not None:
+        change(model)
     took = []
     if not native:
         model._prenorm_run = None
     elif model._prenorm_run is not None:
         forward = model._prenorm_run.forward
-        model._prenorm_run.forward = lambda *a: took.append(1) or forward(*a)
+        model._prenorm_run.forward = lambda *a: (out := forward(*a), took.append(out is not None))[0]
     gen, out, counts = torch.Generator().manual_seed(5), [], []
     for step in steps:
         entries = []
@@ -33,7 +35,7 @@ def _run(native, steps, **config):
         out.append(engine.run_step(entries).clone())
         counts.append(ops.launch_count - before)
     ops.check_device_errors("cuda:0")
-    return out, counts, len(took)
+    return out, counts, sum(took)
 
 
 @pytest.mark.parametrize("steps,native_steps", [
@@ -48,6 +50,52 @@ def test_layers_of_one_call_are_the_parts_layers(steps, native_steps):
     got, counts, took = _run(True, steps)
     assert took == native_steps
     assert counts == want_counts
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
+
+
+STEPS = [[("a", 9)], [("a", 16)], [("b", 17), ("a", 1)], [("c", 900)], [("c", 77), ("a", 1)], [("d", 128)], [("c", 40), ("b", 1), ("d", 3)]]
+
+
+@pytest.mark.parametrize("config", [dict(hidden_size=768, num_attention_heads=6, num_key_value_heads=6, intermediate_size=8200),
+                                    dict(hidden_size=1032, num_attention_heads=16, num_key_value_heads=2, num_hidden_layers=2, intermediate_size=11008)])
+def test_layers_of_other_sizes(config):
+    """Other widths and numbers of heads, at the rows where the kernels change."""
+    want, want_counts, _ = _run(False, STEPS, **config)
+    got, counts, took = _run(True, STEPS, **config)
+    assert took == 6 and counts == want_counts
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
+
+
+def _off_the_boundary(model):
+    linear = model.blocks[1].mixer.o
+    room = torch.empty(linear.weight.numel() + 1, dtype=torch.bfloat16, device=linear.weight.device)
+    linear.weight = room[1:].view(linear.weight.shape).copy_(linear.weight)
+
+
+def _half_the_rotation(model):
+    (position,) = model.positions.values()
+    position.rotary_dim, position.inv_freq = 64, position.inv_freq[:32].contiguous()
+
+
+def _float32_weights(model):
+    linear = model.blocks[2].feed_forward.down
+    linear.weight = linear.weight.float()
+
+
+def _biased(model):
+    linear = model.blocks[0].mixer.o
+    linear.bias = torch.randn(linear.out_features, generator=torch.Generator().manual_seed(2)).to(linear.weight.device)
+
+
+@pytest.mark.parametrize("change", [_off_the_boundary, _half_the_rotation, _float32_weights, _biased])
+def test_what_the_call_does_not_take_goes_through_the_blocks(change):
+    """Weights off the 16-byte boundaries, of another type or with a bias, another width of the rotation: nothing of the call has been
+    done, and the blocks' results come out."""
+    want, want_counts, _ = _run(False, STEPS, change)
+    got, counts, took = _run(True, STEPS, change)
+    assert took == 0 and counts == want_counts
     for w, g in zip(want, got):
         assert torch.equal(w, g)
 
