@@ -181,7 +181,7 @@ class Model:
         if self._keeps_embedding:
             ctx.embedding_output = residual.clone()      # a block reads the stream as the embedding left it
         delta = None
-        if self._prenorm_run is not None and self._prenorm_run.takes(ctx):
+        if self._prenorm_run is not None and self._prenorm_run.takes(self, ctx):
             delta = self._prenorm_run.forward(residual, ctx, self.runs)      # (None: not for these weights)
         if delta is None:
             for info in self.runs:

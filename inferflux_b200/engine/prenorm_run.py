@@ -42,8 +42,8 @@ def _sizes(block) -> tuple:
 class PrenormRun:
     """The layers of a model that one call can launch: all of its runs or none."""
 
-    def __init__(self, model, blocks):
-        self.model, self.blocks = model, blocks         # one block per run, in schedule order
+    def __init__(self, blocks):
+        self.blocks = blocks                            # one per run, in schedule order (the model holds this, not the other way round too)
         self.sizes = _sizes(blocks[0])
 
     @staticmethod
@@ -64,20 +64,20 @@ class PrenormRun:
         # (a shorter down projection goes to the library, which the call does not reach)
         if len(shapes) != 1 or blocks[0].mixer.hidden % 8 or blocks[0].feed_forward.intermediate % 8 or blocks[0].feed_forward.intermediate < FEW_ROWS_MIN_K:
             return None
-        return PrenormRun(model, blocks)
+        return PrenormRun(blocks)
 
-    def takes(self, ctx) -> bool:
+    def takes(self, model, ctx) -> bool:
         step = ctx.extras[GQAttention.describe_key]
-        return MIN_ROWS <= ctx.n_tokens <= MAX_ROWS and step.n_decode != ctx.n_tokens and self._as_made()
+        return MIN_ROWS <= ctx.n_tokens <= MAX_ROWS and step.n_decode != ctx.n_tokens and self._as_made(model)
 
-    def _as_made(self) -> bool:
+    def _as_made(self, model) -> bool:
         """Whether blocks and parts are still of the kinds that the call stands in for, with these kinds' own methods (a microsecond a
         layer)."""
         for cls, methods in _STANDS_FOR.items():
             if any(getattr(cls, name) is not method for name, method in methods.items()):
                 return False
-        for b, run in zip(self.blocks, self.model.spec.schedule):
-            if self.model.blocks[run.layer] is not b:
+        for b, run in zip(self.blocks, model.spec.schedule):
+            if model.blocks[run.layer] is not b:
                 return False
             m, f = b.mixer, b.feed_forward
             if not (type(b) is PreNormBlock and type(m) is GQAttention and type(f) is SwiGLU and type(b.mixer_norm) is RMSNorm

@@ -1,9 +1,11 @@
 """Configuration, registry, safetensors and weight binding (no GPU)."""
 from __future__ import annotations
 
+import gc
 import json
 import os
 import struct
+import weakref
 
 import pytest
 import torch
@@ -244,3 +246,18 @@ def test_another_architecture_can_be_registered():
     names = {w.name for w in m.weight_specs()}
     assert {"blocks.0.attn.o_proj.bias", "blocks.0.ff.down_proj.weight", "emb.weight", "head.weight"} <= names
     assert "blocks.0.attn.q_proj.bias" not in names
+
+
+def test_a_model_is_gone_with_its_last_reference():
+    """Nothing that a model holds holds the model: its weights are given back at once, not when a collector comes by."""
+    config = dict(TINY_A, hidden_size=256, num_attention_heads=2, num_key_value_heads=2, head_dim=128, intermediate_size=8192, torch_dtype="bfloat16")
+    gc.disable()
+    try:
+        for c, dtype in ((config, torch.bfloat16), (TINY_A, torch.float32), (TINY_E, torch.bfloat16)):
+            model = Model(build_spec(load_config(c)), dtype, "cpu")
+            assert (model._prenorm_run is not None) == (c is config)
+            alive = weakref.ref(model)
+            del model
+            assert alive() is None
+    finally:
+        gc.enable()
