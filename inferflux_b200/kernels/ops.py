@@ -422,8 +422,8 @@ def qkv_rope_kv_write(qkv: torch.Tensor, bias: Optional[torch.Tensor], cos: torc
 # before it has waited itself); a copy, a kernel of torch or a synchronisation after the write settles it.  Without the flag
 # ``w`` may be anything, the output of the kernel just before included.
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, w_fixed: bool = False) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32 and to float32's precision: exact thirds of the operands on the
-    tensor cores, or plain FFMA for small matrices (``w_fixed``: see above).  A bounded wait that runs out sets the device's
+    """out[M, N] = a[M, K] @ w[N, K]^T + bias, all float32: the operands' exact parts on the tensor cores (a product
+    within 2^-23 of itself, sums closer to 64 bits than a chain of multiply-adds), or plain FFMA for small matrices (``w_fixed``: see above).  A bounded wait that runs out sets the device's
     error flag (see :func:`check_device_errors`)."""
     m, k = a.shape
     n = w.shape[0]
