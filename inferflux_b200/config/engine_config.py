@@ -26,7 +26,7 @@ class EngineConfig:
     device: str = "cuda:0"
     page_size: int = 16
     kv_cache_tokens: Optional[int] = None   # pool size in tokens per cache group
-    kv_memory_ratio: float = 0.80           # of free memory, when kv_cache_tokens is None
+    kv_memory_ratio: float = 0.80           # of free memory, when kv_cache_tokens is None; a step works in the rest (float32 products in 64 MB of it)
     max_seqs: int = 128                     # state slots = live requests
     max_batch_tokens: int = 16384           # tokens per step
     max_batch_size: int = 32                # requests per step
