@@ -33,7 +33,8 @@
 // (623), N 2,048 K 11,008 94 (373), N 2,560 K 2,048 40 (94); 64 rows 71 (251), 42 (182), 14 (50); 16 rows 41 (111), 28 (76), 8.6 (16.5); 8 rows 40
 // (72), 27 (50), 8.4 (11.5); 4 rows 39 (46), 27 (33), 7.7 (9.7); 2 rows 39 (46), 27 (32), 7.5 (9.5); 1 row 39 (39), 26.5 (27), 7.2 (7.2), N 151,936
 // K 2,048 205 (214).  Behind multiply-adds is one row of a square matrix of up to 2,048, whose blocks have few steps: 2,048 6.8 us (6.2), 1,024
-// 5.7 (4.5), 512 5.3 (4.1), 256 4.2 (3.2); it stays here for the sake of its bits, which are those of every batch.
+// 5.7 (4.5), 512 5.3 (4.1), 256 4.2 (3.2); it stays here for the sake of its bits, which are those of every batch.  A decode step of one
+// request (4 layers of the 3B sizes and the vocabulary) takes 827 us (876).
 #include "gemm_f32_umma.h"
 #include "umma.cuh"
 
@@ -114,9 +115,9 @@ __device__ __forceinline__ bool odd_sum(float v) {
   const unsigned u = __float_as_uint(v) & 0x7FFFFFFFu;
   return u >= 0x7F800000u || (u < U_SMALL && u != 0);
 }
-// Makes the odd ones among sums [BOTH][TN][128] again, of slices slice_len long from k_begin on, called by all workers: the tokens that have any 16 a part at a time, W
-// and the tokens through the shared memory behind the sums, the next 32 along K on their way meanwhile.  In a function of its own and
-// with the sums in memory it leaves the kernel's registers alone (inlined it cost up to 7 %).
+// Makes the odd ones among sums [BOTH][TN][128] again, of slices slice_len long from k_begin on, called by all workers: the tokens that
+// have any 16 a part at a time, W and the tokens through the shared memory behind the sums, the next 32 along K on their way
+// meanwhile.  In a function of its own and with the sums in memory it leaves the kernel's registers alone (inlined it cost up to 7 %).
 // (One NaN among 301 rows, N 22,016 K 2,048: 325 us where the product alone takes 142; in every row 1,750; 1 row 170 and 39.  A
 // thread a sum by itself took 2,600, 55,800 and 1,780.)
 template <int TN, int BOTH>
@@ -516,11 +517,11 @@ constexpr int U_TWO_TOKENS = 96;                 // tokens up to which a block c
 struct TokenTiles { int tn, count, both; };
 // Tiles of tokens, and one slice or two a block, by the time that rounds of blocks over the SMs take.  Clusters of 4 and 8 blocks fit
 // 132 and 120 of 148 SMs only (cudaOccupancyMaxActiveClusters), so two slices a block can save a round: us with two (with one), 1 row
-// N 22,016 K 2,048 38.5 (44), 4,608 x 3,584 19.2 (20.3); 32 rows 2,048 x 2,048 10.6 (15.6); 700 rows 60 (72).  ns, all measured: a step takes 700 with
-// 16 tokens (1,190 with two blocks an SM), 830, 1,000 and 1,090 with 32, 48 and 64, which the workers cut up as well, 800 with 80
-// to 1,110 with 160; a block has 2,000 and 19 a token of its own; two slices with
-// 96 tokens, whose registers spill, a twentieth more; split_kernel takes 2,500.  Over 16 shapes and numbers of rows from
-// 100 to 2,048 the tiles chosen are within 8 % of the best ones, but for 100 rows x 2,048 K 320 (7.2 us, 6.4 with tiles of 32).
+// N 22,016 K 2,048 38.5 (44), 4,608 x 3,584 19.2 (20.3), 32 rows 2,048 x 2,048 10.6 (15.6), 700 rows 60 (72).  All of this is measured, in
+// ns: a step takes 700 with 16 tokens (1,190 with two blocks an SM), 830, 1,000 and 1,090 with 32, 48 and 64, which the workers cut up
+// as well, 800 with 80 to 1,110 with 160; a block has 2,000 and 19 a token of its own; two slices with 96 tokens, whose registers
+// spill, take a twentieth more; split_kernel takes 2,500.  Over 16 shapes and numbers of rows from 100 to 2,048 the tiles chosen are
+// within 8 % of the best ones, but for 100 rows x 2,048 K 320 (7.2 us, 6.4 with tiles of 32).
 TokenTiles token_tiles(int M, int N, int slices, int steps, int sms) {
   TokenTiles best{16, 1, 1};
   long long best_cost = -1;
